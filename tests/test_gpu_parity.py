@@ -36,6 +36,17 @@ def test_generator_sampled_ranges(g500, oracle_mod, scale, ef):
         assert np.array_equal(dev.view(np.uint32), ref.view(np.uint32)), (scale, s)
 
 
+@pytest.mark.parametrize("scale", [2, 3, 5, 6, 7, 8, 9, 31, 32, 33, 47, 48])
+def test_generator_draw_remainders_and_widths(g500, oracle_mod, scale):
+    """Every remainder of the five-draw unrolling, both sides of the 32-bit descent words and the largest
+    scale, from both ends of the edge range."""
+    m = (1 << scale)
+    for s in {0, max(0, m // 3 - 50), max(0, m - 257)}:
+        e = min(m, s + 257)
+        assert np.array_equal(g500.generate_edges(scale, 1, s, e).view(np.uint32),
+                              oracle_mod.generate_edges(scale, 1, s, e).view(np.uint32)), (scale, s)
+
+
 @pytest.mark.parametrize("scale,vr", GOLDEN_CASES)
 def test_generator_matches_reference_fixture(g500, scale, vr):
     rec, arr = load_golden(scale, vr)

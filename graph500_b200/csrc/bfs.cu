@@ -95,6 +95,8 @@ struct RunParams {
   double alpha, beta;
   int count_edges;
   int policy;
+  const unsigned long long* endw;  // [nwords] sum of endp over each word's vertices with edges, or null
+  const uint32_t* endp;            // (endw null: the run does not sum its edges)
 };
 
 constexpr uint32_t FIRST_CHUNK = 0x80000000u;
@@ -121,11 +123,6 @@ __device__ __forceinline__ void put_deferred(const RunParams& p, int64_t r, uint
 
 __device__ __forceinline__ uint32_t chunks_of(uint64_t deg) { return (uint32_t)((deg + TD_CHUNK - 1) / TD_CHUNK); }
 
-__device__ __forceinline__ void flush_counter(unsigned long long* c, unsigned long long v) {
-  v = warp_sum(v);
-  if ((threadIdx.x & 31) == 0 && v) atomicAdd(c, v);
-}
-
 // Append the chunks of one row per lane (rows of degree < 2 and lanes with no
 // row pass deg 0).  The whole warp writes the items, so a hub's thousands of
 // chunks are not left to one lane; a row of more than BIG_CHUNKS chunks is
@@ -135,8 +132,7 @@ __device__ __forceinline__ void flush_counter(unsigned long long* c, unsigned lo
 // counts the items, each listing lane its row) for the phase's totals.
 __device__ __forceinline__ void append_row(uint64_t rb, uint64_t deg, uint32_t orig, TdItem* __restrict__ q_out,
                                            int64_t cap, unsigned long long* qcount, BfsCtl* ctl, TdItem* big,
-                                           unsigned long long* bigcount, unsigned long long* items,
-                                           unsigned long long* bigs) {
+                                           unsigned long long* bigcount, uint32_t* items, uint32_t* bigs) {
   const int lane = threadIdx.x & 31;
   uint32_t nch = chunks_of(deg);
   if (nch > BIG_CHUNKS && deg < (1ull << 31)) {
@@ -310,7 +306,7 @@ __device__ void td_phase(const RunParams& p, const TdItem* __restrict__ q_in, in
 __device__ void chunk_phase(const RunParams& p, const uint2* __restrict__ found_list, int64_t n, TdItem* q_out,
                             unsigned long long* pos, unsigned long long* sh_acc) {
   const int lane = threadIdx.x & 31;
-  unsigned long long skipped = 0, items = 0, bigs = 0;
+  uint32_t skipped = 0, items = 0, bigs = 0;  // per thread: far fewer than 2^32
   for (int64_t base = gwarp_id() * 32; base < n; base += gwarp_count() * 32) {
     const int64_t i = base + lane;
     uint64_t rb = 0, deg = 0;
@@ -519,7 +515,7 @@ __device__ void compact_phase(const RunParams& p, const uint32_t* __restrict__ v
                               const uint32_t* __restrict__ vis_old, TdItem* q_out, unsigned long long* pos,
                               unsigned long long* sh_acc) {
   const int lane = threadIdx.x & 31;
-  unsigned long long skipped = 0, items = 0, bigs = 0;
+  uint32_t skipped = 0, items = 0, bigs = 0;  // per thread: far fewer than 2^32
   const int64_t nwarps = gwarp_count();
   for (int64_t k32 = 0; gwarp_id() + k32 * nwarps < p.nwords; k32 += 32) {
     const int64_t wi = gwarp_id() + (k32 + lane) * nwarps;
@@ -628,6 +624,7 @@ __global__ void __launch_bounds__(BFS_THREADS, BFS_MIN_BLOCKS) bfs_persistent_ke
   int cur_vis = 0;
   bool forward = true, growing = true;
   int64_t qn = root_items, prev_nq = 0, visited = 1, carried = 0, nbig = 0;
+  unsigned td_levels = 0;
   int64_t mu = (int64_t)(p.off[p.nlv] - root_deg);  // degree sum of unvisited vertices (edge policy)
   unsigned phase = 0;
   int level = 1;
@@ -672,6 +669,7 @@ __global__ void __launch_bounds__(BFS_THREADS, BFS_MIN_BLOCKS) bfs_persistent_ke
     const int64_t carried_in = carried;
     visited += nq;
     const bool was_forward = forward;
+    td_levels += was_forward;
     if (!forward) cur_vis ^= 1;  // the bottom-up output is the current visited map
     if (nq == 0) {
       if (tid == 0) write_record(p.rec, level, was_forward, front + carried_in, disc, scan,
@@ -717,15 +715,32 @@ __global__ void __launch_bounds__(BFS_THREADS, BFS_MIN_BLOCKS) bfs_persistent_ke
                    edges + (was_forward ? carried_in : 0), sect + (was_forward ? carried_in : 0), t_mid);
   }
 #undef NEXT_PHASE_SLOT
-  // deferred modes: the entries of the vertices the search did not reach (and
-  // of those without edges) become "unreached", so that the final pass reads
-  // one entry per vertex and no bitmap.  The last level's barrier has passed:
-  // the visited map is final.  Under VERTEX_REORDERING 2 few such vertices lie
-  // below nlv (those without edges sort last).
-  if constexpr (DEF != 0) {
-    const uint32_t* vf = p.vis[cur_vis];
-    for (int64_t wi = tid; wi < p.nwords; wi += nthreads) {
-      uint32_t miss = ~(__ldcg(vf + wi) & ~__ldg(p.vis_init + wi));
+  if (tid == 0) {
+    ctl->num_levels = (unsigned)level;
+    ctl->td_levels = td_levels;
+    ctl->reached = (unsigned long long)visited;
+    ctl->final_vis = cur_vis;
+    ctl->t_end_ns = globaltimer();
+  }
+  // The last level's barrier has passed: the visited map is final.
+  //  - Deferred modes: the entries of the vertices the search did not reach
+  //    (and of those without edges) become "unreached", so that the final pass
+  //    reads one entry per vertex and no bitmap.  Under VERTEX_REORDERING 2 few
+  //    such vertices lie below nlv (those without edges sort last).
+  //  - The input edges inside the reached component: 2 * nedge = the sum of
+  //    endp over the reached vertices (validate.hpp's edge_visit_count for a
+  //    valid tree).  A word's sum over all its vertices with edges is known
+  //    (endw), so only the smaller side of a word, its reached or its
+  //    unreached vertices, is added up: for the usual search, which reaches
+  //    all but a few, that reads 8 bytes per 32 vertices.  A kernel of its own
+  //    that added endp of every reached vertex took 14 / 43 / 150 us at SCALE
+  //    22 / 24 / 26 after every run.
+  const uint32_t* vf = p.vis[cur_vis];
+  unsigned long long e2 = 0;
+  for (int64_t wi = tid; wi < p.nwords; wi += nthreads) {
+    const uint32_t seen = __ldcg(vf + wi), has = ~__ldg(p.vis_init + wi);
+    if constexpr (DEF != 0) {
+      uint32_t miss = ~(seen & has);
       while (miss) {
         const int b = __ffs(miss) - 1;
         miss &= miss - 1;
@@ -733,11 +748,24 @@ __global__ void __launch_bounds__(BFS_THREADS, BFS_MIN_BLOCKS) bfs_persistent_ke
         else p.pred_r[wi * 32 + b] = -1;
       }
     }
+    if (p.endw) {
+      const uint32_t in = seen & has, out = has & ~seen;
+      const bool few_in = __popc(in) < __popc(out);
+      uint32_t side = few_in ? in : out;
+      unsigned long long sum = 0;
+      while (side) {
+        const int b = __ffs(side) - 1;
+        side &= side - 1;
+        sum += __ldg(p.endp + wi * 32 + b);
+      }
+      e2 += few_in ? sum : __ldg(p.endw + wi) - sum;
+    }
   }
-  if (tid == 0) {
-    ctl->num_levels = (unsigned)level;
-    ctl->final_vis = cur_vis;
-    ctl->t_end_ns = globaltimer();
+  if (p.endw) {
+    e2 = warp_sum(e2);
+    if ((threadIdx.x & 31) == 0 && e2) atomicAdd(&sh_acc[0], e2);  // cleared by the last barrier
+    __syncthreads();
+    if (threadIdx.x == 0 && sh_acc[0]) atomicAdd(&ctl->edges2, sh_acc[0]);
   }
 }
 
@@ -784,27 +812,16 @@ __global__ void __launch_bounds__(FINAL_THREADS, 8) deferred_pred_kernel(RunPara
   }
 }
 
-// reached vertices and 2 x the input edges inside the reached component
-// (sum of endpoint occurrences = 2 x validate.hpp's edge_visit_count for a valid tree)
-__global__ void __launch_bounds__(256) reach_kernel(const uint32_t* vis0, const uint32_t* vis1,
-                                                    const uint32_t* __restrict__ vis_init,
-                                                    const uint32_t* __restrict__ endp, int64_t nwords,
-                                                    BfsCtl* ctl) {
-  if (!ctl->root_has_edges) return;
-  const uint32_t* vis = ctl->final_vis ? vis1 : vis0;
-  unsigned long long reached = 0, e2 = 0;
-  for (int64_t wi = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; wi < nwords;
-       wi += (int64_t)gridDim.x * blockDim.x) {
-    uint32_t bits = vis[wi] & ~vis_init[wi];
-    reached += __popc(bits);
-    while (bits) {
-      const int b = __ffs(bits) - 1;
-      bits &= bits - 1;
-      e2 += endp[wi * 32 + b];
-    }
+// endw[w] = sum of endp over the vertices with edges of word w (a warp per word)
+__global__ void __launch_bounds__(256) word_ends_kernel(const uint32_t* __restrict__ vis_init,
+                                                        const uint32_t* __restrict__ endp, int64_t nwords,
+                                                        unsigned long long* __restrict__ endw) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t wi = gwarp_id(); wi < nwords; wi += gwarp_count()) {
+    const bool has = !((__ldg(vis_init + wi) >> lane) & 1u);
+    const unsigned long long v = warp_sum(has ? (unsigned long long)__ldg(endp + wi * 32 + lane) : 0ull);
+    if (lane == 0) endw[wi] = v;
   }
-  flush_counter(&ctl->reach[0], reached);
-  flush_counter(&ctl->reach[1], e2);
 }
 
 }  // namespace g500
@@ -828,6 +845,7 @@ static int bfs_free(g500_bfs* b) {
   dev_free(b->d_ctl);
   dev_free(b->d_rec);
   dev_free(b->d_big);
+  dev_free(b->d_endw);
   if (b->h_ctl) cudaFreeHost(b->h_ctl);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
@@ -889,6 +907,8 @@ static int make_params(g500_bfs* b, int64_t root, int64_t* pred, RunParams* out)
   p.policy = b->policy;
   p.beta = b->beta;
   p.count_edges = b->count_edges;
+  p.endp = g->d_endp;
+  p.endw = nullptr;
   return G500_OK;
 }
 
@@ -928,6 +948,13 @@ extern "C" int g500_bfs_create(g500_graph* g, g500_bfs** out) {
   if (st == G500_OK) st = dev_alloc_n(&b->d_ctl, 1, "bfs control block");
   if (st == G500_OK) st = dev_alloc_n(&b->d_rec, MAX_LEVELS, "level records");
   if (st == G500_OK) st = dev_alloc_n(&b->d_big, BIG_ROWS, "long frontier rows");
+  if (st == G500_OK) st = dev_alloc_n(&b->d_endw, nwords, "endpoint counts per bitmap word");
+  if (st == G500_OK && g->nlv > 0) {
+    const unsigned wg = (unsigned)std::min<int64_t>(ceil_div(nwords * 32, 256), (int64_t)num_sms() * 8);
+    word_ends_kernel<<<wg, 256, 0, b->own_stream>>>(g->d_vis_init, g->d_endp, g->nlv / 32, b->d_endw);
+    chk(cudaGetLastError(), "endpoint counts per bitmap word");
+    chk(cudaStreamSynchronize(b->own_stream), "endpoint counts per bitmap word");
+  }
   if (st == G500_OK) chk(cudaHostAlloc(&b->h_ctl, sizeof(BfsCtl), cudaHostAllocDefault), "cudaHostAlloc");
   if (st == G500_OK) chk(cudaMemset(b->d_ctl, 0, sizeof(BfsCtl)), "cudaMemset");
   if (st == G500_OK) memset(b->h_ctl, 0, sizeof(BfsCtl));
@@ -974,14 +1001,13 @@ int bfs_launch_levels(g500_bfs* b, int64_t root, uint8_t* levels_dst) {
   cudaStream_t s = b->stream;
   RunParams p;
   G500_TRY(make_params(b, root, b->d_pred, &p));
+  p.endw = b->d_endw;
   void* args[] = {&p};
   G500_CUDA(cudaMemsetAsync(b->d_ctl, 0, sizeof(BfsCtl), s));
   G500_CUDA(cudaMemsetAsync(b->d_overflow, 0, sizeof(unsigned), s));
   G500_CUDA(cudaLaunchCooperativeKernel(bfs_kernel_for(p.deferred), dim3(b->grid), dim3(BFS_THREADS), args,
                                         0, s));
   G500_TRY(launch_deferred_pred(p, s));
-  const unsigned rg = (unsigned)std::min<int64_t>(ceil_div(std::max<int64_t>(p.nwords, 1), 256), num_sms() * 8);
-  reach_kernel<<<rg, 256, 0, s>>>(b->d_vis[0], b->d_vis[1], g->d_vis_init, g->d_endp, p.nwords, b->d_ctl);
   const unsigned lg = (unsigned)std::min<int64_t>(ceil_div(g->nolv, 256), num_sms() * 8);
   levels_from_pred_kernel<<<lg, 256, 0, s>>>(b->d_pred, g->nolv, b->d_levels, b->d_overflow);
   G500_CUDA(cudaGetLastError());
@@ -1028,8 +1054,8 @@ int bfs_complete(g500_bfs* b, int64_t* reached, int64_t* nedge) {
   if (c.bar.err & BFS_ERR_DEPTH) return set_error(G500_E_RANGE, "BFS depth exceeds the 16-bit level field");
   if (c.pad_overflow) return set_error(G500_E_RANGE, "a level over 254 does not fit the uint8 levels");
   if (c.root_has_edges) {
-    if (reached) *reached = (int64_t)c.reach[0];
-    if (nedge) *nedge = (int64_t)(c.reach[1] / 2);
+    if (reached) *reached = (int64_t)c.reached;
+    if (nedge) *nedge = (int64_t)(c.edges2 / 2);
   } else {  // a root without edges reached only itself; its self-loops are its edges
     uint32_t root_r = 0, ep = 0;
     G500_CUDA(cudaMemcpy(&root_r, b->g->d_reorder + b->last_root, sizeof(uint32_t), cudaMemcpyDeviceToHost));
@@ -1145,6 +1171,7 @@ extern "C" int g500_bfs_run(g500_bfs* b, int64_t root, int64_t* pred, int pred_o
   cudaStream_t s = b->stream;
   RunParams p;
   G500_TRY(make_params(b, root, pred_on_device ? pred : b->d_pred, &p));
+  if (stats) p.endw = b->d_endw;
   void* args[] = {&p};
   G500_CUDA(cudaMemsetAsync(b->d_ctl, 0, sizeof(BfsCtl), s));
   G500_CUDA(cudaEventRecord(b->ev0, s));
@@ -1152,11 +1179,6 @@ extern "C" int g500_bfs_run(g500_bfs* b, int64_t root, int64_t* pred, int pred_o
                                         0, s));
   G500_TRY(launch_deferred_pred(p, s));
   G500_CUDA(cudaEventRecord(b->ev1, s));
-  if (stats) {
-    const unsigned rg = (unsigned)std::min<int64_t>(ceil_div(std::max<int64_t>(p.nwords, 1), 256), num_sms() * 8);
-    reach_kernel<<<rg, 256, 0, s>>>(b->d_vis[0], b->d_vis[1], g->d_vis_init, g->d_endp, p.nwords, b->d_ctl);
-    G500_CUDA(cudaGetLastError());
-  }
   G500_CUDA(cudaMemcpyAsync(b->h_ctl, b->d_ctl, sizeof(BfsCtl), cudaMemcpyDeviceToHost, s));
   if (!pred_on_device) {
     bool packed = false;
@@ -1180,8 +1202,8 @@ extern "C" int g500_bfs_run(g500_bfs* b, int64_t root, int64_t* pred, int pred_o
     stats->device_ms = ms;
     stats->host_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     if (c.root_has_edges) {
-      stats->reached = (int64_t)c.reach[0];
-      stats->nedge = (int64_t)(c.reach[1] / 2);
+      stats->reached = (int64_t)c.reached;
+      stats->nedge = (int64_t)(c.edges2 / 2);
     } else {
       uint32_t root_r = 0, e = 0;
       G500_CUDA(cudaMemcpy(&root_r, g->d_reorder + root, sizeof(uint32_t), cudaMemcpyDeviceToHost));
@@ -1193,11 +1215,8 @@ extern "C" int g500_bfs_run(g500_bfs* b, int64_t root, int64_t* pred, int pred_o
     stats->kernel_launches = p.deferred ? 2 : 1;
     if (c.t_init_ns >= c.t0_ns) stats->init_ms = (double)(c.t_init_ns - c.t0_ns) * 1e-6;
     if (c.t_end_ns >= c.t_init_ns) stats->search_ms = (double)(c.t_end_ns - c.t_init_ns) * 1e-6;
-    if (c.num_levels) {
-      std::vector<LevelRecord> rec(c.num_levels);
-      G500_CUDA(cudaMemcpy(rec.data(), b->d_rec, sizeof(LevelRecord) * c.num_levels, cudaMemcpyDeviceToHost));
-      for (const auto& r : rec) (r.direction ? stats->td_levels : stats->bu_levels)++;
-    }
+    stats->td_levels = (int32_t)c.td_levels;
+    stats->bu_levels = (int32_t)(c.num_levels - c.td_levels);
   }
   return G500_OK;
 }

@@ -157,7 +157,9 @@ struct BfsCtl {
   unsigned long long t0_ns;
   unsigned long long t_init_ns;  // pred/visited initialised and root seeded
   unsigned long long t_end_ns;
-  unsigned long long reach[2];  // reached vertices, 2 * nedge (filled by reach_kernel)
+  unsigned long long reached;   // reached vertices
+  unsigned long long edges2;    // 2 * nedge (runs that ask for it)
+  unsigned td_levels;           // levels run top-down
   unsigned pad_overflow;        // host copy of the levels-overflow flag of an asynchronous run
 };
 
@@ -209,6 +211,7 @@ struct g500_bfs {
   BfsCtl* h_ctl = nullptr;           // pinned copy after each run
   LevelRecord* d_rec = nullptr;      // [MAX_LEVELS]
   TdItem* d_big = nullptr;           // [BIG_ROWS] long frontier rows, listed whole
+  unsigned long long* d_endw = nullptr;  // [nlv/32] endpoint occurrences per bitmap word
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   int64_t last_root = -1;
 };

@@ -64,8 +64,8 @@ size_t scan_tmp_bytes(int64_t n);
 int exclusive_scan_u32(const uint32_t* in, uint64_t* out, int64_t n, void* tmp, cudaStream_t s);
 int exclusive_scan_u64(const uint64_t* in, uint64_t* out, int64_t n, void* tmp, cudaStream_t s);
 
-// Stable LSD radix sort of 64-bit keys on bits [lo_bit, hi_bit), 8 bits a
-// pass.  Sorts keys (n) using alt (n) as the ping-pong buffer; *result is the
+// Stable LSD radix sort of 64-bit keys on bits [lo_bit, hi_bit), up to 9 bits
+// a pass.  Sorts keys (n) using alt (n) as the ping-pong buffer; *result is the
 // buffer holding the sorted keys (keys or alt).  tmp: sort_tmp_bytes(n).
 size_t sort_tmp_bytes(int64_t n);
 int radix_sort_u64(uint64_t* keys, uint64_t* alt, int64_t n, int lo_bit, int hi_bit,

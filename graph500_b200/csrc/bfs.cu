@@ -833,20 +833,12 @@ static int bfs_free(g500_bfs* b) {
   cudaSetDevice(b->g->device);
   if (b->stream) cudaStreamSynchronize(b->stream);
   pred_expander_free(b);
-  dev_free(b->d_pred);
+  dev_free(b->d_slab);
   dev_free(b->d_pred_r);
   dev_free(b->d_levels);
   dev_free(b->d_overflow);
   if (b->ev_done) cudaEventDestroy(b->ev_done);
-  dev_free(b->d_vis[0]);
-  dev_free(b->d_vis[1]);
-  dev_free(b->d_queue[0]);
-  dev_free(b->d_queue[1]);
-  dev_free(b->d_ctl);
-  dev_free(b->d_rec);
-  dev_free(b->d_big);
-  dev_free(b->d_endw);
-  if (b->h_ctl) cudaFreeHost(b->h_ctl);
+  if (b->h_ctl != &b->host_ctl) cudaFreeHost(b->h_ctl);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
   if (b->own_stream) cudaStreamDestroy(b->own_stream);
@@ -940,24 +932,25 @@ extern "C" int g500_bfs_create(g500_graph* g, g500_bfs** out) {
   b->stream = b->own_stream;
   const int64_t nwords = std::max<int64_t>(g->nlv / 32, 1);
   b->queue_cap = g->nlv + g->nge / TD_CHUNK + 1024;
-  if (st == G500_OK) st = dev_alloc_n(&b->d_pred, g->nolv, "pred");
-  if (st == G500_OK) st = dev_alloc_n(&b->d_vis[0], nwords, "visited bitmap");
-  if (st == G500_OK) st = dev_alloc_n(&b->d_vis[1], nwords, "visited bitmap");
-  if (st == G500_OK) st = dev_alloc_n(&b->d_queue[0], b->queue_cap, "top-down work items");
-  if (st == G500_OK) st = dev_alloc_n(&b->d_queue[1], b->queue_cap, "top-down discovered list");
-  if (st == G500_OK) st = dev_alloc_n(&b->d_ctl, 1, "bfs control block");
-  if (st == G500_OK) st = dev_alloc_n(&b->d_rec, MAX_LEVELS, "level records");
-  if (st == G500_OK) st = dev_alloc_n(&b->d_big, BIG_ROWS, "long frontier rows");
-  if (st == G500_OK) st = dev_alloc_n(&b->d_endw, nwords, "endpoint counts per bitmap word");
+  Slab slab;
+  slab.add(&b->d_pred, g->nolv);
+  slab.add(&b->d_vis[0], nwords);
+  slab.add(&b->d_vis[1], nwords);
+  slab.add(&b->d_queue[0], b->queue_cap);  // top-down work items
+  slab.add(&b->d_queue[1], b->queue_cap);  // top-down discovered list
+  slab.add(&b->d_ctl, 1);
+  slab.add(&b->d_rec, MAX_LEVELS);
+  slab.add(&b->d_big, BIG_ROWS);
+  slab.add(&b->d_endw, nwords);
+  if (st == G500_OK) st = slab.alloc(&b->d_slab, "pred, visited bitmaps and top-down queues");
   if (st == G500_OK && g->nlv > 0) {
     const unsigned wg = (unsigned)std::min<int64_t>(ceil_div(nwords * 32, 256), (int64_t)num_sms() * 8);
     word_ends_kernel<<<wg, 256, 0, b->own_stream>>>(g->d_vis_init, g->d_endp, g->nlv / 32, b->d_endw);
     chk(cudaGetLastError(), "endpoint counts per bitmap word");
     chk(cudaStreamSynchronize(b->own_stream), "endpoint counts per bitmap word");
   }
-  if (st == G500_OK) chk(cudaHostAlloc(&b->h_ctl, sizeof(BfsCtl), cudaHostAllocDefault), "cudaHostAlloc");
+  b->h_ctl = &b->host_ctl;
   if (st == G500_OK) chk(cudaMemset(b->d_ctl, 0, sizeof(BfsCtl)), "cudaMemset");
-  if (st == G500_OK) memset(b->h_ctl, 0, sizeof(BfsCtl));
   chk(cudaEventCreate(&b->ev0), "cudaEventCreate");
   chk(cudaEventCreate(&b->ev1), "cudaEventCreate");
   if (st == G500_OK) {
@@ -998,6 +991,12 @@ int bfs_launch_levels(g500_bfs* b, int64_t root, uint8_t* levels_dst) {
   if (!b->d_levels) G500_TRY(dev_alloc_n(&b->d_levels, std::max<int64_t>(g->nolv, 1), "levels"));
   if (!b->d_overflow) G500_TRY(dev_alloc_n(&b->d_overflow, 1, "level overflow flag"));
   if (!b->ev_done) G500_CUDA(cudaEventCreateWithFlags(&b->ev_done, cudaEventDisableTiming));
+  if (b->h_ctl == &b->host_ctl) {  // an asynchronous copy needs pinned memory
+    BfsCtl* pinned = nullptr;
+    G500_CUDA(cudaHostAlloc(&pinned, sizeof(BfsCtl), cudaHostAllocDefault));
+    *pinned = b->host_ctl;
+    b->h_ctl = pinned;
+  }
   cudaStream_t s = b->stream;
   RunParams p;
   G500_TRY(make_params(b, root, b->d_pred, &p));
@@ -1179,12 +1178,13 @@ extern "C" int g500_bfs_run(g500_bfs* b, int64_t root, int64_t* pred, int pred_o
                                         0, s));
   G500_TRY(launch_deferred_pred(p, s));
   G500_CUDA(cudaEventRecord(b->ev1, s));
-  G500_CUDA(cudaMemcpyAsync(b->h_ctl, b->d_ctl, sizeof(BfsCtl), cudaMemcpyDeviceToHost, s));
   if (!pred_on_device) {
     bool packed = false;
     G500_TRY(pred_to_host_packed(b, pred, s, &packed));
     if (!packed) G500_CUDA(cudaMemcpyAsync(pred, b->d_pred, sizeof(int64_t) * g->nolv, cudaMemcpyDeviceToHost, s));
   }
+  // last, since a copy to pageable memory waits for the run (pinned memory for it would cost 2 ms per handle)
+  G500_CUDA(cudaMemcpyAsync(b->h_ctl, b->d_ctl, sizeof(BfsCtl), cudaMemcpyDeviceToHost, s));
   G500_CUDA(cudaStreamSynchronize(s));
   b->last_root = root;
   const BfsCtl& c = *b->h_ctl;

@@ -219,27 +219,56 @@ static inline unsigned grid_for(int64_t n, int threads = 256) {
   return (unsigned)std::min<int64_t>(b, (int64_t)num_sms() * 16);
 }
 
-// Scoped device buffers freed on every exit path.
+// Scratch of a construction: one allocation for the sort's two key buffers,
+// whose memory also serves the arrays of the steps before and after the sort
+// (all on one stream).  Steps that need more than that (few edges over a large
+// id range) get an allocation of their own.  Freed on every exit path.
 struct Scratch {
-  std::vector<void*> ptrs;
+  void* ptrs[4] = {nullptr, nullptr, nullptr, nullptr};
+  int n = 0;
   ~Scratch() {
-    for (void* p : ptrs) dev_free(p);
+    for (int i = 0; i < n; ++i) dev_free(ptrs[i]);
   }
-  template <typename T>
-  int alloc(T** p, int64_t n, const char* what) {
-    G500_TRY(dev_alloc_n(p, n, what));
-    ptrs.push_back(*p);
+  int alloc(const Slab& slab, const char* what) {  // at most one per step
+    G500_TRY(slab.alloc(&ptrs[n], what));
+    ++n;
+    return G500_OK;
+  }
+  int place(const Slab& slab, void* region, size_t region_bytes, const char* what) {
+    if (slab.bytes > region_bytes) return alloc(slab, what);
+    slab.place(region);
     return G500_OK;
   }
 };
+
+int graph_alloc_maps(g500_graph* g) {
+  Slab m;
+  m.add(&g->d_reorder, g->nolv);
+  m.add(&g->d_invert, g->nolv);
+  m.add(&g->d_endp, g->nolv);
+  m.add(&g->d_offsets, g->nlv + 1);
+  m.add(&g->d_first, g->nlv);
+  m.add(&g->d_vis_init, g->nlv / 32);
+  m.add(&g->d_has_edge, g->nolv / 32);
+  return m.alloc(&g->d_maps, "reorder maps, row offsets and bitmaps");
+}
 
 int graph_destroy_internal(g500_graph* g);
 
 static int build_from_device_edges(g500_graph* g, const g500_packed_edge* d_edges, int64_t m) {
   cudaStream_t s = g->stream;
   Scratch tmp;
+  const int64_t nk = 2 * m;
   unsigned long long* d_scalars = nullptr;  // [0] or, [1] nnz, [2] last+1, [3] maxdeg
-  G500_TRY(tmp.alloc(&d_scalars, 4, "construction scalars"));
+  uint64_t *keys = nullptr, *alt = nullptr;
+  char* d_sort_tmp = nullptr;
+  Slab big;
+  big.add(&keys, nk);
+  big.add(&alt, nk);
+  const size_t both_bytes = big.bytes;  // keys and alt as one region
+  big.add(&d_sort_tmp, (int64_t)sort_tmp_bytes(INT64_MAX / 2));
+  big.add(&d_scalars, 4);
+  G500_TRY(tmp.alloc(big, "construction scratch"));
   G500_CUDA(cudaMemsetAsync(d_scalars, 0, 4 * sizeof(unsigned long long), s));
 
   // searchMaxVertex
@@ -256,8 +285,15 @@ static int build_from_device_edges(g500_graph* g, const g500_packed_edge* d_edge
 
   // degrees
   uint32_t *deg = nullptr, *sl = nullptr;
-  G500_TRY(tmp.alloc(&deg, nolv, "degree"));
-  G500_TRY(tmp.alloc(&sl, nolv, "self loops"));
+  uint64_t *k = nullptr, *k2 = nullptr;
+  Slab verts;
+  verts.add(&deg, nolv);
+  verts.add(&sl, nolv);
+  if (g->reorder_mode != 0) {
+    verts.add(&k, nolv);
+    verts.add(&k2, nolv);
+  }
+  G500_TRY(tmp.place(verts, keys, both_bytes, "degrees and reorder keys"));
   G500_CUDA(cudaMemsetAsync(deg, 0, sizeof(uint32_t) * nolv, s));
   G500_CUDA(cudaMemsetAsync(sl, 0, sizeof(uint32_t) * nolv, s));
   degree_kernel<<<grid_for(m), 256, 0, s>>>(d_edges, m, deg, sl);
@@ -271,67 +307,46 @@ static int build_from_device_edges(g500_graph* g, const g500_packed_edge* d_edge
   const int64_t nnz = (int64_t)sc[1];
   const unsigned maxdeg = (unsigned)(sc[3] & 0xFFFFFFFFu);
   g->ngv = nnz;
-
-  // vertex reordering (calc_degree)
-  G500_TRY(dev_alloc_n(&g->d_reorder, nolv, "reorder_map"));
-  G500_TRY(dev_alloc_n(&g->d_invert, nolv, "invert_map"));
-  const size_t sort_tmp = sort_tmp_bytes(std::max<int64_t>(nolv, 2 * m));
-  void* d_sort_tmp = nullptr;
-  G500_TRY(tmp.alloc(reinterpret_cast<char**>(&d_sort_tmp), (int64_t)sort_tmp, "sort scratch"));
-  if (g->reorder_mode == 0) {
-    maps_from_keys_kernel<<<grid_for(nolv), 256, 0, s>>>(nullptr, nolv, g->d_invert, g->d_reorder);
-  } else {
-    uint64_t *k = nullptr, *k2 = nullptr, *sorted = nullptr;
-    G500_TRY(tmp.alloc(&k, nolv, "reorder keys"));
-    G500_TRY(tmp.alloc(&k2, nolv, "reorder keys (alt)"));
-    reorder_keys_kernel<<<grid_for(nolv), 256, 0, s>>>(deg, nolv, g->reorder_mode, maxdeg, k);
-    G500_CUDA(cudaGetLastError());
-    int hi = 32 + (g->reorder_mode == 2 ? std::max(1, bits_for((uint64_t)maxdeg + 1)) : 1);
-    G500_TRY(radix_sort_u64(k, k2, nolv, 32, hi, d_sort_tmp, s, &sorted));
-    maps_from_keys_kernel<<<grid_for(nolv), 256, 0, s>>>(sorted, nolv, g->d_invert, g->d_reorder);
-  }
-  G500_CUDA(cudaGetLastError());
   const int64_t last_plus1 = (g->reorder_mode == 0) ? (int64_t)sc[2] : nnz;
   g->nlv = roundup(last_plus1, LOCAL_VERTS_UNIT);
   const int64_t nlv = g->nlv;
   const int lb = std::max(1, bits_for((uint64_t)std::max<int64_t>(nlv, 1)));
   g->log_bits = lb;
+  G500_TRY(graph_alloc_maps(g));
 
-  G500_TRY(dev_alloc_n(&g->d_endp, nolv, "endpoint counts"));
+  // vertex reordering (calc_degree)
+  if (g->reorder_mode == 0) {
+    maps_from_keys_kernel<<<grid_for(nolv), 256, 0, s>>>(nullptr, nolv, g->d_invert, g->d_reorder);
+  } else {
+    uint64_t* sorted_v = nullptr;
+    reorder_keys_kernel<<<grid_for(nolv), 256, 0, s>>>(deg, nolv, g->reorder_mode, maxdeg, k);
+    G500_CUDA(cudaGetLastError());
+    int hi = 32 + (g->reorder_mode == 2 ? std::max(1, bits_for((uint64_t)maxdeg + 1)) : 1);
+    G500_TRY(radix_sort_u64(k, k2, nolv, 32, hi, d_sort_tmp, s, &sorted_v));
+    maps_from_keys_kernel<<<grid_for(nolv), 256, 0, s>>>(sorted_v, nolv, g->d_invert, g->d_reorder);
+  }
+  G500_CUDA(cudaGetLastError());
   endp_kernel<<<grid_for(nolv), 256, 0, s>>>(deg, sl, g->d_invert, nolv, g->d_endp);
   G500_CUDA(cudaGetLastError());
-
-  // host bitmap of has_edge over original ids
-  uint32_t* d_hbits = nullptr;
-  G500_TRY(tmp.alloc(&d_hbits, nolv / 32, "has_edge bitmap"));
-  has_edge_orig_kernel<<<grid_for(nolv), 256, 0, s>>>(deg, nolv, d_hbits);
+  has_edge_orig_kernel<<<grid_for(nolv), 256, 0, s>>>(deg, nolv, g->d_has_edge);
   G500_CUDA(cudaGetLastError());
-  g->h_has_edge_orig.assign((size_t)(nolv / 32), 0u);
-  G500_CUDA(cudaMemcpyAsync(g->h_has_edge_orig.data(), d_hbits, sizeof(uint32_t) * (nolv / 32),
-                            cudaMemcpyDeviceToHost, s));
 
-  // CSR: keys for both directions, sort, drop duplicates
-  G500_TRY(dev_alloc_n(&g->d_offsets, nlv + 1, "row offsets"));
-  G500_TRY(dev_alloc_n(&g->d_first, nlv, "first neighbours"));
-  G500_TRY(dev_alloc_n(&g->d_vis_init, std::max<int64_t>(nlv / 32, 1), "visited init bitmap"));
-  const int64_t nk = 2 * m;
-  uint64_t *keys = nullptr, *alt = nullptr, *sorted = nullptr;
-  G500_TRY(tmp.alloc(&keys, nk, "edge keys"));
-  G500_TRY(tmp.alloc(&alt, nk, "edge keys (alt)"));
+  // CSR: keys for both directions (over the degrees' memory), sort, drop duplicates
+  uint64_t* sorted = nullptr;
   edge_keys_kernel<<<grid_for(m), 256, 0, s>>>(d_edges, m, g->d_reorder, lb, keys);
   G500_CUDA(cudaGetLastError());
   G500_TRY(radix_sort_u64(keys, alt, nk, 0, 2 * lb, d_sort_tmp, s, &sorted));
-  uint32_t* rowcnt = nullptr;
-  G500_TRY(tmp.alloc(&rowcnt, nlv + 1, "row lengths"));
-  G500_CUDA(cudaMemsetAsync(rowcnt, 0, sizeof(uint32_t) * (nlv + 1), s));
   const int64_t ntiles = ceil_div(std::max<int64_t>(nk, 1), CP_TILE);
-  uint32_t* tile_counts = nullptr;
+  uint32_t *rowcnt = nullptr, *tile_counts = nullptr;
   uint64_t* tile_offsets = nullptr;
-  G500_TRY(tmp.alloc(&tile_counts, ntiles, "tile counts"));
-  G500_TRY(tmp.alloc(&tile_offsets, ntiles + 1, "tile offsets"));
-  void* scan_tmp = nullptr;
-  G500_TRY(tmp.alloc(reinterpret_cast<char**>(&scan_tmp), (int64_t)scan_tmp_bytes(std::max(ntiles, nlv + 1)),
-                     "scan scratch"));
+  char* scan_tmp = nullptr;
+  Slab rows;  // over the buffer that does not hold the sorted keys
+  rows.add(&rowcnt, nlv + 1);
+  rows.add(&tile_counts, ntiles);
+  rows.add(&tile_offsets, ntiles + 1);
+  rows.add(&scan_tmp, (int64_t)scan_tmp_bytes(std::max(ntiles, nlv + 1)));
+  G500_TRY(tmp.place(rows, sorted == keys ? alt : keys, sizeof(uint64_t) * (size_t)nk, "row lengths"));
+  G500_CUDA(cudaMemsetAsync(rowcnt, 0, sizeof(uint32_t) * (nlv + 1), s));
   if (nk > 0) {
     unique_count_kernel<<<(unsigned)ntiles, CP_THREADS, 0, s>>>(sorted, nk, lb, tile_counts, rowcnt);
     G500_CUDA(cudaGetLastError());
@@ -353,6 +368,10 @@ static int build_from_device_edges(g500_graph* g, const g500_packed_edge* d_edge
                                                      g->d_first, g->d_vis_init);
     G500_CUDA(cudaGetLastError());
   }
+  // host bitmap of has_edge over original ids
+  g->h_has_edge_orig.assign((size_t)(nolv / 32), 0u);
+  G500_CUDA(cudaMemcpyAsync(g->h_has_edge_orig.data(), g->d_has_edge, sizeof(uint32_t) * (nolv / 32),
+                            cudaMemcpyDeviceToHost, s));
   G500_CUDA(cudaStreamSynchronize(s));
 
   // find_max_used_vertex (benchmark_helper.hpp:510-528) on the host bitmap
@@ -391,13 +410,9 @@ int graph_destroy_internal(g500_graph* g) {
   if (!g) return G500_OK;
   cudaSetDevice(g->device);
   if (g->stream) cudaStreamSynchronize(g->stream);
-  dev_free(g->d_offsets);
+  dev_free(g->d_maps);
+  dev_free(g->d_val);
   dev_free(g->d_cols);
-  dev_free(g->d_first);
-  dev_free(g->d_reorder);
-  dev_free(g->d_invert);
-  dev_free(g->d_vis_init);
-  dev_free(g->d_endp);
   if (g->owns_edges) dev_free(g->d_edges);
   if (g->stream) cudaStreamDestroy(g->stream);
   delete g;

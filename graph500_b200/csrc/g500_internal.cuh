@@ -57,6 +57,33 @@ int dev_alloc_n(T** p, int64_t n, const char* what) {
 }
 void dev_free(void* p);
 
+// Several arrays cut from one device allocation.  A cudaMalloc costs about 0.4
+// ms and a cudaFree 0.3 ms whatever their size below 256 MB, which for the two
+// dozen arrays of a graph's construction was half of its time at SCALE 22.
+struct Slab {
+  static constexpr int MAX = 24;
+  struct Part {
+    void** p;
+    size_t off;
+  } parts[MAX];
+  int n = 0;
+  size_t bytes = 0;
+  template <typename T>
+  void add(T** p, int64_t count) {  // at most MAX parts, a fixed list per slab
+    parts[n].p = reinterpret_cast<void**>(p);
+    parts[n++].off = bytes;
+    bytes += (sizeof(T) * (size_t)(count > 0 ? count : 1) + 255) & ~size_t(255);
+  }
+  void place(void* base) const {  // base: 256-byte aligned, `bytes` long
+    for (int i = 0; i < n; ++i) *parts[i].p = static_cast<char*>(base) + parts[i].off;
+  }
+  int alloc(void** base, const char* what) const {
+    G500_TRY(dev_alloc(base, bytes, what));
+    place(*base);
+    return G500_OK;
+  }
+};
+
 // ------------------------------------------------------------- primitives
 // Exclusive prefix sum of n values (uint32 or uint64 input) into uint64
 // out[0..n]; out[n] = total.  tmp: scan_tmp_bytes(n) bytes of device memory.
@@ -104,6 +131,8 @@ struct g500_graph {
   int64_t device_bytes = 0;
   double gen_seconds = 0, build_seconds = 0;
 
+  void* d_maps = nullptr;           // the allocation of every array below but cols and edges
+  void* d_val = nullptr;            // the validator's scratch, kept once a call has needed it
   uint64_t* d_offsets = nullptr;    // [nlv + 1]
   uint32_t* d_cols = nullptr;       // [nge]   reordered targets, ascending per row
   uint32_t* d_first = nullptr;      // [nlv]   first (smallest) neighbour (| FIRST_MORE) or NO_VERTEX
@@ -112,6 +141,7 @@ struct g500_graph {
   uint32_t* d_invert = nullptr;     // [nolv]  reordered -> original
   uint32_t* d_vis_init = nullptr;   // [nlv/32] ~has_edge in reordered space
   uint32_t* d_endp = nullptr;       // [nolv]  input endpoint occurrences per reordered vertex
+  uint32_t* d_has_edge = nullptr;   // [nolv/32] has-edge bitmap over original ids (construction)
   g500_packed_edge* d_edges = nullptr;  // resident input edge list (optional)
   int64_t num_edges = 0;
   bool owns_edges = false;
@@ -187,6 +217,7 @@ struct g500_bfs {
   int count_edges = 0;
   unsigned grid = 0;                 // co-resident blocks of the persistent kernel
 
+  void* d_slab = nullptr;            // the allocation of pred, vis, queue, ctl, rec, big and endw
   int64_t* d_pred = nullptr;         // [nolv]
   int64_t* d_pred_r = nullptr;       // [nlv] deferred mode: pred entries by reordered id
   uint8_t* d_levels = nullptr;       // [nolv] levels of an asynchronous run (serving)
@@ -208,7 +239,8 @@ struct g500_bfs {
   TdItem* d_queue[2] = {nullptr, nullptr};
   int64_t queue_cap = 0;
   BfsCtl* d_ctl = nullptr;
-  BfsCtl* h_ctl = nullptr;           // pinned copy after each run
+  BfsCtl* h_ctl = nullptr;           // copy after each run: &host_ctl, or pinned once a run was asynchronous
+  BfsCtl host_ctl = {};
   LevelRecord* d_rec = nullptr;      // [MAX_LEVELS]
   TdItem* d_big = nullptr;           // [BIG_ROWS] long frontier rows, listed whole
   unsigned long long* d_endw = nullptr;  // [nlv/32] endpoint occurrences per bitmap word
@@ -240,4 +272,6 @@ namespace g500 {
 // An empty graph handle on `device` with its own stream (build.cu).
 int new_graph(int device, int reorder_mode, g500_graph** out);
 int graph_destroy_internal(g500_graph* g);
+// The graph's arrays but cols and edges, once nolv and nlv are known (build.cu).
+int graph_alloc_maps(g500_graph* g);
 }  // namespace g500

@@ -1261,6 +1261,7 @@ struct g500_msbfs {
   int count = 0;                    // counting launches (no CUDA graph): per-level offset reads and sectors
   unsigned grid[3] = {0, 0, 0};     // co-resident blocks per lane width (NW = 1, 2, 4)
 
+  void* slab = nullptr;             // the allocation of the arrays below but the hub tables
   uint32_t *V = nullptr, *F = nullptr, *N = nullptr;  // [nlv][4] words (room for 128 lanes)
   uint8_t* L = nullptr;                               // [nlv][128]
   uint8_t* out = nullptr;                             // [128][nolv]
@@ -1308,20 +1309,10 @@ static int ms_free(g500_msbfs* m) {
   cudaSetDevice(m->g->device);
   if (m->stream) cudaStreamSynchronize(m->stream);
   ms_drop_graphs(m);
-  dev_free(m->V);
-  dev_free(m->F);
-  dev_free(m->N);
-  dev_free(m->L);
-  dev_free(m->out);
-  dev_free(m->ctl);
-  dev_free(m->roots_dev);
-  dev_free(m->nroots_dev);
-  dev_free(m->stats_dev);
-  dev_free(m->deg);
+  dev_free(m->slab);
   dev_free(m->hub_tab);
   dev_free(m->hub_rows);
   dev_free(m->push_tab);
-  dev_free(m->marks);
   if (m->staging) cudaFreeHost(m->staging);
   if (m->h_ctl) cudaFreeHost(m->h_ctl);
   if (m->h_stats) cudaFreeHost(m->h_stats);
@@ -1476,28 +1467,30 @@ extern "C" int g500_msbfs_create(g500_graph* g, g500_msbfs** out) {
   };
   chk(cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking), "cudaStreamCreate");
   const int64_t nlv = std::max<int64_t>(g->nlv, 1);
-  if (st == G500_OK) st = dev_alloc_n(&m->V, nlv * 4, "msbfs visited masks");
-  if (st == G500_OK) st = dev_alloc_n(&m->F, 2 * nlv * 4, "msbfs frontier masks");
-  if (st == G500_OK) st = dev_alloc_n(&m->N, nlv * 4, "msbfs next masks");
-  if (st == G500_OK) st = dev_alloc_n(&m->L, nlv * MS_MAX_LANES, "msbfs levels");
-  if (st == G500_OK) st = dev_alloc_n(&m->deg, nlv, "msbfs row lengths");
   // sparse levels: frontier and touched bitmaps; from 2^22 vertices with
   // edges, a push level is sparse up to a last-frontier degree sum of nlv / 8
   // (on smaller graphs a pass over every vertex costs less than the sparse
   // level's extra steps)
   m->nwords = (nlv + 31) / 32;
   m->sparse_limit = nlv >= (int64_t(1) << 22) ? nlv / 8 : -1;
-  if (st == G500_OK) st = dev_alloc_n(&m->marks, 4 * m->nwords, "msbfs frontier and touched bitmaps");
+  Slab slab;
+  slab.add(&m->V, nlv * 4);                 // visited masks
+  slab.add(&m->F, 2 * nlv * 4);             // frontier masks
+  slab.add(&m->N, nlv * 4);                 // next masks
+  slab.add(&m->L, nlv * MS_MAX_LANES);      // levels
+  slab.add(&m->deg, nlv);                   // row lengths
+  slab.add(&m->marks, 4 * m->nwords);       // frontier and touched bitmaps
+  slab.add(&m->out, (int64_t)MS_MAX_LANES * g->nolv);  // output levels
+  slab.add(&m->ctl, 4);
+  slab.add(&m->roots_dev, 4 * MS_MAX_LANES);
+  slab.add(&m->nroots_dev, 4);
+  slab.add(&m->stats_dev, 2 * MS_MAX_LANES);
+  if (st == G500_OK) st = slab.alloc(&m->slab, "multi-source masks and levels");
   if (st == G500_OK && g->nlv > 0) {
     const unsigned dgrid = (unsigned)std::min<int64_t>(ceil_div(g->nlv, 256), (int64_t)num_sms() * 8);
     ms_degree_kernel<<<dgrid, 256, 0, m->stream>>>(g->d_offsets, g->nlv, m->deg);
     chk(cudaGetLastError(), "row lengths");
   }
-  if (st == G500_OK) st = dev_alloc_n(&m->out, (int64_t)MS_MAX_LANES * g->nolv, "msbfs output levels");
-  if (st == G500_OK) st = dev_alloc_n(&m->ctl, 4, "msbfs control");
-  if (st == G500_OK) st = dev_alloc_n(&m->roots_dev, 4 * MS_MAX_LANES, "msbfs roots");
-  if (st == G500_OK) st = dev_alloc_n(&m->nroots_dev, 4, "msbfs root counts");
-  if (st == G500_OK) st = dev_alloc_n(&m->stats_dev, 2 * MS_MAX_LANES, "msbfs stats");
   if (st == G500_OK)
     chk(cudaHostAlloc(&m->staging, sizeof(int64_t) * (4 * MS_MAX_LANES + 4), cudaHostAllocDefault), "cudaHostAlloc");
   if (st == G500_OK) chk(cudaHostAlloc(&m->h_ctl, sizeof(MsCtl) * 4, cudaHostAllocDefault), "cudaHostAlloc");

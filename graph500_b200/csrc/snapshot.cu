@@ -159,13 +159,8 @@ extern "C" int g500_graph_load(const char* path, int device, g500_graph** out) {
   g->device_bytes = h.device_bytes;
   g->gen_seconds = h.gen_seconds;
   g->build_seconds = h.build_seconds;
-  int st = dev_alloc_n(&g->d_offsets, h.nlv + 1, "offsets");
+  int st = graph_alloc_maps(g);
   if (st == G500_OK) st = dev_alloc_n(&g->d_cols, std::max<int64_t>(h.nge, 1), "cols");
-  if (st == G500_OK) st = dev_alloc_n(&g->d_first, std::max<int64_t>(h.nlv, 1), "first neighbours");
-  if (st == G500_OK) st = dev_alloc_n(&g->d_reorder, std::max<int64_t>(h.nolv, 1), "reorder_map");
-  if (st == G500_OK) st = dev_alloc_n(&g->d_invert, std::max<int64_t>(h.nolv, 1), "invert_map");
-  if (st == G500_OK) st = dev_alloc_n(&g->d_vis_init, std::max<int64_t>(h.nlv / 32, 1), "visited init bitmap");
-  if (st == G500_OK) st = dev_alloc_n(&g->d_endp, std::max<int64_t>(h.nolv, 1), "endpoint counts");
   if (st == G500_OK && h.num_edges > 0) {
     st = dev_alloc_n(&g->d_edges, h.num_edges, "edge list");
     g->owns_edges = true;

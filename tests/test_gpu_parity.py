@@ -80,6 +80,28 @@ def test_csr_bit_exact(g500, oracle_mod, scale, vr):
     dg.close()
 
 
+@pytest.mark.parametrize("m", [1, 2, 31, 4095, 4096, 4097, 12289, 296 * 4096 + 3])
+@pytest.mark.parametrize("vr", [0, 1, 2])
+def test_csr_sort_tiles_and_scratch(g500, oracle_mod, vr, m):
+    """Key counts around the sort's tiles (8192 keys, two per edge) and its blocks' ranges, with skewed ids,
+    duplicates and self loops; the smallest lists leave the sort less memory than the vertex arrays need."""
+    rng = np.random.default_rng(m)
+    ids = np.minimum(rng.integers(0, 1 << 17, (m, 2)), rng.integers(0, 1 << 17, (m, 2)))
+    ids = np.where(rng.random((m, 2)) < 0.5, ids >> 9, ids)
+    edges = np.zeros(m, g500.EDGE_DTYPE)
+    edges["v0_low"], edges["v1_low"] = ids[:, 0], ids[:, 1]
+    og = oracle_mod.Graph(edges, vr)
+    dg = g500.Graph2DCSR.build(edges, vr)
+    info = dg.info
+    assert [info.log_orig_global_verts, info.pred_size, info.num_local_verts, info.num_global_verts,
+            info.num_global_edges, info.max_used_vertex] == list(og.info.values())
+    csr = dg.copy_csr()
+    assert np.array_equal(csr["offsets"], og.offsets)
+    assert np.array_equal(csr["cols"], og.cols)
+    assert np.array_equal(csr["reorder_map"], og.reorder_map)
+    dg.close()
+
+
 @pytest.mark.parametrize("scale,vr", GOLDEN_CASES)
 def test_graph_info_and_roots_match_reference(g500, scale, vr):
     rec, _ = load_golden(scale, vr)

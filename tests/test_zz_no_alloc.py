@@ -86,3 +86,39 @@ def test_noalloc_refuses_buffers_off_the_current_device(g500):
     rc = L.g500_validate_noalloc(None, 0, 1, 64, 0, host_pred.ctypes.data, None, C.byref(evc), C.byref(ok), None)
     assert rc == g500.G500_E_INVAL
     assert b"device memory" in L.g500_last_error()
+
+
+@pytest.mark.parametrize("planted", ["none", "level", "deep", "deepest", "self", "range", "negative", "half_reached",
+                                     "unreached"])
+@pytest.mark.parametrize("skip,drop", [(0, 0), (1, 0), (2, 1), (3, 2), (4, 3)])
+def test_packed_and_unpacked_validation_report_alike(g500, planted, skip, drop):
+    """g500_validate reads packed entries where they fit, g500_validate_noalloc always pred itself: every count
+    must agree, on valid and planted results, for edge lists at every 12-byte alignment and remainder of four."""
+    import torch
+
+    bfs = g500.BfsOnGPU(reorder_mode=2)
+    bfs.construct(g500.EdgeList(None, 12, 16))
+    bfs.prepare_bfs()
+    g = bfs.graph_
+    root = int(g500.find_roots(g, 1)[0])
+    pred = np.zeros(g.pred_size(), np.int64)
+    bfs.run_bfs(root, pred)
+    reached = np.nonzero((pred != -1) & (np.arange(len(pred)) != root))[0]
+    v, w = (int(x) for x in reached[[len(reached) // 3, len(reached) // 2]])
+    parent, level = int(pred[v]) & 0xFFFFFFFFFFFF, int(pred[v]) >> 48
+    pred[v] = {"none": pred[v], "level": parent | (level + 1) << 48, "deep": parent | 30 << 48,
+               "deepest": parent | 31 << 48, "self": v | level << 48, "range": 1 << 30 | level << 48,
+               "negative": -2, "half_reached": 0xFFFFFFFFFFFF | level << 48, "unreached": -1}[planted]
+    if planted == "deep":
+        pred[w] = ((1 << 27) - 1) | 30 << 48  # the largest packed entry
+    dev = torch.from_numpy(pred).cuda()
+    eptr, m = g.device_edges()
+    ptr, n = eptr + 12 * skip, m - skip - drop
+    evc, ok, rep = C.c_int64(), C.c_int(), g500.ValidateReport()
+    g500.check(g500.lib().g500_validate(g.h, ptr, n, 1, root, dev.data_ptr(), 1, C.byref(evc), C.byref(ok),
+                                        C.byref(rep)))
+    want = _noalloc(g500, ptr, n, g.info.max_used_vertex + 1, g.pred_size(), root, dev)
+    assert (bool(ok.value), evc.value, {f[0]: getattr(rep, f[0]) for f in g500.ValidateReport._fields_}) == want
+    if planted not in ("none",):
+        assert not ok.value
+    bfs.close()

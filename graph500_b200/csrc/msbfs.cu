@@ -838,6 +838,7 @@ __device__ void ms_settle_hubs(const MsParams& p, const Mask<NW>& act, uint32_t*
 constexpr int MS_SURVEY_STEP = 8;
 constexpr int MS_SURVEY_DIV = 64;  // a lane is pushed when its frontier degree sum is under entries / this
 constexpr int MS_SURVEY_LEVELS = 1;  // pull levels that survey (the first ones)
+static_assert(MS_SURVEY_LEVELS == 1, "the lanes' sums are cleared once per launch");
 template <int NW>
 __device__ void ms_lane_survey(const MsParams& p, const uint32_t* Fc, unsigned long long* sh_lane) {
   const int lane = threadIdx.x & 31;
@@ -1044,13 +1045,14 @@ __global__ void __launch_bounds__(MS_THREADS, MS_MIN_BLOCKS) msbfs_kernel(MsPara
       if (sparse) ms_clear_marked<NW>(p, Fn, level > 1 ? p.fb[(level - 2) % 3] : nullptr, la.fb);
     }
     pulls += pull;
-    if (!grid_sync<M_NUM>(&ctl->bar, nullptr, sh_acc, nullptr, sh_cnt, &sh_flag)) return;
-    if (tid == 0) ctl->level_mid_ns[level] = globaltimer();
-    // every block read the survey's sums before this barrier; the next
-    // survey adds after the level's closing one
-    if (survey && blockIdx.x == 0)
-      for (int i = threadIdx.x; i < MS_MAX_LANES; i += blockDim.x) ctl->lane_deg[i] = 0;
-    if (pull && !mixed) ms_settle_hubs<NW, SP>(p, act, Fn, lvl4, la);
+    // Rows that pull settle themselves; without hub rows (none under 2^20
+    // entries) such a level has nothing left to wait for.  At SCALE 18 the
+    // barrier and the empty pass were 4 of a pull level's 9-13 us.
+    const bool settled = pull && !mixed && p.nhubs == 0;
+    if (!settled && !grid_sync<M_NUM>(&ctl->bar, nullptr, sh_acc, nullptr, sh_cnt, &sh_flag)) return;
+    if (tid == 0 && !settled) ctl->level_mid_ns[level] = globaltimer();
+    if (settled) {
+    } else if (pull && !mixed) ms_settle_hubs<NW, SP>(p, act, Fn, lvl4, la);
     else if (sparse) ms_apply_marked<NW>(p, act, Fn, lvl4, la);
     else ms_apply<NW, SP>(p, act, Fn, lvl4, la);
     flush_level<NW, COUNT>(la, sh_acc, sh_or, alive);
@@ -1060,6 +1062,7 @@ __global__ void __launch_bounds__(MS_THREADS, MS_MIN_BLOCKS) msbfs_kernel(MsPara
     if (tid == 0) {
       ctl->level_new[level] = nnew;
       ctl->level_t_ns[level] = globaltimer();
+      if (settled) ctl->level_mid_ns[level] = ctl->level_t_ns[level];
       ctl->level_pull[level] = pull ? (mixed ? 2 : 1) : 0;
       if constexpr (COUNT) {
         ctl->level_rows[level] = sh_cnt[M_ROWS];

@@ -64,7 +64,7 @@ struct MsParams {
   uint32_t* V;
   uint32_t* F[2];            // frontier masks by level parity: level l reads F[(l - 1) & 1], writes F[l & 1]
   uint32_t* N;
-  uint8_t* L;                // [nlv][W] levels, 255 unreached
+  uint4* L;                  // [2][nlv][W / 32] level bit planes (see write_levels)
   const int64_t* roots;      // [nroots] original ids (device)
   const int* nroots_dev;     // number of roots of this launch (device, set with the roots)
   const uint2* hub_tab;      // pull: [nhub_chunks] (hub row, chunk index within the row)
@@ -169,33 +169,40 @@ constexpr int MS_PUSH_HUB_DEG = 256;   // push: the same two, smaller: a push wa
 constexpr int MS_PUSH_CHUNK = 256;     //   frontier rows, so short chunks spread the few hub rows wider
 
 
-// byte mask of the 4 lanes whose bits are set in nib (bit i -> byte i)
-__device__ __forceinline__ uint32_t nibble_bytes(uint32_t nib) {
-  return ((nib * 0x00204081u) & 0x01010101u) * 0xFFu;
-}
-
-// level bytes of a row: for each 16-lane group with new lanes, write the
-// group's 16 bytes (new lanes = level, unvisited lanes = 255, lanes visited
-// before keep their byte, read back only when the group has such lanes).
-// Groups without visited lanes are never written; the output pass reads
-// them as 255 from the visited mask.
+// Levels are kept as bit planes: per vertex and 32 lanes one uint4 whose words
+// hold bits 0 .. 3 of the lanes' levels, and for levels from 16 a second array
+// with bits 4 .. 7 (zeroed by every block at level 15, so shallow launches never
+// touch it).  New lanes OR their level's bits in; a group whose vertex had no
+// visited lane among its 32 is written whole, so nothing is cleared up front
+// (groups without visited lanes are never written, and the output pass reads
+// none).  16 bytes per 32 lanes instead of the 32 of a byte per lane, which a
+// dense level rewrites for nearly every vertex.  SCALE 24, 64 lanes: level 4 454
+// -> 303 us, the output pass 535 -> 384 us, a launch 2870 -> 2316 us.
+constexpr uint32_t MS_PLANE_LEVELS = 16;
 template <int NW>
-__device__ __forceinline__ void write_levels(uint8_t* row, const Mask<NW>& nw, const Mask<NW>& vv, uint32_t lvl4) {
+__device__ __forceinline__ void write_levels(const MsParams& p, int64_t v, const Mask<NW>& nw, const Mask<NW>& vv,
+                                             uint32_t level) {
 #pragma unroll
-  for (int g = 0; g < 2 * NW; ++g) {
-    const uint32_t bits = (nw.w[g >> 1] >> ((g & 1) * 16)) & 0xFFFFu;
-    if (!bits) continue;
-    const uint32_t old = (vv.w[g >> 1] >> ((g & 1) * 16)) & 0xFFFFu;
-    uint4* dst = reinterpret_cast<uint4*>(row) + g;
-    uint4 o = make_uint4(~0u, ~0u, ~0u, ~0u);
-    if (old) o = __ldcg(dst);
-    uint32_t w[4] = {o.x, o.y, o.z, o.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t bm = nibble_bytes((bits >> (4 * i)) & 0xFu);
-      w[i] = (w[i] & ~bm) | (lvl4 & bm);
+  for (int k = 0; k < NW; ++k) {
+    const uint32_t x = nw.w[k];
+    if (!x) continue;
+    uint4* dst = p.L + v * NW + k;
+    uint4 o = make_uint4(0, 0, 0, 0);
+    if (vv.w[k]) o = __ldcg(dst);
+    o.x |= (level & 1u) ? x : 0u;
+    o.y |= (level & 2u) ? x : 0u;
+    o.z |= (level & 4u) ? x : 0u;
+    o.w |= (level & 8u) ? x : 0u;
+    *dst = o;
+    if (level >= MS_PLANE_LEVELS) {
+      uint4* hi = p.L + (p.nlv + v) * NW + k;
+      uint4 h = __ldcg(hi);
+      h.x |= (level & 16u) ? x : 0u;
+      h.y |= (level & 32u) ? x : 0u;
+      h.z |= (level & 64u) ? x : 0u;
+      h.w |= (level & 128u) ? x : 0u;
+      *hi = h;
     }
-    *dst = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
 
@@ -226,9 +233,8 @@ struct LevelAcc {
 // Returns whether v found lanes (then it is marked in the level's frontier bitmap).
 template <int NW>
 __device__ __forceinline__ bool settle(const MsParams& p, uint32_t* Fn, int64_t v, const Mask<NW>& vv,
-                                       const Mask<NW>& need, const Mask<NW>& nw, uint32_t deg, uint32_t lvl4,
+                                       const Mask<NW>& need, const Mask<NW>& nw, uint32_t deg, uint32_t level,
                                        LevelAcc<NW>& a) {
-  constexpr int W = 32 * NW;
   store_mask<NW>(Fn + v * NW, nw);
   bool anynew = false, left = false;
 #pragma unroll
@@ -241,7 +247,7 @@ __device__ __forceinline__ bool settle(const MsParams& p, uint32_t* Fn, int64_t 
 #pragma unroll
     for (int k = 0; k < NW; ++k) vn.w[k] = vv.w[k] | nw.w[k];
     store_mask<NW>(p.V + v * NW, vn);
-    write_levels<NW>(p.L + v * W, nw, vv, lvl4);
+    write_levels<NW>(p, v, nw, vv, level);
 #pragma unroll
     for (int k = 0; k < NW; ++k) {
       a.lanes.w[k] |= nw.w[k];
@@ -267,7 +273,7 @@ __device__ __forceinline__ bool settle(const MsParams& p, uint32_t* Fn, int64_t 
 // settle, instead of settling here.
 template <int NW, bool INTO_N, bool COUNT, bool SP>
 __device__ void ms_pull_rows(const MsParams& p, const Mask<NW>& act, const uint32_t* Fc, uint32_t* Fn,
-                             uint32_t lvl4, LevelAcc<NW>& la) {
+                             uint32_t level, LevelAcc<NW>& la) {
   const int lane = threadIdx.x & 31;
   for (int64_t base = gwarp_id() * 32; base < p.nlv; base += gwarp_count() * 32) {
     const int64_t v = base + lane;
@@ -368,7 +374,7 @@ __device__ void ms_pull_rows(const MsParams& p, const Mask<NW>& act, const uint3
         for (int k = 0; k < NW; ++k)
           if (nw.w[k]) atomicOr(p.N + v * NW + k, nw.w[k]);
       } else {
-        app = settle<NW>(p, Fn, v, vv, need, nw, deg, lvl4, la);
+        app = settle<NW>(p, Fn, v, vv, need, nw, deg, level, la);
       }
     }
     if constexpr (SP && !INTO_N) {  // the warp's 32 vertices are one word of the frontier bitmap
@@ -682,7 +688,7 @@ __device__ void ms_push_rows_marked(const MsParams& p, const uint32_t* Fc, const
 // loads first; each warp's 32 vertices of a step are one word of the
 // frontier bitmap.
 template <int NW, bool SP>
-__device__ void ms_apply(const MsParams& p, const Mask<NW>& act, uint32_t* Fn, uint32_t lvl4, LevelAcc<NW>& la) {
+__device__ void ms_apply(const MsParams& p, const Mask<NW>& act, uint32_t* Fn, uint32_t level, LevelAcc<NW>& la) {
   constexpr int U = NW == 4 ? 2 : 4;
   const int lane = threadIdx.x & 31;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -723,7 +729,7 @@ __device__ void ms_apply(const MsParams& p, const Mask<NW>& act, uint32_t* Fn, u
           for (int k = 0; k < NW; ++k) zero.w[k] = 0;
           store_mask<NW>(p.N + v * NW, zero);
         }
-        app = settle<NW>(p, Fn, v, vv[u], need, nw, dg[u], lvl4, la);
+        app = settle<NW>(p, Fn, v, vv[u], need, nw, dg[u], level, la);
       }
       if constexpr (SP) {
         const unsigned word = __ballot_sync(FULL_MASK, app);
@@ -742,7 +748,7 @@ __device__ void ms_apply(const MsParams& p, const Mask<NW>& act, uint32_t* Fn, u
 // sum of vertices with needed lanes left, is not summed here (the caller
 // keeps the last one).
 template <int NW>
-__device__ void ms_apply_marked(const MsParams& p, const Mask<NW>& act, uint32_t* Fn, uint32_t lvl4,
+__device__ void ms_apply_marked(const MsParams& p, const Mask<NW>& act, uint32_t* Fn, uint32_t level,
                                 LevelAcc<NW>& la) {
   const int lane = threadIdx.x & 31;
   for (int64_t wb = gwarp_id() * 32; wb < p.nwords; wb += gwarp_count() * 32) {
@@ -770,7 +776,7 @@ __device__ void ms_apply_marked(const MsParams& p, const Mask<NW>& act, uint32_t
           zero.w[k] = 0;
         }
         store_mask<NW>(p.N + v * NW, zero);
-        if (settle<NW>(p, Fn, v, vv, need, nw, __ldg(p.deg + v), lvl4, la))
+        if (settle<NW>(p, Fn, v, vv, need, nw, __ldg(p.deg + v), level, la))
           atomicOr(la.fb + (v >> 5), 1u << (v & 31));
       }
     }
@@ -800,7 +806,7 @@ __device__ void ms_clear_marked(const MsParams& p, uint32_t* Fn, const uint32_t*
 
 // after a pull level: the hub rows, whose chunks ORed into N
 template <int NW, bool SP>
-__device__ void ms_settle_hubs(const MsParams& p, const Mask<NW>& act, uint32_t* Fn, uint32_t lvl4,
+__device__ void ms_settle_hubs(const MsParams& p, const Mask<NW>& act, uint32_t* Fn, uint32_t level,
                                LevelAcc<NW>& la) {
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
@@ -822,7 +828,7 @@ __device__ void ms_settle_hubs(const MsParams& p, const Mask<NW>& act, uint32_t*
       for (int k = 0; k < NW; ++k) zero.w[k] = 0;
       store_mask<NW>(p.N + (int64_t)h * NW, zero);
     }
-    const bool app = settle<NW>(p, Fn, h, vv, need, nw, __ldg(p.deg + h), lvl4, la);
+    const bool app = settle<NW>(p, Fn, h, vv, need, nw, __ldg(p.deg + h), level, la);
     if constexpr (SP)
       if (app) atomicOr(la.fb + (h >> 5), 1u << (h & 31));  // the pull phase wrote its bit clear
   }
@@ -947,7 +953,7 @@ __global__ void __launch_bounds__(MS_THREADS, MS_MIN_BLOCKS) msbfs_kernel(MsPara
     if ((int64_t)r < p.nlv) {
       atomicOr(p.V + (int64_t)r * NW + tid / 32, 1u << (tid & 31));
       atomicOr(p.F[0] + (int64_t)r * NW + tid / 32, 1u << (tid & 31));
-      p.L[(int64_t)r * W + tid] = 0;
+      p.L[(int64_t)r * NW + tid / 32] = make_uint4(0, 0, 0, 0);  // level 0 (the same from every root here)
       if constexpr (SP) atomicOr(p.fb[0] + (r >> 5), 1u << (r & 31));  // level 0's frontier bitmap
     }
   }
@@ -970,10 +976,11 @@ __global__ void __launch_bounds__(MS_THREADS, MS_MIN_BLOCKS) msbfs_kernel(MsPara
     if (blockIdx.x == 0 && threadIdx.x < 4) ctl->alive[(phase + 1) % 3][threadIdx.x] = 0;
     const uint32_t* Fc = p.F[(level - 1) & 1];
     uint32_t* Fn = p.F[level & 1];
-    const uint32_t lvl4 = (uint32_t)level * 0x01010101u;
     LevelAcc<NW> la;
     la.clear();
     la.fb = p.fb[level % 3];
+    if (level == (int)MS_PLANE_LEVELS - 1)  // the upper planes, first written at the next level
+      for (int64_t i = tid; i < p.nlv * NW; i += nthreads) p.L[p.nlv * NW + i] = make_uint4(0, 0, 0, 0);
     // The first level that would pull surveys the lanes' frontiers: lanes
     // whose frontier degree sum is under 1/MS_SURVEY_DIV of the graph's entries are
     // pushed at that level, the others pulled (a mixed level: both phases
@@ -1029,13 +1036,13 @@ __global__ void __launch_bounds__(MS_THREADS, MS_MIN_BLOCKS) msbfs_kernel(MsPara
     const uint32_t* fbc = p.fb[(level - 1) % 3];
     la.track = sparse;
     if (pull && !mixed) {
-      ms_pull_rows<NW, false, COUNT, SP>(p, act, Fc, Fn, lvl4, la);
+      ms_pull_rows<NW, false, COUNT, SP>(p, act, Fc, Fn, level, la);
       ms_pull_hubs<NW, COUNT>(p, act, Fc, la);
     } else if (mixed) {
       if constexpr (SP) ms_push_rows_marked<NW, COUNT>(p, Fc, fbc, qm, la);
       else ms_push_rows_dense<NW, COUNT>(p, Fc, qm, la);
       ms_push_hubs<NW, COUNT>(p, Fc, qm, la);
-      ms_pull_rows<NW, true, COUNT, SP>(p, pm, Fc, Fn, lvl4, la);
+      ms_pull_rows<NW, true, COUNT, SP>(p, pm, Fc, Fn, level, la);
       ms_pull_hubs<NW, COUNT>(p, pm, Fc, la);
     } else {
       if constexpr (SP) ms_push_rows_marked<NW, COUNT>(p, Fc, fbc, qm, la);
@@ -1052,9 +1059,9 @@ __global__ void __launch_bounds__(MS_THREADS, MS_MIN_BLOCKS) msbfs_kernel(MsPara
     if (!settled && !grid_sync<M_NUM>(&ctl->bar, nullptr, sh_acc, nullptr, sh_cnt, &sh_flag)) return;
     if (tid == 0 && !settled) ctl->level_mid_ns[level] = globaltimer();
     if (settled) {
-    } else if (pull && !mixed) ms_settle_hubs<NW, SP>(p, act, Fn, lvl4, la);
-    else if (sparse) ms_apply_marked<NW>(p, act, Fn, lvl4, la);
-    else ms_apply<NW, SP>(p, act, Fn, lvl4, la);
+    } else if (pull && !mixed) ms_settle_hubs<NW, SP>(p, act, Fn, level, la);
+    else if (sparse) ms_apply_marked<NW>(p, act, Fn, level, la);
+    else ms_apply<NW, SP>(p, act, Fn, level, la);
     flush_level<NW, COUNT>(la, sh_acc, sh_or, alive);
     if (!grid_sync_sum<M_NUM>(cnt, &ctl->bar, sh_acc, sh_cnt)) return;
     ++phase;
@@ -1102,64 +1109,96 @@ __device__ __forceinline__ void transpose4x4(const uint32_t a[4], uint32_t c[4])
   c[3] = __byte_perm(t1, t3, 0x7632u);
 }
 
-// levels [nlv][W] (reordered) -> out[lane][orig] (nroots rows of nolv bytes).
-// Four consecutive original vertices per thread: their rows' visited masks and
-// the level bytes of their visited 16-lane groups (unvisited lanes read as
-// 255).  Each 32-bit word of a row holds 4 lanes of one vertex; a 4x4 byte
-// transpose in registers turns the 4 vertices' words into 4 words of one lane
-// x 4 vertices, so every store instruction of a warp writes 128 consecutive
-// bytes of one lane's output row (nolv is a multiple of 65536, so the
-// 4-vertex steps never straddle the end).
+// 4x4 bit transpose in each of the 8 nibbles: afterwards nibble i of q[j] holds
+// bit 4 * i + j of the four words
+__device__ __forceinline__ void transpose_nibbles(uint32_t q[4]) {
+  uint32_t t = ((q[0] >> 2) ^ q[2]) & 0x33333333u;
+  q[2] ^= t;
+  q[0] ^= t << 2;
+  t = ((q[1] >> 2) ^ q[3]) & 0x33333333u;
+  q[3] ^= t;
+  q[1] ^= t << 2;
+  t = ((q[0] >> 1) ^ q[1]) & 0x55555555u;
+  q[1] ^= t;
+  q[0] ^= t << 1;
+  t = ((q[2] >> 1) ^ q[3]) & 0x55555555u;
+  q[3] ^= t;
+  q[2] ^= t << 1;
+}
+
+// level bit planes (reordered) -> out[lane][orig] (nroots rows of nolv bytes).
+// Four consecutive original vertices per thread and 32 lanes at a time: their
+// visited words and planes (all ones where unvisited).  A bit transpose turns a
+// vertex's four planes into words of one 4-bit level per nibble; splitting the
+// nibbles and a 4x4 byte transpose over the 4 vertices give words of one lane x
+// 4 vertices (about 6 operations per word), so every store instruction of a
+// warp writes 128 consecutive bytes of one lane's output row (nolv is a
+// multiple of 65536, so the 4-vertex steps never straddle the end).  Levels of
+// 15 and more (num_levels over 15) take their upper four bits from the second
+// planes; below, 15 only means unvisited and becomes 255.
 constexpr int TR_BLOCK = 256;
 template <int NW>
-__global__ void __launch_bounds__(TR_BLOCK) ms_transpose_kernel(const uint8_t* __restrict__ L,
+__global__ void __launch_bounds__(TR_BLOCK, 4) ms_transpose_kernel(const uint4* __restrict__ L,
                                                                 const uint32_t* __restrict__ V,
                                                                 const uint32_t* __restrict__ reorder, int64_t nlv,
                                                                 int64_t nolv, const int* nroots_dev,
+                                                                const MsCtl* __restrict__ ctl,
                                                                 uint8_t* __restrict__ out) {
-  constexpr int W = 32 * NW;
-  constexpr int CHUNKS = W / 16;
   const int nroots = *nroots_dev;
+  const bool deep = ctl->num_levels > MS_PLANE_LEVELS - 1;
   for (int64_t u0 = ((int64_t)blockIdx.x * TR_BLOCK + threadIdx.x) * 4; u0 < nolv;
        u0 += (int64_t)gridDim.x * TR_BLOCK * 4) {
     const uint4 rr = __ldg(reinterpret_cast<const uint4*>(reorder + u0));
     const uint32_t r[4] = {rr.x, rr.y, rr.z, rr.w};
     uint32_t vb[4][NW];
 #pragma unroll
-    for (int v = 0; v < 4; ++v)
+    for (int v = 0; v < 4; ++v) {
+      Mask<NW> m;
 #pragma unroll
-      for (int k = 0; k < NW; ++k) vb[v][k] = (int64_t)r[v] < nlv ? __ldg(V + (int64_t)r[v] * NW + k) : 0u;
-    // one 16-lane group at a time (keeps the registers, hence occupancy, low)
+      for (int k = 0; k < NW; ++k) m.w[k] = 0;
+      if ((int64_t)r[v] < nlv) m = load_mask<NW>(V + (int64_t)r[v] * NW);
+#pragma unroll
+      for (int k = 0; k < NW; ++k) vb[v][k] = m.w[k];
+    }
+    // 32 lanes at a time (keeps the registers, hence occupancy, low)
 #pragma unroll 1
-    for (int q = 0; q < CHUNKS; ++q) {
-      uint4 x[4];
+    for (int k = 0; k < NW; ++k) {
+      if (32 * k >= nroots) break;
+      uint32_t lo[4][4], hi[4][4];
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
-        uint32_t word = vb[v][0];
+        uint32_t vis = vb[v][0];
 #pragma unroll
-        for (int k = 1; k < NW; ++k) word = (q >> 1) == k ? vb[v][k] : word;
-        const uint32_t bits = (word >> ((q & 1) * 16)) & 0xFFFFu;
-        x[v] = make_uint4(~0u, ~0u, ~0u, ~0u);
-        if (bits) {
-          x[v] = __ldg(reinterpret_cast<const uint4*>(L + (int64_t)r[v] * W) + q);
-          x[v].x |= ~nibble_bytes(bits & 0xFu);
-          x[v].y |= ~nibble_bytes((bits >> 4) & 0xFu);
-          x[v].z |= ~nibble_bytes((bits >> 8) & 0xFu);
-          x[v].w |= ~nibble_bytes((bits >> 12) & 0xFu);
+        for (int q = 1; q < NW; ++q) vis = k == q ? vb[v][q] : vis;
+        uint4 x = make_uint4(0, 0, 0, 0), y = x;
+        if (vis) {
+          x = __ldg(L + (int64_t)r[v] * NW + k);
+          if (deep) y = __ldg(L + (nlv + (int64_t)r[v]) * NW + k);
         }
+        lo[v][0] = x.x | ~vis; lo[v][1] = x.y | ~vis; lo[v][2] = x.z | ~vis; lo[v][3] = x.w | ~vis;
+        hi[v][0] = y.x | ~vis; hi[v][1] = y.y | ~vis; hi[v][2] = y.z | ~vis; hi[v][3] = y.w | ~vis;
+        transpose_nibbles(lo[v]);
+        if (deep) transpose_nibbles(hi[v]);
       }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int lb = 4 * (4 * q + i);  // lanes lb .. lb + 3
-        if (lb >= nroots) break;
-        uint32_t a[4], c[4];
+      for (int j = 0; j < 4; ++j)
 #pragma unroll
-        for (int v = 0; v < 4; ++v) a[v] = i == 0 ? x[v].x : i == 1 ? x[v].y : i == 2 ? x[v].z : x[v].w;
-        transpose4x4(a, c);
+        for (int s = 0; s < 2; ++s) {
+          uint32_t a[4], c[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (lb + j < nroots) *reinterpret_cast<uint32_t*>(out + (int64_t)(lb + j) * nolv + u0) = c[j];
-      }
+          for (int v = 0; v < 4; ++v) {
+            uint32_t x = (lo[v][j] >> (4 * s)) & 0x0F0F0F0Fu;
+            if (deep) x |= ((hi[v][j] >> (4 * s)) & 0x0F0F0F0Fu) << 4;
+            else x |= (((x + 0x01010101u) & 0x10101010u) >> 4) * 0xF0u;
+            a[v] = x;
+          }
+          transpose4x4(a, c);
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            const int lane = 32 * k + 8 * t + 4 * s + j;
+            if (lane < nroots) *reinterpret_cast<uint32_t*>(out + (int64_t)lane * nolv + u0) = c[t];
+          }
+        }
     }
   }
 }
@@ -1266,7 +1305,7 @@ struct g500_msbfs {
 
   void* slab = nullptr;             // the allocation of the arrays below but the hub tables
   uint32_t *V = nullptr, *F = nullptr, *N = nullptr;  // [nlv][4] words (room for 128 lanes)
-  uint8_t* L = nullptr;                               // [nlv][128]
+  uint4* L = nullptr;                                 // [2][nlv][4] level bit planes (room for 128 lanes)
   uint8_t* out = nullptr;                             // [128][nolv]
   MsCtl* ctl = nullptr;                               // [4] one per batch
   int64_t* roots_dev = nullptr;                       // [4][128]
@@ -1451,9 +1490,9 @@ static int ms_enqueue_batch(g500_msbfs* m, int b, cudaStream_t s) {
   }
   uint8_t* out = m->out + (int64_t)b * W * g->nolv;
   const unsigned tg = (unsigned)std::min<int64_t>(ceil_div(g->nolv, 4 * TR_BLOCK), (int64_t)num_sms() * 8);
-  if (W == 32) ms_transpose_kernel<1><<<tg, TR_BLOCK, 0, s>>>(m->L, m->V, g->d_reorder, g->nlv, g->nolv, m->nroots_dev + b, out);
-  else if (W == 64) ms_transpose_kernel<2><<<tg, TR_BLOCK, 0, s>>>(m->L, m->V, g->d_reorder, g->nlv, g->nolv, m->nroots_dev + b, out);
-  else ms_transpose_kernel<4><<<tg, TR_BLOCK, 0, s>>>(m->L, m->V, g->d_reorder, g->nlv, g->nolv, m->nroots_dev + b, out);
+  if (W == 32) ms_transpose_kernel<1><<<tg, TR_BLOCK, 0, s>>>(m->L, m->V, g->d_reorder, g->nlv, g->nolv, m->nroots_dev + b, m->ctl + b, out);
+  else if (W == 64) ms_transpose_kernel<2><<<tg, TR_BLOCK, 0, s>>>(m->L, m->V, g->d_reorder, g->nlv, g->nolv, m->nroots_dev + b, m->ctl + b, out);
+  else ms_transpose_kernel<4><<<tg, TR_BLOCK, 0, s>>>(m->L, m->V, g->d_reorder, g->nlv, g->nolv, m->nroots_dev + b, m->ctl + b, out);
   ms_root_fixup_kernel<<<1, MS_MAX_LANES, 0, s>>>(m->roots_dev + b * MS_MAX_LANES, m->nroots_dev + b, g->nolv, out);
   G500_CUDA(cudaGetLastError());
   return G500_OK;
@@ -1480,7 +1519,7 @@ extern "C" int g500_msbfs_create(g500_graph* g, g500_msbfs** out) {
   slab.add(&m->V, nlv * 4);                 // visited masks
   slab.add(&m->F, 2 * nlv * 4);             // frontier masks
   slab.add(&m->N, nlv * 4);                 // next masks
-  slab.add(&m->L, nlv * MS_MAX_LANES);      // levels
+  slab.add(&m->L, 2 * nlv * 4);             // level bit planes
   slab.add(&m->deg, nlv);                   // row lengths
   slab.add(&m->marks, 4 * m->nwords);       // frontier and touched bitmaps
   slab.add(&m->out, (int64_t)MS_MAX_LANES * g->nolv);  // output levels
@@ -1738,7 +1777,7 @@ extern "C" int g500_msbfs_get_grid(const g500_msbfs* m, int lane_width, int* blo
 extern "C" int g500_msbfs_workspace_bytes(const g500_graph* g, uint64_t* bytes) {
   if (!g || !bytes) return set_error(G500_E_INVAL, "null argument");
   const uint64_t nlv = (uint64_t)std::max<int64_t>(g->nlv, 1);
-  // V, F, N (4 words each), L (128 bytes), row lengths, output rows, the
+  // V, F, N (4 words each), level planes (128 bytes), row lengths, output rows, the
   // sparse-level bitmaps (4 bits), with room for the hub tables and control
   // blocks
   *bytes = nlv * (4 * 16 + MS_MAX_LANES + 4) + (uint64_t)MS_MAX_LANES * (uint64_t)g->nolv + (16ull << 20) +

@@ -174,3 +174,37 @@ def test_msbfs_refuses_depth_beyond_uint8(g500):
     assert ms.levels(np.array([150]))[0][150] == 0
     ms.close()
     g.close()
+
+
+@pytest.mark.parametrize("depth", [13, 14, 15, 16, 17, 33, 253])
+@pytest.mark.parametrize("vr", [0, 2])
+def test_msbfs_levels_across_bit_planes_and_stats(g500, depth, vr):
+    """A path of `depth` edges with leaves, seen from several roots at once: levels on both sides of the first
+    four bit planes (14 | 15 | 16) and up to the uint8 limit, in every lane width, with and without sparse
+    levels; and each root's statistics against its plain BFS, for a second component and for roots without
+    edges (one with a self loop) too."""
+    pairs = [(i, i + 1) for i in range(depth)] + [(i, 1000 + i) for i in range(1, depth - 1, 3)]
+    pairs += [(2000, 2001), (2001, 2002), (2003, 2003)]
+    edges = np.zeros(len(pairs), g500.EDGE_DTYPE)
+    edges["v0_low"], edges["v1_low"] = np.array(pairs).T
+    bfs = g500.BfsOnGPU(reorder_mode=vr)
+    bfs.construct(edges)
+    bfs.prepare_bfs()
+    n = bfs.graph_.pred_size()
+    roots = np.array([0, depth, depth // 2, 1, 1001, 2001, 2003, 1999, 0, 2000] + list(range(2, 12)), np.int64)
+    want, stats = [], []
+    pred = np.zeros(n, np.int64)
+    for r in roots:
+        st = bfs.run_bfs(int(r), pred)
+        lv = g500.levels_from_pred(pred)
+        want.append(np.where(lv == 0xFFFF, 255, lv).astype(np.uint8))
+        stats.append((st.reached, st.nedge))
+    assert max(int(w[w != 255].max()) for w in want) == depth
+    for lanes in (32, 64, 128):
+        ms = g500.MultiSourceBFS(bfs.graph_, lanes)
+        for sparse in (False, True):
+            ms.set_sparse(sparse)
+            assert np.array_equal(ms.levels(roots), np.array(want)), (lanes, sparse)
+            assert list(zip(*(a.tolist() for a in ms.root_stats(len(roots))))) == stats, (lanes, sparse)
+        ms.close()
+    bfs.close()

@@ -1203,17 +1203,21 @@ __global__ void __launch_bounds__(TR_BLOCK, 4) ms_transpose_kernel(const uint4* 
   }
 }
 
-// a root outside the CSR range (no edges) reached only itself; its self-loop
-// occurrences are its edge count
-__global__ void ms_root_stats_fixup_kernel(const int64_t* roots, const int* nroots_dev, const uint32_t* reorder,
-                                           int64_t nlv, const uint32_t* endp, unsigned long long* reached,
-                                           unsigned long long* e2) {
+// Per-root statistics from the sums of ms_stats_kernel: all vertices with edges
+// less those the lane did not reach.  A root outside the CSR range (no edges)
+// reached only itself; its self-loop occurrences are its edge count.
+__global__ void ms_root_stats_kernel(const int64_t* roots, const int* nroots_dev, const uint32_t* reorder,
+                                     int64_t nlv, const uint32_t* endp, const unsigned long long* all,
+                                     unsigned long long* reached, unsigned long long* e2) {
   const int i = threadIdx.x;
   if (i >= *nroots_dev) return;
   const uint32_t r = reorder[roots[i]];
   if ((int64_t)r >= nlv) {
     reached[i] = 1;
     e2[i] = endp[r];
+  } else {
+    reached[i] = all[0] - reached[i];
+    e2[i] = all[1] - e2[i];
   }
 }
 
@@ -1229,41 +1233,73 @@ __global__ void ms_degree_kernel(const uint64_t* __restrict__ off, int64_t nlv, 
 }
 
 
-// per lane: reached vertices and the sum of endpoint occurrences (2 x nedge)
+// The vertices with edges and the sum of their endpoint occurrences (all), and
+// per lane the part of both that the lane did not reach (2 x nedge and the
+// reached count follow).  Nearly every vertex is reached by every lane, so a
+// warp looks at single lanes only for the words where one of its 32 vertices
+// lacks some: SCALE 24, 64 roots: two reductions per lane and 32 vertices took
+// 1.03 ms, now 0.13 ms with its launches.  A vertex without edges can
+// only be a root itself: its lane's missing sums get it taken off.
 template <int NW>
 __global__ void __launch_bounds__(256) ms_stats_kernel(const uint32_t* __restrict__ V,
+                                                       const uint32_t* __restrict__ vis_init,
                                                        const uint32_t* __restrict__ endp, int64_t nlv, int nroots,
-                                                       unsigned long long* reached, unsigned long long* e2) {
+                                                       unsigned long long* missing, unsigned long long* missing_e2,
+                                                       unsigned long long* all) {
   __shared__ unsigned long long s_r[MS_MAX_LANES], s_e[MS_MAX_LANES];
   for (int i = threadIdx.x; i < MS_MAX_LANES; i += blockDim.x) s_r[i] = s_e[i] = 0;
   __syncthreads();
   const int lane = threadIdx.x & 31;
-  for (int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < nlv;
+  unsigned long long nv = 0, ne = 0;
+  for (int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < nlv;  // nlv: a multiple of 32
        base += (int64_t)gridDim.x * blockDim.x) {
     const int64_t v = base + lane;
-    Mask<NW> m;
-    uint32_t e = 0;
-    if (v < nlv) {
-      m = load_mask<NW>(V + v * NW);
-      e = __ldg(endp + v);
-    } else {
+    const bool has = !((__ldg(vis_init + (base >> 5)) >> lane) & 1u);
+    const Mask<NW> m = load_mask<NW>(V + v * NW);
+    const uint32_t e = __ldg(endp + v);
+    nv += has;
+    ne += has ? e : 0u;
+    bool any = false;
+    uint32_t x[NW];
 #pragma unroll
-      for (int k = 0; k < NW; ++k) m.w[k] = 0;
+    for (int k = 0; k < NW; ++k) {
+      const uint32_t act = active_word(nroots, k);
+      x[k] = has ? act & ~m.w[k] : act & m.w[k];
+      any |= x[k] != 0;
     }
-    for (int l = 0; l < nroots; ++l) {
-      const uint32_t bit = (m.w[l >> 5] >> (l & 31)) & 1u;
-      const unsigned rs = __reduce_add_sync(FULL_MASK, bit);
-      const unsigned es = __reduce_add_sync(FULL_MASK, bit ? e : 0u);
-      if (lane == 0 && rs) {
-        atomicAdd(&s_r[l], (unsigned long long)rs);
-        atomicAdd(&s_e[l], (unsigned long long)es);
+    if (!__any_sync(FULL_MASK, any)) continue;
+#pragma unroll
+    for (int k = 0; k < NW; ++k) {
+      unsigned todo = __reduce_or_sync(FULL_MASK, has ? x[k] : 0u);
+      while (todo) {
+        const int b = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const bool miss = has && ((x[k] >> b) & 1u);
+        const unsigned rs = __popc(__ballot_sync(FULL_MASK, miss));
+        const unsigned es = __reduce_add_sync(FULL_MASK, miss ? e : 0u);
+        if (lane == 0) {
+          atomicAdd(&s_r[k * 32 + b], (unsigned long long)rs);
+          atomicAdd(&s_e[k * 32 + b], (unsigned long long)es);
+        }
       }
+      if (!has)
+        for (uint32_t own = x[k]; own; own &= own - 1) {
+          const int l = k * 32 + __ffs(own) - 1;
+          atomicAdd(&s_r[l], ~0ull);  // - 1
+          atomicAdd(&s_e[l], 0ull - e);
+        }
     }
+  }
+  nv = warp_sum(nv);
+  ne = warp_sum(ne);
+  if (lane == 0) {
+    atomicAdd(&all[0], nv);
+    atomicAdd(&all[1], ne);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < nroots; i += blockDim.x) {
-    if (s_r[i]) atomicAdd(&reached[i], s_r[i]);
-    if (s_e[i]) atomicAdd(&e2[i], s_e[i]);
+    if (s_r[i]) atomicAdd(&missing[i], s_r[i]);
+    if (s_e[i]) atomicAdd(&missing_e2[i], s_e[i]);
   }
 }
 
@@ -1312,7 +1348,7 @@ struct g500_msbfs {
   int* nroots_dev = nullptr;                          // [4]
   int64_t* staging = nullptr;                         // pinned: [4][128] roots + [4] counts
   MsCtl* h_ctl = nullptr;                             // pinned [4]
-  unsigned long long* stats_dev = nullptr;            // [2][128]
+  unsigned long long* stats_dev = nullptr;            // [2][128] and the sums over all vertices
   unsigned long long* h_stats = nullptr;              // pinned [2][128]: reached, 2 * nedge per lane
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_done = nullptr;
   unsigned grid_full[3] = {0, 0, 0};                  // the whole device's co-resident blocks
@@ -1526,7 +1562,7 @@ extern "C" int g500_msbfs_create(g500_graph* g, g500_msbfs** out) {
   slab.add(&m->ctl, 4);
   slab.add(&m->roots_dev, 4 * MS_MAX_LANES);
   slab.add(&m->nroots_dev, 4);
-  slab.add(&m->stats_dev, 2 * MS_MAX_LANES);
+  slab.add(&m->stats_dev, 2 * MS_MAX_LANES + 2);
   if (st == G500_OK) st = slab.alloc(&m->slab, "multi-source masks and levels");
   if (st == G500_OK && g->nlv > 0) {
     const unsigned dgrid = (unsigned)std::min<int64_t>(ceil_div(g->nlv, 256), (int64_t)num_sms() * 8);
@@ -1575,18 +1611,19 @@ extern "C" int g500_msbfs_set_params(g500_msbfs* m, int lane_width, double alpha
 // Per-lane reached / 2*nedge of the last launch into h_stats (enqueued on s).
 static int ms_enqueue_stats(g500_msbfs* m, int nroots, cudaStream_t s) {
   g500_graph* g = m->g;
-  G500_CUDA(cudaMemsetAsync(m->stats_dev, 0, sizeof(unsigned long long) * 2 * MS_MAX_LANES, s));
+  G500_CUDA(cudaMemsetAsync(m->stats_dev, 0, sizeof(unsigned long long) * (2 * MS_MAX_LANES + 2), s));
   const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(std::max<int64_t>(g->nlv, 1), 256), num_sms() * 8);
   const int W = m->lane_width;
   unsigned long long* r = m->stats_dev;
   unsigned long long* e = m->stats_dev + MS_MAX_LANES;
+  unsigned long long* all = m->stats_dev + 2 * MS_MAX_LANES;
   if (g->nlv > 0) {
-    if (W == 32) ms_stats_kernel<1><<<grid, 256, 0, s>>>(m->V, g->d_endp, g->nlv, nroots, r, e);
-    else if (W == 64) ms_stats_kernel<2><<<grid, 256, 0, s>>>(m->V, g->d_endp, g->nlv, nroots, r, e);
-    else ms_stats_kernel<4><<<grid, 256, 0, s>>>(m->V, g->d_endp, g->nlv, nroots, r, e);
+    if (W == 32) ms_stats_kernel<1><<<grid, 256, 0, s>>>(m->V, g->d_vis_init, g->d_endp, g->nlv, nroots, r, e, all);
+    else if (W == 64) ms_stats_kernel<2><<<grid, 256, 0, s>>>(m->V, g->d_vis_init, g->d_endp, g->nlv, nroots, r, e, all);
+    else ms_stats_kernel<4><<<grid, 256, 0, s>>>(m->V, g->d_vis_init, g->d_endp, g->nlv, nroots, r, e, all);
   }
-  ms_root_stats_fixup_kernel<<<1, MS_MAX_LANES, 0, s>>>(m->roots_dev, m->nroots_dev, g->d_reorder, g->nlv, g->d_endp,
-                                                        r, e);
+  ms_root_stats_kernel<<<1, MS_MAX_LANES, 0, s>>>(m->roots_dev, m->nroots_dev, g->d_reorder, g->nlv, g->d_endp,
+                                                  all, r, e);
   G500_CUDA(cudaGetLastError());
   G500_CUDA(cudaMemcpyAsync(m->h_stats, m->stats_dev, sizeof(unsigned long long) * 2 * MS_MAX_LANES,
                             cudaMemcpyDeviceToHost, s));

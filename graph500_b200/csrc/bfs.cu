@@ -599,6 +599,7 @@ __global__ void __launch_bounds__(BFS_THREADS, BFS_MIN_BLOCKS) bfs_persistent_ke
     if (has_edges && tid == 0) put_deferred<DEF>(p, root_r, (uint32_t)p.root, 0);
   if (blockIdx.x == 0 && threadIdx.x < 3 * C_NUM) (&ctl->cnt[0][0])[threadIdx.x] = 0;
   if (blockIdx.x == 0 && threadIdx.x < 3 * P_NUM) (&ctl->pos[0][0])[threadIdx.x] = 0;
+  if (tid == 0) ctl->edges2 = 0;
 
   // first_expand (bfs.hpp:477-518): the root's row becomes the first queue
   for (int64_t c = tid; c < root_items; c += nthreads) {
@@ -613,6 +614,7 @@ __global__ void __launch_bounds__(BFS_THREADS, BFS_MIN_BLOCKS) bfs_persistent_ke
   if (!has_edges) {  // the search is over before it starts: only the root has a parent
     if (tid == 0) {
       ctl->num_levels = 0;
+      ctl->td_levels = 0;
       ctl->final_vis = 0;
       ctl->t_init_ns = ctl->t_end_ns = globaltimer();
     }
@@ -904,6 +906,18 @@ static int make_params(g500_bfs* b, int64_t root, int64_t* pred, RunParams* out)
   return G500_OK;
 }
 
+// The control block before a run.  A run clears what it needs but the error
+// bits and the arrivals of its one plain grid barrier, which a complete run
+// leaves at a multiple of its grid, as the barrier wants them: so the block is
+// cleared only before the first run, after an error, and when the grid
+// changes (one launch less per run).
+static int prepare_ctl(g500_bfs* b, cudaStream_t s) {
+  if (!b->ctl_ready) G500_CUDA(cudaMemsetAsync(b->d_ctl, 0, sizeof(BfsCtl), s));
+  b->ctl_ready = 0;  // until the run is known to have ended well
+  return G500_OK;
+}
+static void check_ctl(g500_bfs* b) { b->ctl_ready = b->h_ctl->bar.err == 0 && b->h_ctl->bar.count < (1u << 30); }
+
 // pred -> uint8 levels (255 unreached); a level over 254 raises *overflow
 __global__ void levels_from_pred_kernel(const int64_t* __restrict__ pred, int64_t n, uint8_t* __restrict__ out,
                                         unsigned* overflow) {
@@ -976,6 +990,7 @@ extern "C" int g500_bfs_set_grid(g500_bfs* b, int blocks) {
   if (blocks < 0) return set_error(G500_E_INVAL, "negative block count");
   if (b->in_flight) return set_error(G500_E_STATE, "a run is in flight");
   b->grid = blocks == 0 ? b->grid_full : std::min<unsigned>((unsigned)blocks, b->grid_full);
+  b->ctl_ready = 0;
   return G500_OK;
 }
 
@@ -1002,7 +1017,7 @@ int bfs_launch_levels(g500_bfs* b, int64_t root, uint8_t* levels_dst) {
   G500_TRY(make_params(b, root, b->d_pred, &p));
   p.endw = b->d_endw;
   void* args[] = {&p};
-  G500_CUDA(cudaMemsetAsync(b->d_ctl, 0, sizeof(BfsCtl), s));
+  G500_TRY(prepare_ctl(b, s));
   G500_CUDA(cudaMemsetAsync(b->d_overflow, 0, sizeof(unsigned), s));
   G500_CUDA(cudaLaunchCooperativeKernel(bfs_kernel_for(p.deferred), dim3(b->grid), dim3(BFS_THREADS), args,
                                         0, s));
@@ -1043,6 +1058,7 @@ int bfs_complete(g500_bfs* b, int64_t* reached, int64_t* nedge) {
   const cudaError_t e = cudaEventSynchronize(b->ev_done);
   if (e != cudaSuccess) return cuda_error(e, "cudaEventSynchronize", __FILE__, __LINE__);
   const BfsCtl& c = *b->h_ctl;
+  check_ctl(b);
   if (c.bar.err & BFS_ERR_TIMEOUT) return set_error(G500_E_TIMEOUT, "grid barrier wait gave up (bounded spin)");
   if (c.bar.err & BFS_ERR_PACK) {  // deeper than the packed entries hold: the same run with 64-bit entries
     b->pack_off = 1;
@@ -1172,7 +1188,7 @@ extern "C" int g500_bfs_run(g500_bfs* b, int64_t root, int64_t* pred, int pred_o
   G500_TRY(make_params(b, root, pred_on_device ? pred : b->d_pred, &p));
   if (stats) p.endw = b->d_endw;
   void* args[] = {&p};
-  G500_CUDA(cudaMemsetAsync(b->d_ctl, 0, sizeof(BfsCtl), s));
+  G500_TRY(prepare_ctl(b, s));
   G500_CUDA(cudaEventRecord(b->ev0, s));
   G500_CUDA(cudaLaunchCooperativeKernel(bfs_kernel_for(p.deferred), dim3(b->grid), dim3(BFS_THREADS), args,
                                         0, s));
@@ -1188,6 +1204,7 @@ extern "C" int g500_bfs_run(g500_bfs* b, int64_t root, int64_t* pred, int pred_o
   G500_CUDA(cudaStreamSynchronize(s));
   b->last_root = root;
   const BfsCtl& c = *b->h_ctl;
+  check_ctl(b);
   if (c.bar.err & BFS_ERR_TIMEOUT) return set_error(G500_E_TIMEOUT, "grid barrier wait gave up (bounded spin)");
   if (c.bar.err & BFS_ERR_PACK) {  // deeper than the packed entries hold: the same run with 64-bit entries
     b->pack_off = 1;

@@ -241,6 +241,7 @@ struct g500_bfs {
   BfsCtl* d_ctl = nullptr;
   BfsCtl* h_ctl = nullptr;           // copy after each run: &host_ctl, or pinned once a run was asynchronous
   BfsCtl host_ctl = {};
+  int ctl_ready = 0;                 // d_ctl is as a run needs it (see prepare_ctl)
   LevelRecord* d_rec = nullptr;      // [MAX_LEVELS]
   TdItem* d_big = nullptr;           // [BIG_ROWS] long frontier rows, listed whole
   unsigned long long* d_endw = nullptr;  // [nlv/32] endpoint occurrences per bitmap word

@@ -65,6 +65,8 @@ constexpr int TD_UNROLL = TD_CHUNK / 32;  // virtual edges per lane per pass
 constexpr int BU_WORDS = 4;               // 32-vertex words a warp keeps in flight (bottom-up pass A)
 constexpr int BU_SERIAL = 8;              // row entries a lane checks alone per step (one sector)
 constexpr int BU_LANE_MAX = 64;           // a row with at most this many entries left is scanned by its own lane
+constexpr int BU_LIST = 64;               // unvisited vertices a warp keeps listed (late bottom-up levels)
+constexpr int BU_LIST_WORDS = 48;
 // A frontier row of more than BIG_CHUNKS work items is listed whole (up to
 // BIG_ROWS rows per level) instead of cut into items by one warp; the next
 // top-down level spreads its chunks over every warp.
@@ -357,6 +359,50 @@ __device__ __forceinline__ void scan_serial(const RunParams& p, const uint32_t* 
   }
 }
 
+// The rows of a warp's lanes from pos on (pos == end: none), each to its first
+// entry visited before this level.
+__device__ __forceinline__ void scan_rows(const RunParams& p, const uint32_t* __restrict__ vis_cur, uint64_t& pos,
+                                          uint64_t end, uint32_t& parent, uint32_t& k) {
+  const int lane = threadIdx.x & 31;
+  // rows with at most BU_LANE_MAX entries left: every lane goes on along
+  // its own row, all rows at once (one warp-wide scan per row serialised
+  // the rows); longer rows are scanned by the whole warp below
+  for (;;) {
+    const bool mine = pos < end && end - pos <= (uint64_t)BU_LANE_MAX;
+    if (!__any_sync(FULL_MASK, mine)) break;
+    if (mine) scan_serial(p, vis_cur, pos, end, parent, k);
+  }
+  unsigned rest = __ballot_sync(FULL_MASK, pos < end);
+  while (rest) {
+    const int r = __ffs(rest) - 1;
+    rest &= rest - 1;
+    const uint64_t rb = __shfl_sync(FULL_MASK, pos, r);
+    const uint64_t re = __shfl_sync(FULL_MASK, end, r);
+    uint32_t hitc = NO_VERTEX;
+    uint64_t hitpos = re;
+    for (uint64_t p0 = rb; p0 < re; p0 += 32) {
+      const uint64_t pp = p0 + lane;
+      bool h = false;
+      uint32_t cv = 0;
+      if (pp < re) {
+        cv = __ldg(p.col + pp);
+        h = vis_test(vis_cur, cv);
+      }
+      const unsigned hm = __ballot_sync(FULL_MASK, h);
+      if (hm) {
+        const int hl = __ffs(hm) - 1;
+        hitc = __shfl_sync(FULL_MASK, cv, hl);
+        hitpos = p0 + hl;
+        break;
+      }
+    }
+    if (lane == r) {
+      parent = hitc;
+      k += (uint32_t)((hitpos + 1 < re ? hitpos + 1 : re) - rb);
+    }
+  }
+}
+
 // Bottom-up level (bottom_up_search_bitmap, bfs.hpp:1839-2038), one warp per
 // 32 words of the visited bitmap at a time, both steps on the same words so
 // that no grid barrier separates them:
@@ -445,43 +491,7 @@ __device__ void bu_level(const RunParams& p, const uint32_t* __restrict__ vis_cu
         k = 1;
         scan_serial(p, vis_cur, pos, end, parent, k);
       }
-      // rows with at most BU_LANE_MAX entries left: every lane goes on along
-      // its own row, all rows at once (one warp-wide scan per row serialised
-      // the rows); longer rows are scanned by the whole warp below
-      for (;;) {
-        const bool mine = pos < end && end - pos <= (uint64_t)BU_LANE_MAX;
-        if (!__any_sync(FULL_MASK, mine)) break;
-        if (mine) scan_serial(p, vis_cur, pos, end, parent, k);
-      }
-      unsigned rest = __ballot_sync(FULL_MASK, pos < end);
-      while (rest) {
-        const int r = __ffs(rest) - 1;
-        rest &= rest - 1;
-        const uint64_t rb = __shfl_sync(FULL_MASK, pos, r);
-        const uint64_t re = __shfl_sync(FULL_MASK, end, r);
-        uint32_t hitc = NO_VERTEX;
-        uint64_t hitpos = re;
-        for (uint64_t p0 = rb; p0 < re; p0 += 32) {
-          const uint64_t pp = p0 + lane;
-          bool h = false;
-          uint32_t cv = 0;
-          if (pp < re) {
-            cv = __ldg(p.col + pp);
-            h = vis_test(vis_cur, cv);
-          }
-          const unsigned hm = __ballot_sync(FULL_MASK, h);
-          if (hm) {
-            const int hl = __ffs(hm) - 1;
-            hitc = __shfl_sync(FULL_MASK, cv, hl);
-            hitpos = p0 + hl;
-            break;
-          }
-        }
-        if (lane == r) {
-          parent = hitc;
-          k += (uint32_t)((hitpos + 1 < re ? hitpos + 1 : re) - rb);
-        }
-      }
+      scan_rows(p, vis_cur, pos, end, parent, k);
       if (parent != NO_VERTEX) {
         atomicOr(vis_next + (v >> 5), 1u << (v & 31));
         const uint32_t par = __ldg(p.invert + parent);
@@ -500,6 +510,121 @@ __device__ void bu_level(const RunParams& p, const uint32_t* __restrict__ vis_cu
   if (p.count_edges) {  // a first-neighbour hit or a one-edge miss examined one edge (one sector)
     block_add(sh_acc, C_EDGES, found_a + single_misses + edges);
     block_add(sh_acc, C_SECT, found_a + single_misses + sectors);
+  }
+}
+
+// Late bottom-up levels.  Once few vertices are unvisited, a pass over the
+// bitmap costs more than they do (SCALE 26: 18 us a level for 20 thousand
+// vertices).  So, on graphs of at least BU_LIST_WORDS bitmap words per warp
+// (listing costs 3 us, as much as three listed levels save at SCALE 22 with 16
+// words per warp; SCALE 26 has 221: levels 5-7 29 / 18 / 18 -> 19 / 6 / 5 us) and
+// where the direction rule lets a search with so few unvisited vertices stay
+// bottom-up, a bottom-up level that follows another one ends by listing, per
+// warp and in shared memory, the vertices its own words leave unvisited; if no
+// warp has more than BU_LIST of them, the following bottom-up levels only scan
+// the listed rows.  The visited maps still alternate: a listed level writes the
+// other buffer, which it first brings up to date with its own words (the first
+// such level) or with the vertices it found one level before.
+struct WarpLists {
+  uint32_t left[BFS_THREADS / 32][BU_LIST];   // unvisited vertices of the warp's words
+  uint32_t found[BFS_THREADS / 32][BU_LIST];  // found by the last listed level
+  uint32_t nleft[BFS_THREADS / 32], nfound[BFS_THREADS / 32];
+};
+
+// List what the level leaves; a warp with too many raises C_BIG, which
+// bottom-up levels do not use otherwise.
+__device__ void bu_collect(const RunParams& p, const uint32_t* vis_next, WarpLists& wl, unsigned long long* sh_acc) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t nwarps = gwarp_count();
+  constexpr int U = 4;
+  uint32_t n = 0;
+  __syncwarp();  // the warp's own writes of its words
+  for (int64_t k32 = 0; gwarp_id() + k32 * nwarps < p.nwords && n <= (uint32_t)BU_LIST; k32 += 32 * U) {
+    uint32_t rem[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t wi = gwarp_id() + (k32 + 32 * u + lane) * nwarps;
+      rem[u] = wi < p.nwords ? ~__ldcg(vis_next + wi) : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t c = __popc(rem[u]);
+      if (!__any_sync(FULL_MASK, c)) continue;
+      const uint32_t incl = warp_incl_scan(c);
+      const uint32_t total = __shfl_sync(FULL_MASK, incl, 31);
+      if (n + total <= (uint32_t)BU_LIST) {
+        uint32_t at = n + incl - c;
+        const uint32_t base = (uint32_t)(gwarp_id() + (k32 + 32 * u + lane) * nwarps) * 32;
+        for (uint32_t m = rem[u]; m; m &= m - 1) wl.left[warp][at++] = base + __ffs(m) - 1;
+      }
+      n += total;
+    }
+  }
+  if (lane == 0) {
+    wl.nleft[warp] = n;
+    wl.nfound[warp] = 0;
+    if (n > (uint32_t)BU_LIST) atomicAdd(&sh_acc[C_BIG], 1ull);
+  }
+}
+
+template <int DEF>
+__device__ void bu_list_level(const RunParams& p, const uint32_t* __restrict__ vis_cur, uint32_t* __restrict__ vis_next,
+                              bool first, WarpLists& wl, unsigned long long* sh_acc, int64_t lvl) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (first) {
+    const int64_t nwarps = gwarp_count();
+    for (int64_t wi = gwarp_id() + lane * nwarps; wi < p.nwords; wi += 32 * nwarps) vis_next[wi] = __ldcg(vis_cur + wi);
+  } else {
+    for (uint32_t i = lane; i < wl.nfound[warp]; i += 32) {
+      const uint32_t v = wl.found[warp][i];
+      atomicOr(vis_next + (v >> 5), 1u << (v & 31));
+    }
+  }
+  const uint32_t n = wl.nleft[warp];
+  __syncwarp();
+  uint32_t keep = 0, nfound = 0;
+  unsigned long long edges = 0, sectors = 0;
+  for (uint32_t b0 = 0; b0 < n; b0 += 32) {
+    uint32_t v = NO_VERTEX, parent = NO_VERTEX, k = 0;
+    uint64_t pos = 0, end = 0;
+    if (b0 + lane < n) {
+      v = wl.left[warp][b0 + lane];
+      pos = __ldg(p.off + v);
+      end = __ldg(p.off + v + 1);
+      scan_serial(p, vis_cur, pos, end, parent, k);
+    }
+    scan_rows(p, vis_cur, pos, end, parent, k);
+    const bool hit = parent != NO_VERTEX;
+    const unsigned hits = __ballot_sync(FULL_MASK, hit);
+    const unsigned rest = __ballot_sync(FULL_MASK, v != NO_VERTEX && !hit);
+    const unsigned below = (1u << lane) - 1u;
+    __syncwarp();  // the batch's list entries have been read
+    if (hit) {
+      wl.found[warp][nfound + __popc(hits & below)] = v;
+      atomicOr(vis_next + (v >> 5), 1u << (v & 31));
+      const uint32_t par = __ldg(p.invert + parent);
+      if constexpr (DEF != 0) put_deferred<DEF>(p, v, par, lvl);
+      else p.pred[__ldg(p.invert + v)] = (int64_t)par | lvl;
+    } else if (v != NO_VERTEX) {
+      wl.left[warp][keep + __popc(rest & below)] = v;
+    }
+    nfound += __popc(hits);
+    keep += __popc(rest);
+    if (p.count_edges && v != NO_VERTEX) {
+      edges += k;
+      sectors += (k + 7) / 8;
+    }
+    __syncwarp();
+  }
+  if (lane == 0) {
+    wl.nleft[warp] = keep;
+    wl.nfound[warp] = nfound;
+    if (nfound) atomicAdd(&sh_acc[C_DISC], (unsigned long long)nfound);
+    if (n) atomicAdd(&sh_acc[C_SCAN], (unsigned long long)n);
+  }
+  if (p.count_edges) {
+    block_add(sh_acc, C_EDGES, edges);
+    block_add(sh_acc, C_SECT, sectors);
   }
 }
 
@@ -570,6 +695,7 @@ __global__ void __launch_bounds__(BFS_THREADS, BFS_MIN_BLOCKS) bfs_persistent_ke
   __shared__ unsigned long long sh_cnt[C_NUM];
   __shared__ unsigned long long sh_acc[C_NUM];
   __shared__ unsigned sh_flag;
+  __shared__ WarpLists lists;
   BfsCtl* ctl = p.ctl;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
@@ -625,6 +751,10 @@ __global__ void __launch_bounds__(BFS_THREADS, BFS_MIN_BLOCKS) bfs_persistent_ke
 
   int cur_vis = 0;
   bool forward = true, growing = true;
+  bool bu_before = false;  // the last level was bottom-up
+  int listed_levels = -1;  // bottom-up levels run from the lists (-1: there are none)
+  const bool lists_pay = p.policy == G500_DIR_REFERENCE && p.nwords >= BU_LIST_WORDS * gwarp_count() &&
+                         (double)p.ngv / p.beta < (double)(BU_LIST * gwarp_count());
   int64_t qn = root_items, prev_nq = 0, visited = 1, carried = 0, nbig = 0;
   unsigned td_levels = 0;
   int64_t mu = (int64_t)(p.off[p.nlv] - root_deg);  // degree sum of unvisited vertices (edge policy)
@@ -658,8 +788,14 @@ __global__ void __launch_bounds__(BFS_THREADS, BFS_MIN_BLOCKS) bfs_persistent_ke
       listed = sh_cnt[C_QITEMS];
       mf = sh_cnt[C_MF];
     } else {
-      bu_level<DEF>(p, p.vis[cur_vis], p.vis[cur_vis ^ 1], sh_acc, lvl);
+      if (listed_levels >= 0) {
+        bu_list_level<DEF>(p, p.vis[cur_vis], p.vis[cur_vis ^ 1], listed_levels == 0, lists, sh_acc, lvl);
+      } else {
+        bu_level<DEF>(p, p.vis[cur_vis], p.vis[cur_vis ^ 1], sh_acc, lvl);
+        if (bu_before && lists_pay) bu_collect(p, p.vis[cur_vis ^ 1], lists, sh_acc);
+      }
       if (!grid_sync_sum<C_NUM>(cnt, &ctl->bar, sh_acc, sh_cnt)) return;
+      if (listed_levels >= 0 || (bu_before && lists_pay && sh_cnt[C_BIG] == 0)) ++listed_levels;
       if (tid == 0) t_mid = globaltimer();
       ++phase;
       disc = sh_cnt[C_DISC];
@@ -671,6 +807,8 @@ __global__ void __launch_bounds__(BFS_THREADS, BFS_MIN_BLOCKS) bfs_persistent_ke
     const int64_t carried_in = carried;
     visited += nq;
     const bool was_forward = forward;
+    bu_before = !forward;
+    if (forward) listed_levels = -1;
     td_levels += was_forward;
     if (!forward) cur_vis ^= 1;  // the bottom-up output is the current visited map
     if (nq == 0) {

@@ -349,3 +349,38 @@ def test_device_validator_matches_oracle(g500, oracle_mod, mutation):
     if ok_d:
         assert evc_d == evc_o == pf_nedge()[12]
     g.close()
+
+
+@pytest.mark.parametrize("pred_mode", [1, 2, 3])
+@pytest.mark.parametrize("pendants", [3, 10, 90])
+def test_listed_bottom_up_levels(g500, oracle_mod, pred_mode, pendants):
+    """A star (which turns the search bottom-up) with a caterpillar of 60 spine vertices on one leaf: dozens of
+    late bottom-up levels over rows of 1 to 92 entries.  One or two blocks have enough words per warp to run
+    them from their lists (90 pendants overflow the lists at first), the whole device does not: levels and
+    per-level counters must be the same."""
+    leaves, spine = 60000, 60
+    pairs = [(0, i) for i in range(1, leaves + 1)]
+    base, pend = leaves + 1, leaves + 1 + spine
+    pairs += [(1 if i == 0 else base + i - 1, base + i) for i in range(spine)]
+    pairs += [(base + i, pend + i * pendants + j) for i in range(spine) for j in range(pendants)]
+    edges = np.zeros(len(pairs), g500.EDGE_DTYPE)
+    edges["v0_low"], edges["v1_low"] = np.array(pairs).T
+    og = oracle_mod.Graph(edges, 2)
+    bfs = g500.BfsOnGPU(reorder_mode=2)
+    bfs.construct(edges)
+    bfs.prepare_bfs(2000.0, 1e9, True)
+    bfs.set_pred_mode(pred_mode)
+    pred = np.zeros(bfs.graph_.pred_size(), np.int64)
+    keys = ("direction", "level", "discovered", "scanned", "edges_examined", "edge_sectors")
+    want = None
+    for blocks in (0, 1, 2, 1):
+        g500.check(g500.lib().g500_bfs_set_grid(bfs.h, blocks))
+        st = bfs.run_bfs(77, pred)
+        assert np.array_equal(g500.levels_from_pred(pred), og.bfs_levels(77)), blocks
+        ok, evc, rep = oracle_mod.validate(edges, bfs.graph_.info.max_used_vertex + 1, len(pred), 77, pred)
+        assert ok and evc == st.nedge, rep
+        got = [tuple(lv[k] for k in keys) for lv in bfs.level_stats()]
+        assert sum(not lv[0] for lv in got) == st.bu_levels > spine and len(got) == st.num_levels
+        want = want or got
+        assert got == want, blocks
+    bfs.close()

@@ -60,6 +60,7 @@ constexpr uint64_t BFS_DEFERRED_PRED_BYTES = 100ull << 20;
 constexpr int PACK_SHIFT = 27;
 constexpr int PACK_LEVELS = 1 << (32 - PACK_SHIFT);
 constexpr uint32_t PACK_NONE = 0xFFFFFFFFu;
+constexpr int64_t BFS_SMALL_VERTS = 1 << 20;
 constexpr int BFS_MIN_BLOCKS = 2;        // co-resident blocks per SM (64 registers, no spills)
 constexpr int TD_UNROLL = TD_CHUNK / 32;  // virtual edges per lane per pass
 constexpr int BU_WORDS = 4;               // 32-vertex words a warp keeps in flight (bottom-up pass A)
@@ -1113,7 +1114,11 @@ extern "C" int g500_bfs_create(g500_graph* g, g500_bfs** out) {
     chk(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, g->device), "cudaDeviceGetAttribute");
     if (st == G500_OK && (!coop || per_sm <= 0))
       st = set_error(G500_E_DEVICE, "device cannot co-schedule the persistent BFS kernel");
-    b->grid = b->grid_full = (unsigned)(num_sms() * std::max(per_sm, 1));
+    b->grid_full = (unsigned)(num_sms() * std::max(per_sm, 1));
+    // one block per SM on small graphs: a barrier of half the blocks is shorter,
+    // and the levels have no work for more (SCALE 16 / 18 / 20: 63.8 / 68.0 / 83.2
+    // us with two blocks per SM, 59.9 / 63.4 / 79.8 with one; SCALE 21: 101.4 / 102.5)
+    b->grid = g->nlv <= BFS_SMALL_VERTS ? std::min(b->grid_full, (unsigned)num_sms()) : b->grid_full;
   }
   if (st != G500_OK) {
     bfs_free(b);

@@ -34,6 +34,7 @@ namespace g500 {
 constexpr int MS_THREADS = 256;
 constexpr int MS_MIN_BLOCKS = 4;
 constexpr int MS_MAX_LANES = 128;
+constexpr int64_t MS_SMALL_VERTS = 3 << 17, MS_MEDIUM_VERTS = 1 << 20;  // grid choice at creation
 constexpr int MS_MAX_LEVEL = 254;  // level bytes: 255 marks unreached
 // M_ROWS / M_SECT (counting launches only): row and chunk offset reads, and
 // the 32-byte adjacency sectors the level's entries span
@@ -1586,7 +1587,16 @@ extern "C" int g500_msbfs_create(g500_graph* g, g500_msbfs** out) {
     int per_sm = 0;
     chk(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernels[i], MS_THREADS, 0), "occupancy");
     if (st == G500_OK && per_sm <= 0) st = set_error(G500_E_DEVICE, "multi-source kernel cannot be co-scheduled");
-    m->grid[i] = m->grid_full[i] = (unsigned)(num_sms() * std::max(per_sm, 1));
+    m->grid_full[i] = (unsigned)(num_sms() * std::max(per_sm, 1));
+    // Fewer blocks on small graphs, whose levels are short against a barrier of
+    // all of them.  Launch times in us by blocks per SM, for 32 lanes and 24
+    // roots / 64 and 64 / 128 and 128:
+    //   SCALE 16 (65 k vertices)   4: 142 / 191 / 295    2: 129 / 167 / 252
+    //   SCALE 18 (197 k)           4: 248 / 323 / 477    3: 220 / 281 / 423    2: 216 / 261 / 396
+    //   SCALE 20 (655 k)           4: 291 / 390 / 590    3: 292 / 384 / 566    2: 323 / 422 / 615
+    //   SCALE 21 (1.2 M)           4: 282 / 403 / 1551   3: 299 / 403 / 1441   2: 351 / 481 / 1492
+    const unsigned per = g->nlv <= MS_SMALL_VERTS ? 2u : (g->nlv <= MS_MEDIUM_VERTS ? 3u : 4u);
+    m->grid[i] = std::min(m->grid_full[i], per * (unsigned)num_sms());
   }
   if (st != G500_OK) {
     ms_free(m);

@@ -150,12 +150,12 @@ __device__ __forceinline__ void append_row(uint64_t rb, uint64_t deg, uint32_t o
       nch = 0;
     }
   }
+  unsigned long long base = 0;
   const uint32_t incl = warp_incl_scan(nch);
   const uint32_t total = __shfl_sync(FULL_MASK, incl, 31);
   if (total == 0) return;
   if (lane == 0) *items += total;
   const uint32_t excl = incl - nch;
-  unsigned long long base = 0;
   if (lane == 31) base = atomicAdd(qcount, (unsigned long long)total);
   base = __shfl_sync(FULL_MASK, base, 31);
   if (base + total > (unsigned long long)cap) {
@@ -636,7 +636,9 @@ __device__ void bu_list_level(const RunParams& p, const uint32_t* __restrict__ v
 // word cost up to 32 such chains per warp), and its words are strided over the
 // whole id range as in the bottom-up levels, which spreads small graphs and
 // dense id ranges over every warp: SCALE 16 unordered 26-34 -> 6 us, SCALE 24
-// (2.1 M found) 121 -> 40 us.
+// (2.1 M found) 121 -> 40 us.  Four rows per lane share one queue position where
+// every row is one item (nearly all of a late frontier), which takes a quarter
+// of the waits for it: 40 -> 26 us.
 __device__ void compact_phase(const RunParams& p, const uint32_t* __restrict__ vis_new,
                               const uint32_t* __restrict__ vis_old, TdItem* q_out, unsigned long long* pos,
                               unsigned long long* sh_acc) {
@@ -650,23 +652,68 @@ __device__ void compact_phase(const RunParams& p, const uint32_t* __restrict__ v
     const uint32_t incl = warp_incl_scan(c);
     const uint32_t excl = incl - c;
     const uint32_t total = __shfl_sync(FULL_MASK, incl, 31);
-    for (uint32_t b0 = 0; b0 < total; b0 += 32) {
-      const uint32_t idx = b0 + lane;
-      const int o = owner_lane(excl, idx);
-      const uint32_t fo = __shfl_sync(FULL_MASK, f, o);
-      const uint32_t exo = __shfl_sync(FULL_MASK, excl, o);
-      const uint32_t wo = __shfl_sync(FULL_MASK, (uint32_t)wi, o);
-      uint64_t rb = 0, deg = 0;
-      uint32_t ow = 0;
-      if (idx < total) {
-        const uint32_t v = wo * 32 + select_bit(fo, idx - exo);
-        rb = __ldg(p.off + v);
-        deg = __ldg(p.off + v + 1) - rb;
-        ow = __ldg(p.invert + v);
-        skipped += (deg < 2);
-        if (deg < 2) deg = 0;
+    constexpr int U = 4;
+    for (uint32_t b0 = 0; b0 < total; b0 += 32 * U) {
+      uint64_t rb[U];
+      uint32_t deg[U], ow[U];  // a row is shorter than 2^32: one entry per vertex id
+      bool longer = false;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint32_t idx = b0 + 32 * u + lane;
+        const int o = owner_lane(excl, idx);
+        const uint32_t fo = __shfl_sync(FULL_MASK, f, o);
+        const uint32_t exo = __shfl_sync(FULL_MASK, excl, o);
+        const uint32_t wo = __shfl_sync(FULL_MASK, (uint32_t)wi, o);
+        rb[u] = 0;
+        deg[u] = ow[u] = 0;
+        if (idx < total) {
+          const uint32_t v = wo * 32 + select_bit(fo, idx - exo);
+          rb[u] = __ldg(p.off + v);
+          deg[u] = (uint32_t)(__ldg(p.off + v + 1) - rb[u]);
+          ow[u] = __ldg(p.invert + v);
+        }
       }
-      append_row(rb, deg, ow, q_out, p.cap, &pos[P_ITEMS], p.ctl, p.big, &pos[P_BIG], &items, &bigs);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        skipped += b0 + 32 * u + lane < total && deg[u] < 2;
+        if (deg[u] < 2) deg[u] = 0;
+        longer |= deg[u] > (uint32_t)TD_CHUNK;
+      }
+      if (__any_sync(FULL_MASK, longer)) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          append_row(rb[u], deg[u], ow[u], q_out, p.cap, &pos[P_ITEMS], p.ctl, p.big, &pos[P_BIG], &items, &bigs);
+        continue;
+      }
+      unsigned with[U];  // items stay in vertex order: neighbouring items read neighbouring rows
+      uint32_t all = 0;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        with[u] = __ballot_sync(FULL_MASK, deg[u] != 0);
+        all += __popc(with[u]);
+      }
+      if (all == 0) continue;
+      unsigned long long base = 0;
+      if (lane == 0) {
+        items += all;
+        base = atomicAdd(&pos[P_ITEMS], (unsigned long long)all);
+      }
+      base = __shfl_sync(FULL_MASK, base, 0);
+      if (base + all > (unsigned long long)p.cap) {
+        if (lane == 0) atomicOr(&p.ctl->bar.err, (unsigned)BFS_ERR_QUEUE);
+        continue;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (deg[u]) {
+          TdItem it;
+          it.begin = rb[u];
+          it.orig = ow[u];
+          it.len = deg[u] | FIRST_CHUNK;
+          q_out[base + __popc(with[u] & ((1u << lane) - 1u))] = it;
+        }
+        base += __popc(with[u]);
+      }
     }
   }
   block_add(sh_acc, C_SKIP, skipped);

@@ -384,3 +384,32 @@ def test_listed_bottom_up_levels(g500, oracle_mod, pred_mode, pendants):
         want = want or got
         assert got == want, blocks
     bfs.close()
+
+
+@pytest.mark.parametrize("blocks", [1, 3])
+def test_switch_back_to_top_down_keeps_levels(g500, oracle_mod, blocks):
+    """The bottom-up to top-down switch with rows of one edge, of one work item, of several and of more than a
+    warp lists (8192 entries), found by the last bottom-up level."""
+    rng = np.random.default_rng(3)
+    pairs = [(0, i) for i in range(1, 40001)]                                      # turns the search bottom-up
+    sizes = [1, 2, 127, 128, 129, 255, 256, 257, 8191, 8192, 8193, 9000, 20000]
+    nxt = 100000
+    for k, s in enumerate(sizes):                                                  # hubs two steps away from 0
+        pairs.append((1 + 7 * k, 50000 + k))
+        pairs += [(50000 + k, nxt + j) for j in range(s)]
+        nxt += s
+    pairs += [(int(a), int(b)) for a, b in rng.integers(100000, nxt, (5000, 2))]
+    edges = np.zeros(len(pairs), g500.EDGE_DTYPE)
+    edges["v0_low"], edges["v1_low"] = np.array(pairs).T
+    og = oracle_mod.Graph(edges, 2)
+    bfs = g500.BfsOnGPU(reorder_mode=2)
+    bfs.construct(edges)
+    bfs.prepare_bfs(2000.0, 1.2, True)  # back to top-down as soon as the bottom-up level shrinks
+    g500.check(g500.lib().g500_bfs_set_grid(bfs.h, blocks))
+    pred = np.zeros(bfs.graph_.pred_size(), np.int64)
+    for root in (99, 0, 50012):
+        st = bfs.run_bfs(root, pred)
+        assert np.array_equal(g500.levels_from_pred(pred), og.bfs_levels(root)), root
+        ok, evc, rep = oracle_mod.validate(edges, bfs.graph_.info.max_used_vertex + 1, len(pred), root, pred)
+        assert ok and evc == st.nedge, rep
+    bfs.close()

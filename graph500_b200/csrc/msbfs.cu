@@ -49,7 +49,7 @@ struct MsCtl {
   unsigned long long t0_ns, t_init_ns, t_end_ns;
   unsigned alive[3][4];      // lanes that found vertices in the phase (rotating like cnt)
   unsigned long long level_new[MS_MAX_LEVEL + 2];
-  unsigned long long lane_deg[MS_MAX_LANES];  // sampled frontier degree sum per lane (lane survey)
+  unsigned long long lane_deg[4][MS_MAX_LANES];  // sampled frontier degree sum per lane, by survey (MS_SURVEYS)
   unsigned long long level_t_ns[MS_MAX_LEVEL + 2];
   unsigned long long level_mid_ns[MS_MAX_LEVEL + 2];  // end of the pull/push phase
   unsigned char level_pull[MS_MAX_LEVEL + 2];
@@ -83,6 +83,7 @@ struct MsParams {
   int64_t nwords;            // (nlv + 31) / 32
   int64_t sparse_limit;
   int64_t nlv;
+  int64_t ngv;               // vertices with edges
   double alpha;
   MsCtl* ctl;
 };
@@ -844,8 +845,15 @@ __device__ void ms_settle_hubs(const MsParams& p, const Mask<NW>& act, uint32_t*
 // the block adds them up in shared memory and once into ctl->lane_deg.
 constexpr int MS_SURVEY_STEP = 8;
 constexpr int MS_SURVEY_DIV = 64;  // a lane is pushed when its frontier degree sum is under entries / this
-constexpr int MS_SURVEY_LEVELS = 1;  // pull levels that survey (the first ones)
-static_assert(MS_SURVEY_LEVELS == 1, "the lanes' sums are cleared once per launch");
+// Every pull level surveys while less than 1/MS_SURVEY_FOUND of the launch's
+// (vertex, lane) pairs are found, that is up to and including its densest level.
+// With one survey per launch, spent where the second level already pulled, lanes
+// whose roots lie a step further out kept every row of the dense level scanned
+// to its end, the longest by one warp: 128 roots at SCALE 22 took 7.5 ms (level 3
+// 6.4) and take 1.5 (0.4) with a survey at both; launches that surveyed at the
+// dense level before are the same within 1 %.
+constexpr int MS_SURVEY_FOUND = 4;
+constexpr int MS_SURVEYS = 4;  // at most, each with its own sums
 template <int NW>
 __device__ void ms_lane_survey(const MsParams& p, const uint32_t* Fc, unsigned long long* sh_lane) {
   const int lane = threadIdx.x & 31;
@@ -970,6 +978,8 @@ __global__ void __launch_bounds__(MS_THREADS, MS_MIN_BLOCKS) msbfs_kernel(MsPara
   const unsigned long long survey_thr = __ldg(p.off + p.nlv) / ((unsigned long long)MS_SURVEY_DIV * MS_SURVEY_STEP);
   unsigned long long mu_last = __ldg(p.off + p.nlv);  // every vertex needs every lane
   unsigned long long mf_last = 0;                     // level 1: the roots' rows
+  unsigned long long found = 0;                       // (vertex, lane) pairs so far
+  const unsigned long long found_limit = (unsigned long long)p.ngv * (unsigned)nroots / MS_SURVEY_FOUND;
   for (;; ++level) {
     unsigned long long* cnt = ctl->cnt[phase % 3];
     unsigned* alive = ctl->alive[phase % 3];
@@ -982,8 +992,7 @@ __global__ void __launch_bounds__(MS_THREADS, MS_MIN_BLOCKS) msbfs_kernel(MsPara
     la.fb = p.fb[level % 3];
     if (level == (int)MS_PLANE_LEVELS - 1)  // the upper planes, first written at the next level
       for (int64_t i = tid; i < p.nlv * NW; i += nthreads) p.L[p.nlv * NW + i] = make_uint4(0, 0, 0, 0);
-    // The first level that would pull surveys the lanes' frontiers: lanes
-    // whose frontier degree sum is under 1/MS_SURVEY_DIV of the graph's entries are
+    // A level that would pull surveys the lanes' frontiers: lanes whose frontier degree sum is under 1/MS_SURVEY_DIV of the graph's entries are
     // pushed at that level, the others pulled (a mixed level: both phases
     // leave their finds in N and the apply pass settles every vertex).
     Mask<NW> qm, pm;  // lanes pushed, lanes pulled
@@ -992,14 +1001,14 @@ __global__ void __launch_bounds__(MS_THREADS, MS_MIN_BLOCKS) msbfs_kernel(MsPara
       qm.w[k] = pull ? 0u : ~0u;
       pm.w[k] = act.w[k];
     }
-    const bool survey = pull && surveys < MS_SURVEY_LEVELS;
+    const bool survey = pull && surveys < MS_SURVEYS && found < found_limit;
     if (survey) {
-      ++surveys;
+      unsigned long long* lane_deg = ctl->lane_deg[surveys++];
       for (int i = threadIdx.x; i < MS_MAX_LANES; i += blockDim.x) sh_lane[i] = 0;
       __syncthreads();
       ms_lane_survey<NW>(p, Fc, sh_lane);
       __syncthreads();
-      if (threadIdx.x < W && sh_lane[threadIdx.x]) atomicAdd(&ctl->lane_deg[threadIdx.x], sh_lane[threadIdx.x]);
+      if (threadIdx.x < W && sh_lane[threadIdx.x]) atomicAdd(&lane_deg[threadIdx.x], sh_lane[threadIdx.x]);
       if (!grid_sync<M_NUM>(&ctl->bar, nullptr, sh_acc, nullptr, sh_cnt, &sh_flag)) return;
       if (threadIdx.x < NW) {
         uint32_t aw = 0;  // act.w[threadIdx.x], selected so that act stays in registers
@@ -1009,7 +1018,7 @@ __global__ void __launch_bounds__(MS_THREADS, MS_MIN_BLOCKS) msbfs_kernel(MsPara
         uint32_t q = 0;
         for (int b = 0; b < 32; ++b) {
           const int k = threadIdx.x * 32 + b;
-          if (((aw >> b) & 1u) && __ldcg(&ctl->lane_deg[k]) < survey_thr) q |= 1u << b;
+          if (((aw >> b) & 1u) && __ldcg(&lane_deg[k]) < survey_thr) q |= 1u << b;
         }
         sh_qm[threadIdx.x] = q;
       }
@@ -1067,6 +1076,7 @@ __global__ void __launch_bounds__(MS_THREADS, MS_MIN_BLOCKS) msbfs_kernel(MsPara
     if (!grid_sync_sum<M_NUM>(cnt, &ctl->bar, sh_acc, sh_cnt)) return;
     ++phase;
     const unsigned long long nnew = sh_cnt[M_NEW];
+    found += nnew;
     if (tid == 0) {
       ctl->level_new[level] = nnew;
       ctl->level_t_ns[level] = globaltimer();
@@ -1496,6 +1506,7 @@ static int ms_enqueue_batch(g500_msbfs* m, int b, cudaStream_t s) {
   p.roots = m->roots_dev + b * MS_MAX_LANES;
   p.nroots_dev = m->nroots_dev + b;
   p.nlv = g->nlv;
+  p.ngv = g->ngv;
   p.hub_tab = m->hub_tab;
   p.nhub_chunks = m->nhub_chunks;
   p.push_tab = m->push_tab;

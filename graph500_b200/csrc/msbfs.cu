@@ -41,11 +41,20 @@ constexpr int MS_MAX_LEVEL = 254;  // level bytes: 255 marks unreached
 enum MsCounter { M_NEW = 0, M_NF, M_MF, M_MU, M_EDGES, M_ROWS, M_SECT, M_NUM = 8 };
 enum MsErr { MS_ERR_DEPTH = 4 };
 
+// What a launch needs from the host, in one upload.
+struct MsHead {
+  int64_t roots[MS_MAX_LANES];     // original ids
+  uint8_t* row[2][MS_MAX_LANES];   // where each root's level row goes (device memory, 4-byte aligned; null: nowhere)
+  int32_t nroots;
+  int32_t second;                  // row[1] has any
+};
+
 struct MsCtl {
   unsigned long long cnt[3][M_NUM];
   GridBarrier bar;
   unsigned num_levels;
   unsigned pull_levels;
+  unsigned out_blocks;       // blocks of the output pass that have finished
   unsigned long long t0_ns, t_init_ns, t_end_ns;
   unsigned alive[3][4];      // lanes that found vertices in the phase (rotating like cnt)
   unsigned long long level_new[MS_MAX_LEVEL + 2];
@@ -1146,21 +1155,24 @@ __device__ __forceinline__ void transpose_nibbles(uint32_t q[4]) {
 // warp writes 128 consecutive bytes of one lane's output row (nolv is a
 // multiple of 65536, so the 4-vertex steps never straddle the end).  Levels of
 // 15 and more (num_levels over 15) take their upper four bits from the second
-// planes; below, 15 only means unvisited and becomes 255.
+// planes; below, 15 only means unvisited and becomes 255.  The next vertices' map
+// entries load while these are turned, and every row goes straight to where its
+// caller wants it (a copy per row took as long as the pass for 64 rows).  The
+// last block to finish sets each root's own level, which the planes of a root
+// outside the CSR range do not hold.  SCALE 24, 64
+// rows: 385 -> 356 us; SCALE 21, 128 rows into the caller's memory: 110 and 75 for
+// the copy -> 154 us.
 constexpr int TR_BLOCK = 256;
-template <int NW>
-__global__ void __launch_bounds__(TR_BLOCK, 4) ms_transpose_kernel(const uint4* __restrict__ L,
-                                                                const uint32_t* __restrict__ V,
-                                                                const uint32_t* __restrict__ reorder, int64_t nlv,
-                                                                int64_t nolv, const int* nroots_dev,
-                                                                const MsCtl* __restrict__ ctl,
-                                                                uint8_t* __restrict__ out) {
-  const int nroots = *nroots_dev;
-  const bool deep = ctl->num_levels > MS_PLANE_LEVELS - 1;
-  for (int64_t u0 = ((int64_t)blockIdx.x * TR_BLOCK + threadIdx.x) * 4; u0 < nolv;
-       u0 += (int64_t)gridDim.x * TR_BLOCK * 4) {
-    const uint4 rr = __ldg(reinterpret_cast<const uint4*>(reorder + u0));
+template <int NW, bool DEEP>
+__device__ __forceinline__ void write_rows(const uint4* __restrict__ L, const uint32_t* __restrict__ V,
+                                           const uint32_t* __restrict__ reorder, int64_t nlv, int64_t nolv,
+                                           int nroots, bool second, uint8_t* (*rows)[32 * NW]) {
+  const int64_t step = (int64_t)gridDim.x * TR_BLOCK * 4;
+  int64_t u0 = ((int64_t)blockIdx.x * TR_BLOCK + threadIdx.x) * 4;
+  uint4 rr = u0 < nolv ? __ldcs(reinterpret_cast<const uint4*>(reorder + u0)) : make_uint4(0, 0, 0, 0);
+  for (; u0 < nolv; u0 += step) {
     const uint32_t r[4] = {rr.x, rr.y, rr.z, rr.w};
+    if (u0 + step < nolv) rr = __ldcs(reinterpret_cast<const uint4*>(reorder + u0 + step));
     uint32_t vb[4][NW];
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
@@ -1175,21 +1187,22 @@ __global__ void __launch_bounds__(TR_BLOCK, 4) ms_transpose_kernel(const uint4* 
 #pragma unroll 1
     for (int k = 0; k < NW; ++k) {
       if (32 * k >= nroots) break;
-      uint32_t lo[4][4], hi[4][4];
+      uint32_t lo[4][4], hi[DEEP ? 4 : 1][4];
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
         uint32_t vis = vb[v][0];
 #pragma unroll
         for (int q = 1; q < NW; ++q) vis = k == q ? vb[v][q] : vis;
-        uint4 x = make_uint4(0, 0, 0, 0), y = x;
-        if (vis) {
-          x = __ldg(L + (int64_t)r[v] * NW + k);
-          if (deep) y = __ldg(L + (nlv + (int64_t)r[v]) * NW + k);
-        }
+        uint4 x = make_uint4(0, 0, 0, 0);
+        if (vis) x = __ldg(L + (int64_t)r[v] * NW + k);
         lo[v][0] = x.x | ~vis; lo[v][1] = x.y | ~vis; lo[v][2] = x.z | ~vis; lo[v][3] = x.w | ~vis;
-        hi[v][0] = y.x | ~vis; hi[v][1] = y.y | ~vis; hi[v][2] = y.z | ~vis; hi[v][3] = y.w | ~vis;
         transpose_nibbles(lo[v]);
-        if (deep) transpose_nibbles(hi[v]);
+        if constexpr (DEEP) {
+          uint4 y = make_uint4(0, 0, 0, 0);
+          if (vis) y = __ldg(L + (nlv + (int64_t)r[v]) * NW + k);
+          hi[v][0] = y.x | ~vis; hi[v][1] = y.y | ~vis; hi[v][2] = y.z | ~vis; hi[v][3] = y.w | ~vis;
+          transpose_nibbles(hi[v]);
+        }
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j)
@@ -1199,7 +1212,7 @@ __global__ void __launch_bounds__(TR_BLOCK, 4) ms_transpose_kernel(const uint4* 
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
             uint32_t x = (lo[v][j] >> (4 * s)) & 0x0F0F0F0Fu;
-            if (deep) x |= ((hi[v][j] >> (4 * s)) & 0x0F0F0F0Fu) << 4;
+            if constexpr (DEEP) x |= ((hi[v][j] >> (4 * s)) & 0x0F0F0F0Fu) << 4;
             else x |= (((x + 0x01010101u) & 0x10101010u) >> 4) * 0xF0u;
             a[v] = x;
           }
@@ -1207,35 +1220,43 @@ __global__ void __launch_bounds__(TR_BLOCK, 4) ms_transpose_kernel(const uint4* 
 #pragma unroll
           for (int t = 0; t < 4; ++t) {
             const int lane = 32 * k + 8 * t + 4 * s + j;
-            if (lane < nroots) *reinterpret_cast<uint32_t*>(out + (int64_t)lane * nolv + u0) = c[t];
+            uint8_t* d = rows[0][lane];
+            if (d) *reinterpret_cast<uint32_t*>(d + u0) = c[t];
+            if (second && (d = rows[1][lane])) *reinterpret_cast<uint32_t*>(d + u0) = c[t];
           }
         }
     }
   }
 }
 
-// Per-root statistics from the sums of ms_stats_kernel: all vertices with edges
-// less those the lane did not reach.  A root outside the CSR range (no edges)
-// reached only itself; its self-loop occurrences are its edge count.
-__global__ void ms_root_stats_kernel(const int64_t* roots, const int* nroots_dev, const uint32_t* reorder,
-                                     int64_t nlv, const uint32_t* endp, const unsigned long long* all,
-                                     unsigned long long* reached, unsigned long long* e2) {
-  const int i = threadIdx.x;
-  if (i >= *nroots_dev) return;
-  const uint32_t r = reorder[roots[i]];
-  if ((int64_t)r >= nlv) {
-    reached[i] = 1;
-    e2[i] = endp[r];
-  } else {
-    reached[i] = all[0] - reached[i];
-    e2[i] = all[1] - e2[i];
+template <int NW>
+__global__ void __launch_bounds__(TR_BLOCK, 4) ms_transpose_kernel(const uint4* __restrict__ L,
+                                                                const uint32_t* __restrict__ V,
+                                                                const uint32_t* __restrict__ reorder, int64_t nlv,
+                                                                int64_t nolv, const MsHead* __restrict__ head,
+                                                                MsCtl* ctl) {
+  constexpr int W = 32 * NW;
+  __shared__ uint8_t* rows[2][W];
+  __shared__ int last;
+  const int nroots = head->nroots;
+  bool any = false;
+  for (int i = threadIdx.x; i < W; i += TR_BLOCK) {
+    rows[0][i] = i < nroots ? head->row[0][i] : nullptr;
+    rows[1][i] = i < nroots ? head->row[1][i] : nullptr;
+    any |= rows[0][i] || rows[1][i];
   }
-}
-
-// every root is its own level 0 (also a root outside the CSR range)
-__global__ void ms_root_fixup_kernel(const int64_t* roots, const int* nroots_dev, int64_t nolv, uint8_t* out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < *nroots_dev) out[(int64_t)i * nolv + roots[i]] = 0;
+  if (!__syncthreads_or(any)) return;  // no row is wanted
+  if (ctl->num_levels > MS_PLANE_LEVELS - 1) write_rows<NW, true>(L, V, reorder, nlv, nolv, nroots, head->second, rows);
+  else write_rows<NW, false>(L, V, reorder, nlv, nolv, nroots, head->second, rows);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&ctl->out_blocks, 1u) + 1 == gridDim.x;
+  __syncthreads();
+  if (last)
+    for (int i = threadIdx.x; i < nroots; i += TR_BLOCK) {
+      if (rows[0][i]) rows[0][i][head->roots[i]] = 0;
+      if (rows[1][i]) rows[1][i][head->roots[i]] = 0;
+    }
 }
 
 __global__ void ms_degree_kernel(const uint64_t* __restrict__ off, int64_t nlv, uint32_t* __restrict__ deg) {
@@ -1251,12 +1272,22 @@ __global__ void ms_degree_kernel(const uint64_t* __restrict__ off, int64_t nlv, 
 // lacks some: SCALE 24, 64 roots: two reductions per lane and 32 vertices took
 // 1.03 ms, now 0.13 ms with its launches.  A vertex without edges can
 // only be a root itself: its lane's missing sums get it taken off.
+// The last block to finish turns the sums into each root's reached count and 2 x
+// nedge (a root outside the CSR range, without edges, reached only itself; its
+// self-loop occurrences are its edge count) and clears them for the next call.
+struct MsSums {
+  unsigned long long missing[MS_MAX_LANES], missing_e2[MS_MAX_LANES];
+  unsigned long long verts, ends;  // over all vertices with edges
+  unsigned blocks;                 // that have finished
+};
 template <int NW>
 __global__ void __launch_bounds__(256) ms_stats_kernel(const uint32_t* __restrict__ V,
                                                        const uint32_t* __restrict__ vis_init,
                                                        const uint32_t* __restrict__ endp, int64_t nlv, int nroots,
-                                                       unsigned long long* missing, unsigned long long* missing_e2,
-                                                       unsigned long long* all) {
+                                                       const MsHead* __restrict__ head,
+                                                       const uint32_t* __restrict__ reorder, MsSums* sums,
+                                                       unsigned long long* out /* [2][MS_MAX_LANES] */) {
+  __shared__ int last;
   __shared__ unsigned long long s_r[MS_MAX_LANES], s_e[MS_MAX_LANES];
   for (int i = threadIdx.x; i < MS_MAX_LANES; i += blockDim.x) s_r[i] = s_e[i] = 0;
   __syncthreads();
@@ -1304,13 +1335,32 @@ __global__ void __launch_bounds__(256) ms_stats_kernel(const uint32_t* __restric
   nv = warp_sum(nv);
   ne = warp_sum(ne);
   if (lane == 0) {
-    atomicAdd(&all[0], nv);
-    atomicAdd(&all[1], ne);
+    atomicAdd(&sums->verts, nv);
+    atomicAdd(&sums->ends, ne);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < nroots; i += blockDim.x) {
-    if (s_r[i]) atomicAdd(&missing[i], s_r[i]);
-    if (s_e[i]) atomicAdd(&missing_e2[i], s_e[i]);
+    if (s_r[i]) atomicAdd(&sums->missing[i], s_r[i]);
+    if (s_e[i]) atomicAdd(&sums->missing_e2[i], s_e[i]);
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&sums->blocks, 1u) + 1 == gridDim.x;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const unsigned long long verts = __ldcg(&sums->verts), ends = __ldcg(&sums->ends);
+  for (int i = threadIdx.x; i < nroots; i += blockDim.x) {
+    const uint32_t r = reorder[head->roots[i]];
+    const bool inside = (int64_t)r < nlv;
+    out[i] = inside ? verts - __ldcg(&sums->missing[i]) : 1ull;
+    out[MS_MAX_LANES + i] = inside ? ends - __ldcg(&sums->missing_e2[i]) : (unsigned long long)endp[r];
+    sums->missing[i] = sums->missing_e2[i] = 0;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    sums->verts = sums->ends = 0;
+    sums->blocks = 0;
   }
 }
 
@@ -1355,11 +1405,11 @@ struct g500_msbfs {
   uint4* L = nullptr;                                 // [2][nlv][4] level bit planes (room for 128 lanes)
   uint8_t* out = nullptr;                             // [128][nolv]
   MsCtl* ctl = nullptr;                               // [4] one per batch
-  int64_t* roots_dev = nullptr;                       // [4][128]
-  int* nroots_dev = nullptr;                          // [4]
-  int64_t* staging = nullptr;                         // pinned: [4][128] roots + [4] counts
+  MsHead* head = nullptr;                             // [4]
+  MsHead* staging = nullptr;                          // pinned [4]
+  MsSums* sums = nullptr;
   MsCtl* h_ctl = nullptr;                             // pinned [4]
-  unsigned long long* stats_dev = nullptr;            // [2][128] and the sums over all vertices
+  unsigned long long* stats_dev = nullptr;            // [2][128]
   unsigned long long* h_stats = nullptr;              // pinned [2][128]: reached, 2 * nedge per lane
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_done = nullptr;
   unsigned grid_full[3] = {0, 0, 0};                  // the whole device's co-resident blocks
@@ -1480,16 +1530,13 @@ static int ms_build_hubs(g500_msbfs* m, uint64_t thresh, uint64_t chunk, uint2**
   return st;
 }
 
-// Enqueue one batch: roots upload, control reset, the persistent kernel, the
-// transpose into out + batch * W * nolv, and the root fix-up.
+// Enqueue one batch: its head's upload, control reset, the persistent kernel and
+// the output pass into the rows the head names.
 static int ms_enqueue_batch(g500_msbfs* m, int b, cudaStream_t s) {
   g500_graph* g = m->g;
   const int W = m->lane_width;
   const int ni = nw_index(W);
-  G500_CUDA(cudaMemcpyAsync(m->roots_dev + b * MS_MAX_LANES, m->staging + b * MS_MAX_LANES,
-                            sizeof(int64_t) * MS_MAX_LANES, cudaMemcpyHostToDevice, s));
-  G500_CUDA(cudaMemcpyAsync(m->nroots_dev + b, reinterpret_cast<int*>(m->staging + 4 * MS_MAX_LANES) + b,
-                            sizeof(int), cudaMemcpyHostToDevice, s));
+  G500_CUDA(cudaMemcpyAsync(m->head + b, m->staging + b, sizeof(MsHead), cudaMemcpyHostToDevice, s));
   G500_CUDA(cudaMemsetAsync(m->ctl + b, 0, sizeof(MsCtl), s));
   MsParams p;
   p.off = g->d_offsets;
@@ -1503,8 +1550,8 @@ static int ms_enqueue_batch(g500_msbfs* m, int b, cudaStream_t s) {
   p.nhubs = m->nhub_rows;
   p.N = m->N;
   p.L = m->L;
-  p.roots = m->roots_dev + b * MS_MAX_LANES;
-  p.nroots_dev = m->nroots_dev + b;
+  p.roots = m->head[b].roots;  // device addresses
+  p.nroots_dev = &m->head[b].nroots;
   p.nlv = g->nlv;
   p.ngv = g->ngv;
   p.hub_tab = m->hub_tab;
@@ -1536,12 +1583,10 @@ static int ms_enqueue_batch(g500_msbfs* m, int b, cudaStream_t s) {
     else if (W == 64) G500_CUDA(cudaLaunchKernelEx(&cfg, sp ? msbfs_kernel<2, false, true> : msbfs_kernel<2, false, false>, p));
     else G500_CUDA(cudaLaunchKernelEx(&cfg, sp ? msbfs_kernel<4, false, true> : msbfs_kernel<4, false, false>, p));
   }
-  uint8_t* out = m->out + (int64_t)b * W * g->nolv;
   const unsigned tg = (unsigned)std::min<int64_t>(ceil_div(g->nolv, 4 * TR_BLOCK), (int64_t)num_sms() * 8);
-  if (W == 32) ms_transpose_kernel<1><<<tg, TR_BLOCK, 0, s>>>(m->L, m->V, g->d_reorder, g->nlv, g->nolv, m->nroots_dev + b, m->ctl + b, out);
-  else if (W == 64) ms_transpose_kernel<2><<<tg, TR_BLOCK, 0, s>>>(m->L, m->V, g->d_reorder, g->nlv, g->nolv, m->nroots_dev + b, m->ctl + b, out);
-  else ms_transpose_kernel<4><<<tg, TR_BLOCK, 0, s>>>(m->L, m->V, g->d_reorder, g->nlv, g->nolv, m->nroots_dev + b, m->ctl + b, out);
-  ms_root_fixup_kernel<<<1, MS_MAX_LANES, 0, s>>>(m->roots_dev + b * MS_MAX_LANES, m->nroots_dev + b, g->nolv, out);
+  if (W == 32) ms_transpose_kernel<1><<<tg, TR_BLOCK, 0, s>>>(m->L, m->V, g->d_reorder, g->nlv, g->nolv, m->head + b, m->ctl + b);
+  else if (W == 64) ms_transpose_kernel<2><<<tg, TR_BLOCK, 0, s>>>(m->L, m->V, g->d_reorder, g->nlv, g->nolv, m->head + b, m->ctl + b);
+  else ms_transpose_kernel<4><<<tg, TR_BLOCK, 0, s>>>(m->L, m->V, g->d_reorder, g->nlv, g->nolv, m->head + b, m->ctl + b);
   G500_CUDA(cudaGetLastError());
   return G500_OK;
 }
@@ -1572,17 +1617,18 @@ extern "C" int g500_msbfs_create(g500_graph* g, g500_msbfs** out) {
   slab.add(&m->marks, 4 * m->nwords);       // frontier and touched bitmaps
   slab.add(&m->out, (int64_t)MS_MAX_LANES * g->nolv);  // output levels
   slab.add(&m->ctl, 4);
-  slab.add(&m->roots_dev, 4 * MS_MAX_LANES);
-  slab.add(&m->nroots_dev, 4);
-  slab.add(&m->stats_dev, 2 * MS_MAX_LANES + 2);
+  slab.add(&m->head, 4);
+  slab.add(&m->sums, 1);
+  slab.add(&m->stats_dev, 2 * MS_MAX_LANES);
   if (st == G500_OK) st = slab.alloc(&m->slab, "multi-source masks and levels");
+  if (st == G500_OK) chk(cudaMemsetAsync(m->sums, 0, sizeof(MsSums), m->stream), "root sums");
   if (st == G500_OK && g->nlv > 0) {
     const unsigned dgrid = (unsigned)std::min<int64_t>(ceil_div(g->nlv, 256), (int64_t)num_sms() * 8);
     ms_degree_kernel<<<dgrid, 256, 0, m->stream>>>(g->d_offsets, g->nlv, m->deg);
     chk(cudaGetLastError(), "row lengths");
   }
   if (st == G500_OK)
-    chk(cudaHostAlloc(&m->staging, sizeof(int64_t) * (4 * MS_MAX_LANES + 4), cudaHostAllocDefault), "cudaHostAlloc");
+    chk(cudaHostAlloc(&m->staging, sizeof(MsHead) * 4, cudaHostAllocDefault), "cudaHostAlloc");
   if (st == G500_OK) chk(cudaHostAlloc(&m->h_ctl, sizeof(MsCtl) * 4, cudaHostAllocDefault), "cudaHostAlloc");
   chk(cudaEventCreate(&m->ev0), "cudaEventCreate");
   chk(cudaEventCreate(&m->ev1), "cudaEventCreate");
@@ -1632,27 +1678,33 @@ extern "C" int g500_msbfs_set_params(g500_msbfs* m, int lane_width, double alpha
 // Per-lane reached / 2*nedge of the last launch into h_stats (enqueued on s).
 static int ms_enqueue_stats(g500_msbfs* m, int nroots, cudaStream_t s) {
   g500_graph* g = m->g;
-  G500_CUDA(cudaMemsetAsync(m->stats_dev, 0, sizeof(unsigned long long) * (2 * MS_MAX_LANES + 2), s));
   const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(std::max<int64_t>(g->nlv, 1), 256), num_sms() * 8);
   const int W = m->lane_width;
-  unsigned long long* r = m->stats_dev;
-  unsigned long long* e = m->stats_dev + MS_MAX_LANES;
-  unsigned long long* all = m->stats_dev + 2 * MS_MAX_LANES;
-  if (g->nlv > 0) {
-    if (W == 32) ms_stats_kernel<1><<<grid, 256, 0, s>>>(m->V, g->d_vis_init, g->d_endp, g->nlv, nroots, r, e, all);
-    else if (W == 64) ms_stats_kernel<2><<<grid, 256, 0, s>>>(m->V, g->d_vis_init, g->d_endp, g->nlv, nroots, r, e, all);
-    else ms_stats_kernel<4><<<grid, 256, 0, s>>>(m->V, g->d_vis_init, g->d_endp, g->nlv, nroots, r, e, all);
-  }
-  ms_root_stats_kernel<<<1, MS_MAX_LANES, 0, s>>>(m->roots_dev, m->nroots_dev, g->d_reorder, g->nlv, g->d_endp,
-                                                  all, r, e);
+  if (W == 32) ms_stats_kernel<1><<<grid, 256, 0, s>>>(m->V, g->d_vis_init, g->d_endp, g->nlv, nroots, m->head, g->d_reorder, m->sums, m->stats_dev);
+  else if (W == 64) ms_stats_kernel<2><<<grid, 256, 0, s>>>(m->V, g->d_vis_init, g->d_endp, g->nlv, nroots, m->head, g->d_reorder, m->sums, m->stats_dev);
+  else ms_stats_kernel<4><<<grid, 256, 0, s>>>(m->V, g->d_vis_init, g->d_endp, g->nlv, nroots, m->head, g->d_reorder, m->sums, m->stats_dev);
   G500_CUDA(cudaGetLastError());
   G500_CUDA(cudaMemcpyAsync(m->h_stats, m->stats_dev, sizeof(unsigned long long) * 2 * MS_MAX_LANES,
                             cudaMemcpyDeviceToHost, s));
   return G500_OK;
 }
 
+// Whether the output pass can write a level row at p itself.
+static bool ms_direct_row(const g500_msbfs* m, const void* p) {
+  if (reinterpret_cast<uintptr_t>(p) & 3) return false;
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeDevice && a.device == m->g->device;
+}
+
 // Enqueue a whole call (every launch, the optional level copy, the control
 // blocks' copy back, the optional root statistics) and record ev_done.
+// Rows in device memory are written by the output pass itself; levels also stay
+// in m->out for g500_msbfs_device_levels.  With root_dsts (the serving loop,
+// whose handles nobody reads) a row goes only where it is wanted.
 static int ms_launch(g500_msbfs* m, const int64_t* roots, int nroots, uint8_t* levels, int levels_on_device,
                      uint8_t* const* root_dsts = nullptr) {
   if (!m || !roots) return set_error(G500_E_INVAL, "null argument");
@@ -1668,11 +1720,23 @@ static int ms_launch(g500_msbfs* m, const int64_t* roots, int nroots, uint8_t* l
   const int W = m->lane_width;
   const int ni = nw_index(W);
   const int batches = (nroots + W - 1) / W;
-  int* counts = reinterpret_cast<int*>(m->staging + 4 * MS_MAX_LANES);
+  const bool levels_direct = levels && levels_on_device && ms_direct_row(m, levels);
+  bool copied[MS_MAX_LANES];  // root_dsts: the row is copied after the launch
   for (int b = 0; b < 4; ++b) {
-    const int n = b < batches ? std::min(W, nroots - b * W) : 0;
-    counts[b] = n;
-    for (int i = 0; i < MS_MAX_LANES; ++i) m->staging[b * MS_MAX_LANES + i] = i < n ? roots[b * W + i] : 0;
+    MsHead& h = m->staging[b];
+    h.nroots = b < batches ? std::min(W, nroots - b * W) : 0;
+    h.second = levels_direct ? 1 : 0;
+    for (int i = 0; i < h.nroots; ++i) {
+      const int r = b * W + i;
+      uint8_t* own = m->out + (int64_t)r * g->nolv;
+      h.roots[i] = roots[r];
+      h.row[0][i] = own;
+      h.row[1][i] = levels_direct ? levels + (int64_t)r * g->nolv : nullptr;
+      if (root_dsts) {
+        copied[r] = root_dsts[r] && !ms_direct_row(m, root_dsts[r]);
+        if (!copied[r]) h.row[0][i] = root_dsts[r];
+      }
+    }
   }
   cudaStream_t s = m->stream;
   G500_CUDA(cudaEventRecord(m->ev0, s));
@@ -1701,13 +1765,13 @@ static int ms_launch(g500_msbfs* m, const int64_t* roots, int nroots, uint8_t* l
     }
   }
   G500_CUDA(cudaEventRecord(m->ev1, s));
-  if (levels) {
+  if (levels && !levels_direct) {
     G500_CUDA(cudaMemcpyAsync(levels, m->out, (size_t)nroots * g->nolv,
                               levels_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s));
   }
   if (root_dsts)
     for (int i = 0; i < nroots; ++i)
-      if (root_dsts[i])
+      if (copied[i])
         G500_CUDA(cudaMemcpyAsync(root_dsts[i], m->out + (int64_t)i * g->nolv, (size_t)g->nolv, cudaMemcpyDefault, s));
   G500_CUDA(cudaMemcpyAsync(m->h_ctl, m->ctl, sizeof(MsCtl) * batches, cudaMemcpyDeviceToHost, s));
   m->fl_stats = m->want_stats && batches == 1;
@@ -1750,7 +1814,7 @@ static int ms_complete(g500_msbfs* m, g500_msbfs_stats* stats) {
       if (c.t_init_ns >= c.t0_ns) stats->init_ms += (double)(c.t_init_ns - c.t0_ns) * 1e-6;
       if (c.t_end_ns >= c.t_init_ns) stats->search_ms += (double)(c.t_end_ns - c.t_init_ns) * 1e-6;
     }
-    stats->kernel_launches = 3 * batches + (m->fl_stats ? 2 : 0);
+    stats->kernel_launches = 2 * batches + (m->fl_stats ? 1 : 0);
   }
   return G500_OK;
 }

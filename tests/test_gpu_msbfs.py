@@ -208,3 +208,23 @@ def test_msbfs_levels_across_bit_planes_and_stats(g500, depth, vr):
             assert list(zip(*(a.tolist() for a in ms.root_stats(len(roots))))) == stats, (lanes, sparse)
         ms.close()
     bfs.close()
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2, 3, 4])
+@pytest.mark.parametrize("lanes,n", [(32, 70), (64, 64), (128, 5)])
+def test_msbfs_levels_into_device_memory(g500, s13, offset, lanes, n):
+    """Rows in device memory are written by the output pass when they are 4-byte aligned and copied otherwise;
+    the handle's own output holds the levels too, and nothing beyond the rows is written."""
+    import torch
+    g, og, roots, want = s13
+    rr = np.resize(roots, n)
+    ms = g500.MultiSourceBFS(g, lanes)
+    size = n * g.pred_size()
+    buf = torch.full((size + 16,), 77, dtype=torch.uint8, device="cuda")
+    for _ in range(2):
+        ms.run(rr, buf[offset:offset + size])
+        got = buf.cpu().numpy()
+        assert np.array_equal(got[offset:offset + size].reshape(n, -1), np.resize(want, (n, g.pred_size())))
+        assert (got[:offset] == 77).all() and (got[offset + size:] == 77).all()
+        assert np.array_equal(ms.device_levels(n).cpu().numpy(), got[offset:offset + size].reshape(n, -1))
+    ms.close()

@@ -218,3 +218,38 @@ def test_msbfs_async_launch_and_small_grid(g500, served):
         assert list(reached) == [int((lv[i] != 255).sum()) for i in range(len(roots))]
     assert ms.grid(64)[0] == 24
     ms.close()
+
+
+def test_rows_in_device_host_and_no_memory(g500):
+    """A batch whose rows go to aligned and unaligned device memory, pinned and pageable host memory and nowhere:
+    each buffer holds exactly its query's levels."""
+    import torch
+    g = g500.Graph2DCSR.generate(13, 16, 2)
+    n = g.pred_size()
+    roots = g500.find_roots(g, 40)
+    ms = g500.MultiSourceBFS(g, 64)
+    want = ms.levels(roots)
+    ms.close()
+    srv = g500.Server([g], plain_below=0)
+    dev = torch.full((len(roots), n + 16), 77, dtype=torch.uint8, device="cuda")
+    pinned = torch.full((len(roots), n), 77, dtype=torch.uint8, pin_memory=True).numpy()
+    pageable = np.full((len(roots), n), 77, np.uint8)
+    for _ in range(2):
+        for i, r in enumerate(roots):
+            kind = i % 5
+            buf = (dev[i, :n], dev[i, 3:3 + n], pinned[i], pageable[i], None)[kind]
+            srv.submit(0, int(r), i, buf)
+        srv.drain()
+        res = sorted(srv.poll(len(roots)), key=lambda q: q["tag"])
+        assert [q["status"] for q in res] == [0] * len(roots)
+        host = dev.cpu().numpy()
+        for i in range(len(roots)):
+            kind = i % 5
+            if kind == 0:
+                assert np.array_equal(host[i, :n], want[i]) and (host[i, n:] == 77).all()
+            elif kind == 1:
+                assert np.array_equal(host[i, 3:3 + n], want[i]) and (host[i, :3] == 77).all()
+            elif kind < 4:
+                assert np.array_equal((pinned, pageable)[kind - 2][i], want[i])
+    srv.close()
+    g.close()

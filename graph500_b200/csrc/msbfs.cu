@@ -279,12 +279,14 @@ __device__ __forceinline__ bool settle(const MsParams& p, uint32_t* Fn, int64_t 
 // Each row is its own only writer, so it settles at once (next frontier,
 // visited mask, levels): pull levels need no separate apply pass over all
 // vertices, only one over the hub rows.
-// INTO_N (a level that pulls some lanes and pushes the others): a row's
-// finds go into its next mask N, beside the push's, for the apply pass to
-// settle, instead of settling here.
-template <int NW, bool INTO_N, bool COUNT, bool SP>
-__device__ void ms_pull_rows(const MsParams& p, const Mask<NW>& act, const uint32_t* Fc, uint32_t* Fn,
-                             uint32_t level, LevelAcc<NW>& la) {
+// MIXED (a level that pushed some lanes first and pulls the others, pm): a row
+// walks only for the lanes pulled and settles its finds together with what the
+// push left in its next mask N, so that such a level needs no apply pass either:
+// pulling into N by atomics beside the push and settling every vertex afterwards
+// took 3-5 % longer (SCALE 24, 64 roots: level 3 905 -> 867 us).
+template <int NW, bool MIXED, bool COUNT, bool SP>
+__device__ void ms_pull_rows(const MsParams& p, const Mask<NW>& act, const Mask<NW>& pm, const uint32_t* Fc,
+                             uint32_t* Fn, uint32_t level, LevelAcc<NW>& la) {
   const int lane = threadIdx.x & 31;
   for (int64_t base = gwarp_id() * 32; base < p.nlv; base += gwarp_count() * 32) {
     const int64_t v = base + lane;
@@ -302,7 +304,7 @@ __device__ void ms_pull_rows(const MsParams& p, const Mask<NW>& act, const uint3
       vv = load_mask<NW>(p.V + v * NW);
 #pragma unroll
       for (int k = 0; k < NW; ++k) {
-        need.w[k] = act.w[k] & ~vv.w[k];
+        need.w[k] = pm.w[k] & ~vv.w[k];  // lanes to walk for
         any |= need.w[k] != 0;
       }
       if (any) {
@@ -376,19 +378,32 @@ __device__ void ms_pull_rows(const MsParams& p, const Mask<NW>& act, const uint3
     }
     // hub rows settle after the hub phase (deg is 0 here for rows without needed lanes)
     bool app = false;
+    if constexpr (MIXED) {
+      bool more = false;  // lanes left of any kind: the row's length, if the walk did not need it
+#pragma unroll
+      for (int k = 0; k < NW; ++k) more |= (act.w[k] & ~vv.w[k]) != 0;
+      if (v < p.nlv && more && !any) deg = __ldg(p.deg + v);
+    }
     if (v < p.nlv && deg <= (uint32_t)MS_HUB_DEG) {
       Mask<NW> nw;
 #pragma unroll
       for (int k = 0; k < NW; ++k) nw.w[k] = acc.w[k] & need.w[k];
-      if constexpr (INTO_N) {
+      if constexpr (MIXED) {
+        const Mask<NW> n = load_mask<NW>(p.N + v * NW);
+        Mask<NW> zero;
+        bool pushed = false;
 #pragma unroll
-        for (int k = 0; k < NW; ++k)
-          if (nw.w[k]) atomicOr(p.N + v * NW + k, nw.w[k]);
-      } else {
-        app = settle<NW>(p, Fn, v, vv, need, nw, deg, level, la);
+        for (int k = 0; k < NW; ++k) {
+          need.w[k] = act.w[k] & ~vv.w[k];
+          nw.w[k] |= n.w[k] & need.w[k];
+          pushed |= n.w[k] != 0;
+          zero.w[k] = 0;
+        }
+        if (pushed) store_mask<NW>(p.N + v * NW, zero);
       }
+      app = settle<NW>(p, Fn, v, vv, need, nw, deg, level, la);
     }
-    if constexpr (SP && !INTO_N) {  // the warp's 32 vertices are one word of the frontier bitmap
+    if constexpr (SP) {  // the warp's 32 vertices are one word of the frontier bitmap
       const unsigned word = __ballot_sync(FULL_MASK, app);
       if (lane == 0 && base < p.nlv) la.fb[base >> 5] = word;
     }
@@ -1055,13 +1070,14 @@ __global__ void __launch_bounds__(MS_THREADS, MS_MIN_BLOCKS) msbfs_kernel(MsPara
     const uint32_t* fbc = p.fb[(level - 1) % 3];
     la.track = sparse;
     if (pull && !mixed) {
-      ms_pull_rows<NW, false, COUNT, SP>(p, act, Fc, Fn, level, la);
+      ms_pull_rows<NW, false, COUNT, SP>(p, act, act, Fc, Fn, level, la);
       ms_pull_hubs<NW, COUNT>(p, act, Fc, la);
     } else if (mixed) {
       if constexpr (SP) ms_push_rows_marked<NW, COUNT>(p, Fc, fbc, qm, la);
       else ms_push_rows_dense<NW, COUNT>(p, Fc, qm, la);
       ms_push_hubs<NW, COUNT>(p, Fc, qm, la);
-      ms_pull_rows<NW, true, COUNT, SP>(p, pm, Fc, Fn, level, la);
+      if (!grid_sync<M_NUM>(&ctl->bar, nullptr, sh_acc, nullptr, sh_cnt, &sh_flag)) return;
+      ms_pull_rows<NW, true, COUNT, SP>(p, act, pm, Fc, Fn, level, la);
       ms_pull_hubs<NW, COUNT>(p, pm, Fc, la);
     } else {
       if constexpr (SP) ms_push_rows_marked<NW, COUNT>(p, Fc, fbc, qm, la);
@@ -1074,11 +1090,11 @@ __global__ void __launch_bounds__(MS_THREADS, MS_MIN_BLOCKS) msbfs_kernel(MsPara
     // Rows that pull settle themselves; without hub rows (none under 2^20
     // entries) such a level has nothing left to wait for.  At SCALE 18 the
     // barrier and the empty pass were 4 of a pull level's 9-13 us.
-    const bool settled = pull && !mixed && p.nhubs == 0;
+    const bool settled = pull && p.nhubs == 0;
     if (!settled && !grid_sync<M_NUM>(&ctl->bar, nullptr, sh_acc, nullptr, sh_cnt, &sh_flag)) return;
     if (tid == 0 && !settled) ctl->level_mid_ns[level] = globaltimer();
     if (settled) {
-    } else if (pull && !mixed) ms_settle_hubs<NW, SP>(p, act, Fn, level, la);
+    } else if (pull) ms_settle_hubs<NW, SP>(p, act, Fn, level, la);
     else if (sparse) ms_apply_marked<NW>(p, act, Fn, level, la);
     else ms_apply<NW, SP>(p, act, Fn, level, la);
     flush_level<NW, COUNT>(la, sh_acc, sh_or, alive);

@@ -228,3 +228,32 @@ def test_msbfs_levels_into_device_memory(g500, s13, offset, lanes, n):
         assert (got[:offset] == 77).all() and (got[offset + size:] == 77).all()
         assert np.array_equal(ms.device_levels(n).cpu().numpy(), got[offset:offset + size].reshape(n, -1))
     ms.close()
+
+
+@pytest.mark.parametrize("lane_width", [32, 64, 128])
+@pytest.mark.parametrize("alpha", [15.0, 1e6])
+@pytest.mark.parametrize("sparse", [True, False])
+def test_msbfs_mixed_levels_on_hub_rows(g500, star, lane_width, alpha, sparse):
+    """Lanes pulled and pushed at one level, with the hub row (over 2^20 entries) reached by pushed lanes while
+    others pull: roots on the star's leaves take the hub at level 1 and everything at level 2, roots on the
+    path reach it at levels 2 to 5."""
+    g, _, _ = star
+    leaves = (1 << 20) + 300
+    roots = np.array([17, 123456, leaves, 99] + [leaves + 1 + i for i in (0, 1, 2, 3, 0)] + [5, 0], np.int64)
+    bfs = g500.BfsOnGPU()
+    bfs.graph_ = g
+    bfs.prepare_bfs()
+    pred = np.zeros(g.pred_size(), np.int64)
+    want, stats = [], []
+    for r in roots:
+        st = bfs.run_bfs(int(r), pred)
+        want.append(as_u8(g500.levels_from_pred(pred)))
+        stats.append((st.reached, st.nedge))
+    bfs.end_bfs()
+    ms = g500.MultiSourceBFS(g, lane_width, alpha)
+    ms.set_sparse(sparse)
+    for _ in range(2):
+        assert np.array_equal(ms.levels(roots), np.array(want))
+        assert list(zip(*(a.tolist() for a in ms.root_stats(len(roots))))) == stats
+    assert any(lv["pull"] == 2 for lv in ms.level_info()), ms.level_info()
+    ms.close()

@@ -1025,7 +1025,7 @@ static int bfs_free(g500_bfs* b) {
   if (b->stream) cudaStreamSynchronize(b->stream);
   pred_expander_free(b);
   dev_free(b->d_slab);
-  dev_free(b->d_pred_r);
+  if (b->owns_pred_r) dev_free(b->d_pred_r);
   dev_free(b->d_levels);
   dev_free(b->d_overflow);
   if (b->ev_done) cudaEventDestroy(b->ev_done);
@@ -1070,7 +1070,10 @@ static int make_params(g500_bfs* b, int64_t root, int64_t* pred, RunParams* out)
   if (mode == 0) mode = (uint64_t)g->nolv * 8 > BFS_DEFERRED_PRED_BYTES ? 3 : 1;
   if (mode == 3 && (b->pack_off || g->nolv > (1ll << PACK_SHIFT))) mode = 2;
   p.deferred = mode == 1 ? 0 : (mode == 2 ? 1 : 2);
-  if (p.deferred && !b->d_pred_r) G500_TRY(dev_alloc_n(&b->d_pred_r, std::max<int64_t>(g->nlv, 1), "deferred pred"));
+  if (p.deferred && !b->d_pred_r) {  // a mode asked for on a graph that defaults to another
+    G500_TRY(dev_alloc_n(&b->d_pred_r, std::max<int64_t>(g->nlv, 1), "deferred pred"));
+    b->owns_pred_r = 1;
+  }
   p.pred_r = b->d_pred_r;
   p.pred_p = reinterpret_cast<uint32_t*>(b->d_pred_r);
   p.big = b->d_big;
@@ -1145,6 +1148,7 @@ extern "C" int g500_bfs_create(g500_graph* g, g500_bfs** out) {
   slab.add(&b->d_rec, MAX_LEVELS);
   slab.add(&b->d_big, BIG_ROWS);
   slab.add(&b->d_endw, nwords);
+  if ((uint64_t)g->nolv * 8 > BFS_DEFERRED_PRED_BYTES) slab.add(&b->d_pred_r, std::max<int64_t>(g->nlv, 1));
   if (st == G500_OK) st = slab.alloc(&b->d_slab, "pred, visited bitmaps and top-down queues");
   if (st == G500_OK && g->nlv > 0) {
     const unsigned wg = (unsigned)std::min<int64_t>(ceil_div(nwords * 32, 256), (int64_t)num_sms() * 8);

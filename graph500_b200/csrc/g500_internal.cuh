@@ -220,6 +220,7 @@ struct g500_bfs {
   void* d_slab = nullptr;            // the allocation of pred, vis, queue, ctl, rec, big and endw
   int64_t* d_pred = nullptr;         // [nolv]
   int64_t* d_pred_r = nullptr;       // [nlv] deferred mode: pred entries by reordered id
+  int owns_pred_r = 0;               // ... in an allocation of its own
   uint8_t* d_levels = nullptr;       // [nolv] levels of an asynchronous run (serving)
   unsigned* d_overflow = nullptr;    // a level over 254 in d_levels
   cudaEvent_t ev_done = nullptr;

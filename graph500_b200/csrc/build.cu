@@ -416,7 +416,7 @@ static int build_from_device_edges(g500_graph* g, const g500_packed_edge* d_edge
   G500_CUDA(cudaMemcpyAsync(&nge, g->d_offsets + nlv, sizeof(nge), cudaMemcpyDeviceToHost, s));
   G500_CUDA(cudaStreamSynchronize(s));
   g->nge = (int64_t)nge;
-  G500_TRY(dev_alloc_n(&g->d_cols, (int64_t)nge, "adjacency"));
+  G500_TRY(dev_alloc_n(&g->d_cols, (int64_t)nge + COLS_PAD, "adjacency"));
   if (nk > 0) {
     unique_write_kernel<<<(unsigned)ntiles, CP_THREADS, 0, s>>>(sorted, nk, lb, tile_offsets, g->d_cols);
     G500_CUDA(cudaGetLastError());

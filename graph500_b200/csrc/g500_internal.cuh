@@ -32,6 +32,7 @@ constexpr unsigned FULL_MASK = 0xFFFFFFFFu;
 constexpr int64_t LOCAL_VERTS_UNIT = 65536;  // max(11, 16) bits, bfs.hpp:109 + graph_constructor.hpp:557
 constexpr int TD_CHUNK = 128;                // edges per top-down work item (one warp pass)
 constexpr uint32_t NO_VERTEX = 0xFFFFFFFFu;
+constexpr int64_t COLS_PAD = 4;              // entries after the adjacency, for aligned 16-byte loads at its end
 // first[v] of a row with more than one edge carries FIRST_MORE (when the graph
 // has first_flags: every reordered id then fits in 31 bits), so that a
 // bottom-up miss on a one-edge row needs no further scan

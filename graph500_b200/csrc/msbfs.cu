@@ -313,15 +313,17 @@ __device__ void ms_pull_rows(const MsParams& p, const Mask<NW>& act, const Mask<
       }
     }
     if (any && deg <= (uint32_t)MS_SMALL_DEG) {
+      // one aligned 16-byte load per step (the adjacency is padded): four loads
+      // of a lane's own row each cost a pass through L1, as many as the masks
+      static_assert(MS_UNROLL == 4, "one uint4 of neighbours per step");
       const uint64_t re = rb + deg;
-      uint64_t e = rb;
+      uint64_t e = rb & ~uint64_t(3);
       for (; e < re; e += MS_UNROLL) {
-        uint32_t nb[MS_UNROLL];
-#pragma unroll
-        for (int t = 0; t < MS_UNROLL; ++t) nb[t] = e + t < re ? __ldg(p.col + e + t) : NO_VERTEX;
+        const uint4 q4 = __ldg(reinterpret_cast<const uint4*>(p.col + e));
+        const uint32_t nb[MS_UNROLL] = {q4.x, q4.y, q4.z, q4.w};
 #pragma unroll
         for (int t = 0; t < MS_UNROLL; ++t)
-          if (nb[t] != NO_VERTEX) {
+          if (e + t >= rb && e + t < re) {
             const Mask<NW> f = gather_mask<NW>(Fc + (int64_t)nb[t] * NW);
 #pragma unroll
             for (int q = 0; q < NW; ++q) acc.w[q] |= f.w[q];

@@ -160,7 +160,7 @@ extern "C" int g500_graph_load(const char* path, int device, g500_graph** out) {
   g->gen_seconds = h.gen_seconds;
   g->build_seconds = h.build_seconds;
   int st = graph_alloc_maps(g);
-  if (st == G500_OK) st = dev_alloc_n(&g->d_cols, std::max<int64_t>(h.nge, 1), "cols");
+  if (st == G500_OK) st = dev_alloc_n(&g->d_cols, h.nge + COLS_PAD, "cols");
   if (st == G500_OK && h.num_edges > 0) {
     st = dev_alloc_n(&g->d_edges, h.num_edges, "edge list");
     g->owns_edges = true;

@@ -38,7 +38,7 @@ constexpr int64_t MS_SMALL_VERTS = 3 << 17, MS_MEDIUM_VERTS = 1 << 20;  // grid 
 constexpr int MS_MAX_LEVEL = 254;  // level bytes: 255 marks unreached
 // M_ROWS / M_SECT (counting launches only): row and chunk offset reads, and
 // the 32-byte adjacency sectors the level's entries span
-enum MsCounter { M_NEW = 0, M_NF, M_MF, M_MU, M_EDGES, M_ROWS, M_SECT, M_NUM = 8 };
+enum MsCounter { M_NEW = 0, M_MF, M_MU, M_EDGES, M_ROWS, M_SECT, M_NUM };
 enum MsErr { MS_ERR_DEPTH = 4 };
 
 // What a launch needs from the host, in one upload.
@@ -226,13 +226,15 @@ __device__ __forceinline__ unsigned long long sector_span(uint64_t b, uint64_t k
 // the level's frontier bitmap, track whether its push marks touched vertices.
 template <int NW>
 struct LevelAcc {
-  unsigned long long nnew, nf, mf, mu;
+  unsigned long long mf, mu;
+  uint32_t nnew;  // per thread: at most 128 lanes of each of its rows
   unsigned long long rows, sect;  // counting launches only
   Mask<NW> lanes;  // lanes that found vertices
   uint32_t* fb;
   bool track;
   __device__ void clear() {
-    nnew = nf = mf = mu = rows = sect = 0;
+    mf = mu = rows = sect = 0;
+    nnew = 0;
 #pragma unroll
     for (int k = 0; k < NW; ++k) lanes.w[k] = 0;
   }
@@ -264,7 +266,6 @@ __device__ __forceinline__ bool settle(const MsParams& p, uint32_t* Fn, int64_t 
       a.lanes.w[k] |= nw.w[k];
       a.nnew += __popc(nw.w[k]);
     }
-    ++a.nf;
     a.mf += deg;
   }
   if (left) a.mu += deg;  // still has unvisited live lanes after this level
@@ -288,29 +289,62 @@ template <int NW, bool MIXED, bool COUNT, bool SP>
 __device__ void ms_pull_rows(const MsParams& p, const Mask<NW>& act, const Mask<NW>& pm, const uint32_t* Fc,
                              uint32_t* Fn, uint32_t level, LevelAcc<NW>& la) {
   const int lane = threadIdx.x & 31;
-  for (int64_t base = gwarp_id() * 32; base < p.nlv; base += gwarp_count() * 32) {
-    const int64_t v = base + lane;
-    Mask<NW> need, acc, vv;
+  const int64_t stride = gwarp_count() * 32;
+  // The loads of a row wait for one another (visited mask, row start, neighbours,
+  // their masks), and a launch is bound by that (two thirds of its stalls at SCALE
+  // 23), so the mask is loaded two rows ahead, the row start one, and a walk's
+  // next neighbours while it gathers: 64 lanes at SCALE 24 search 1826 -> 1716 us,
+  // 32 at SCALE 18 82 -> 78.  128 lanes have no registers for it (spills, 4 %
+  // slower; three blocks per SM instead of four with the registers: 2-5 % faster
+  // up to SCALE 21, 6-9 % slower from SCALE 23).
+  constexpr bool AHEAD = NW <= 2;
+  Mask<NW> vnext, vafter;
+  uint64_t rb_next = 0;
+  uint32_t deg_next = 0;
+  const auto load_row = [&](int64_t v, const Mask<NW>& m) {  // a visited mask of all ones: no such row
+    bool left = false;
+#pragma unroll
+    for (int k = 0; k < NW; ++k) left |= (act.w[k] & ~m.w[k]) != 0;
+    deg_next = 0;
+    if (left) {
+      rb_next = __ldg(p.off + v);
+      deg_next = __ldg(p.deg + v);
+    }
+  };
+  const auto load_visited = [&](int64_t v) {
+    Mask<NW> m;
+#pragma unroll
+    for (int k = 0; k < NW; ++k) m.w[k] = ~0u;
+    if (v < p.nlv) m = load_mask<NW>(p.V + v * NW);
+    return m;
+  };
+  if constexpr (AHEAD) {
+    const int64_t first = gwarp_id() * 32 + lane;
+    vnext = load_visited(first);
+    vafter = load_visited(first + stride);
+    load_row(first, vnext);
+  }
+  for (int64_t base = gwarp_id() * 32; base < p.nlv; base += stride) {
+    const int64_t v = base + lane;  // nlv is a multiple of 32
+    if constexpr (!AHEAD) {
+      vnext = load_visited(v);
+      load_row(v, vnext);
+    }
+    const Mask<NW> vv = vnext;
+    const uint64_t rb = rb_next;
+    const uint32_t deg = deg_next;  // 0 for a row without live lanes left
+    if constexpr (AHEAD) {
+      vnext = vafter;
+      load_row(v + stride, vnext);
+      vafter = load_visited(v + 2 * stride);
+    }
+    Mask<NW> need, acc;
     bool any = false;
-    uint32_t deg = 0;
-    uint64_t rb = 0;
 #pragma unroll
     for (int k = 0; k < NW; ++k) {
       acc.w[k] = 0;
-      need.w[k] = 0;
-      vv.w[k] = 0;
-    }
-    if (v < p.nlv) {
-      vv = load_mask<NW>(p.V + v * NW);
-#pragma unroll
-      for (int k = 0; k < NW; ++k) {
-        need.w[k] = pm.w[k] & ~vv.w[k];  // lanes to walk for
-        any |= need.w[k] != 0;
-      }
-      if (any) {
-        rb = __ldg(p.off + v);
-        deg = __ldg(p.deg + v);
-      }
+      need.w[k] = pm.w[k] & ~vv.w[k];  // lanes to walk for
+      any |= need.w[k] != 0;
     }
     if (any && deg <= (uint32_t)MS_SMALL_DEG) {
       // one aligned 16-byte load per step (the adjacency is padded): four loads
@@ -318,9 +352,13 @@ __device__ void ms_pull_rows(const MsParams& p, const Mask<NW>& act, const Mask<
       static_assert(MS_UNROLL == 4, "one uint4 of neighbours per step");
       const uint64_t re = rb + deg;
       uint64_t e = rb & ~uint64_t(3);
+      uint4 ahead;
+      if constexpr (AHEAD) ahead = __ldg(reinterpret_cast<const uint4*>(p.col + e));
       for (; e < re; e += MS_UNROLL) {
-        const uint4 q4 = __ldg(reinterpret_cast<const uint4*>(p.col + e));
-        const uint32_t nb[MS_UNROLL] = {q4.x, q4.y, q4.z, q4.w};
+        if constexpr (!AHEAD) ahead = __ldg(reinterpret_cast<const uint4*>(p.col + e));
+        const uint32_t nb[MS_UNROLL] = {ahead.x, ahead.y, ahead.z, ahead.w};
+        if constexpr (AHEAD)
+          if (e + MS_UNROLL < re) ahead = __ldg(reinterpret_cast<const uint4*>(p.col + e + MS_UNROLL));
 #pragma unroll
         for (int t = 0; t < MS_UNROLL; ++t)
           if (e + t >= rb && e + t < re) {
@@ -380,13 +418,7 @@ __device__ void ms_pull_rows(const MsParams& p, const Mask<NW>& act, const Mask<
     }
     // hub rows settle after the hub phase (deg is 0 here for rows without needed lanes)
     bool app = false;
-    if constexpr (MIXED) {
-      bool more = false;  // lanes left of any kind: the row's length, if the walk did not need it
-#pragma unroll
-      for (int k = 0; k < NW; ++k) more |= (act.w[k] & ~vv.w[k]) != 0;
-      if (v < p.nlv && more && !any) deg = __ldg(p.deg + v);
-    }
-    if (v < p.nlv && deg <= (uint32_t)MS_HUB_DEG) {
+    if (deg <= (uint32_t)MS_HUB_DEG) {
       Mask<NW> nw;
 #pragma unroll
       for (int k = 0; k < NW; ++k) nw.w[k] = acc.w[k] & need.w[k];
@@ -923,7 +955,6 @@ __device__ void flush_level(const LevelAcc<NW>& la, unsigned long long* sh_acc, 
     block_add(sh_acc, M_SECT, la.sect);
   }
   block_add(sh_acc, M_NEW, la.nnew);
-  block_add(sh_acc, M_NF, la.nf);
   block_add(sh_acc, M_MF, la.mf);
   block_add(sh_acc, M_MU, la.mu);
 #pragma unroll

@@ -66,7 +66,7 @@ constexpr int TD_UNROLL = TD_CHUNK / 32;  // virtual edges per lane per pass
 constexpr int BU_WORDS = 4;               // 32-vertex words a warp keeps in flight (bottom-up pass A)
 constexpr int BU_SERIAL = 8;              // row entries a lane checks alone per step (one sector)
 constexpr int BU_LANE_MAX = 64;           // a row with at most this many entries left is scanned by its own lane
-constexpr int BU_LIST = 64;               // unvisited vertices a warp keeps listed (late bottom-up levels)
+constexpr int BU_LIST = 32;               // unvisited vertices a warp keeps listed (late bottom-up levels)
 constexpr int BU_LIST_WORDS = 48;
 // A frontier row of more than BIG_CHUNKS work items is listed whole (up to
 // BIG_ROWS rows per level) instead of cut into items by one warp; the next
@@ -182,6 +182,20 @@ __device__ __forceinline__ void append_row(uint64_t rb, uint64_t deg, uint32_t o
   }
 }
 
+// Per warp: what late bottom-up levels work on (see bu_collect).
+struct WarpLists {
+  uint32_t left[BFS_THREADS / 32][BU_LIST];   // unvisited vertices of the warp's words
+  uint32_t found[BFS_THREADS / 32][BU_LIST];  // found by the last listed level
+  uint32_t nleft[BFS_THREADS / 32], nfound[BFS_THREADS / 32];
+};
+// One piece of shared memory for the phases' own use: what a block takes is
+// missing from its SM's L1, and 8 KB more made the big bottom-up levels 3 %
+// slower.
+union PhaseShared {
+  uint32_t bigpre[BIG_ROWS + 1];  // top-down: chunks of long rows 0 .. i - 1
+  WarpLists lists;                // bottom-up
+};
+
 // Top-down level: expand the work items, claim unvisited targets, and list the
 // discovered (vertex, original id) pairs.  Rows are cut into work items only
 // if the next level is top-down as well (chunk_phase).  The nbig rows listed
@@ -191,8 +205,7 @@ __device__ __forceinline__ void append_row(uint64_t rb, uint64_t deg, uint32_t o
 template <int DEF>
 __device__ void td_phase(const RunParams& p, const TdItem* __restrict__ q_in, int64_t qn, int64_t nbig, uint32_t* vis,
                          uint2* __restrict__ found_list, unsigned long long* pos, unsigned long long* sh_acc,
-                         int64_t lvl) {
-  __shared__ uint32_t sh_bigpre[BIG_ROWS + 1];  // sh_bigpre[i] = chunks of big rows 0 .. i-1
+                         uint32_t* sh_bigpre, int64_t lvl) {
   const int lane = threadIdx.x & 31;
   int64_t nall = qn;
   if (nbig > 0) {
@@ -526,12 +539,6 @@ __device__ void bu_level(const RunParams& p, const uint32_t* __restrict__ vis_cu
 // the listed rows.  The visited maps still alternate: a listed level writes the
 // other buffer, which it first brings up to date with its own words (the first
 // such level) or with the vertices it found one level before.
-struct WarpLists {
-  uint32_t left[BFS_THREADS / 32][BU_LIST];   // unvisited vertices of the warp's words
-  uint32_t found[BFS_THREADS / 32][BU_LIST];  // found by the last listed level
-  uint32_t nleft[BFS_THREADS / 32], nfound[BFS_THREADS / 32];
-};
-
 // List what the level leaves; a warp with too many raises C_BIG, which
 // bottom-up levels do not use otherwise.
 __device__ void bu_collect(const RunParams& p, const uint32_t* vis_next, WarpLists& wl, unsigned long long* sh_acc) {
@@ -743,7 +750,8 @@ __global__ void __launch_bounds__(BFS_THREADS, BFS_MIN_BLOCKS) bfs_persistent_ke
   __shared__ unsigned long long sh_cnt[C_NUM];
   __shared__ unsigned long long sh_acc[C_NUM];
   __shared__ unsigned sh_flag;
-  __shared__ WarpLists lists;
+  __shared__ PhaseShared sh_phase;
+  WarpLists& lists = sh_phase.lists;
   BfsCtl* ctl = p.ctl;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
@@ -825,7 +833,7 @@ __global__ void __launch_bounds__(BFS_THREADS, BFS_MIN_BLOCKS) bfs_persistent_ke
     const int64_t lvl = (int64_t)level << 48;
     unsigned long long disc, scan = 0, edges, sect, front = 0, listed = 0, t_mid = 0, mf = 0;
     if (forward) {
-      td_phase<DEF>(p, items, qn, nbig, p.vis[cur_vis], found_list, ctl->pos[phase % 3], sh_acc, lvl);
+      td_phase<DEF>(p, items, qn, nbig, p.vis[cur_vis], found_list, ctl->pos[phase % 3], sh_acc, sh_phase.bigpre, lvl);
       if (!grid_sync_sum<C_NUM>(cnt, &ctl->bar, sh_acc, sh_cnt)) return;
       if (tid == 0) t_mid = globaltimer();
       ++phase;

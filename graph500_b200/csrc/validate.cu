@@ -32,6 +32,7 @@ constexpr int VAL_SHIFT = 27;
 constexpr uint32_t VAL_ID = (1u << VAL_SHIFT) - 1u;
 constexpr uint32_t VAL_NONE = 0xFFFFFFFFu;
 constexpr int VAL_MAX_DEPTH = 30;
+constexpr int VAL_VERTS = 4;  // vertices per thread in flight (vertex and parent passes: 86 / 81 us at SCALE 24 with one)
 
 __device__ __forceinline__ int64_t pred_of(int64_t e) { return (int64_t)((uint64_t)e << 16) >> 16; }  // :809
 __device__ __forceinline__ int depth_of(int64_t e) { return (int)((e >> 48) & 0xFFFF); }              // :813
@@ -44,30 +45,47 @@ __device__ __forceinline__ void warp_add(unsigned long long* dst, unsigned long 
 
 // pack: null, or the packed entries to write; entries that do not fit raise
 // VE_UNPACKED, and the later passes then read pred itself.
-__global__ void val_vertex_kernel(const int64_t* __restrict__ pred, int64_t nlocal, int64_t nglobal, int64_t root,
-                                  uint32_t* __restrict__ pack, unsigned long long* err) {
-  unsigned long long range = 0, self = 0, depth = 0;
+__global__ void __launch_bounds__(256) val_vertex_kernel(const int64_t* __restrict__ pred, int64_t nlocal,
+                                                         int64_t nglobal, int64_t root, uint32_t* __restrict__ pack,
+                                                         unsigned long long* err) {
+  uint32_t range = 0, self = 0, depth = 0;  // per thread: far fewer than 2^32
   bool unpacked = false;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nlocal; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t e = pred[i];
-    const int64_t p = pred_of(e);
-    const int d = depth_of(e);
-    if (pack) {
-      const bool none = p == -1 && d == 0xFFFF;
-      unpacked |= !none && (p < 0 || p > (int64_t)VAL_ID || d > VAL_MAX_DEPTH);
-      pack[i] = none ? VAL_NONE : (uint32_t)p | ((uint32_t)d << VAL_SHIFT);
+  const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < nlocal; i0 += nthreads * VAL_VERTS) {
+    int64_t e[VAL_VERTS], parent[VAL_VERTS];
+    bool look[VAL_VERTS];  // the parent's entry is read, all of them in flight together
+#pragma unroll
+    for (int u = 0; u < VAL_VERTS; ++u) {
+      const int64_t i = i0 + u * nthreads;
+      e[u] = i < nlocal ? pred[i] : -1;
     }
-    if (p < -1 || p >= nglobal) {
-      ++range;
-      continue;
+#pragma unroll
+    for (int u = 0; u < VAL_VERTS; ++u) {
+      const int64_t i = i0 + u * nthreads, p = pred_of(e[u]);
+      look[u] = i < nlocal && p >= 0 && p < nglobal && i != root;  // nglobal <= nlocal
+      parent[u] = look[u] ? pred[p] : 0;
     }
-    if (i != root && p != -1 && p == i) ++self;
-    if (p == -1 && d != 0xFFFF) ++depth;
-    else if (p != -1 && d == 0xFFFF) ++depth;
-    if (i != root && p != -1) {
-      const int64_t pp = pred[p];  // p in [0, nglobal) and nglobal <= nlocal
-      if (depth_of(pp) == 0xFFFF) ++depth;
-      if (d != depth_of(pp) + 1) ++depth;
+#pragma unroll
+    for (int u = 0; u < VAL_VERTS; ++u) {
+      const int64_t i = i0 + u * nthreads, p = pred_of(e[u]);
+      const int d = depth_of(e[u]);
+      if (i >= nlocal) continue;
+      if (pack) {
+        const bool none = p == -1 && d == 0xFFFF;
+        unpacked |= !none && (p < 0 || p > (int64_t)VAL_ID || d > VAL_MAX_DEPTH);
+        pack[i] = none ? VAL_NONE : (uint32_t)p | ((uint32_t)d << VAL_SHIFT);
+      }
+      if (p < -1 || p >= nglobal) {
+        ++range;
+        continue;
+      }
+      if (i != root && p != -1 && p == i) ++self;
+      if (p == -1 && d != 0xFFFF) ++depth;
+      else if (p != -1 && d == 0xFFFF) ++depth;
+      if (look[u]) {
+        if (depth_of(parent[u]) == 0xFFFF) ++depth;
+        if (d != depth_of(parent[u]) + 1) ++depth;
+      }
     }
   }
   warp_add(&err[VE_RANGE], range);
@@ -183,12 +201,23 @@ __global__ void __launch_bounds__(256) val_edge_kernel(const g500_packed_edge* _
   warp_add(&err[VE_COUNT_EDGES], c.count);
 }
 
-__global__ void val_parent_kernel(const int64_t* __restrict__ pred, int64_t nlocal, int64_t root,
-                                  const uint8_t* __restrict__ valid, unsigned long long* err) {
-  unsigned long long missing = 0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nlocal; i += (int64_t)gridDim.x * blockDim.x) {
-    if (i == root || pred_of(pred[i]) == -1) continue;
-    if (!valid[i]) ++missing;
+__global__ void __launch_bounds__(256) val_parent_kernel(const int64_t* __restrict__ pred,
+                                                         const uint32_t* __restrict__ pack, int64_t nlocal,
+                                                         int64_t root, const uint8_t* __restrict__ valid,
+                                                         unsigned long long* err) {
+  const bool use_pack = pack && *(volatile unsigned long long*)&err[VE_UNPACKED] == 0;
+  uint32_t missing = 0;
+  const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < nlocal; i0 += nthreads * VAL_VERTS) {
+    bool reached[VAL_VERTS], ok[VAL_VERTS];
+#pragma unroll
+    for (int u = 0; u < VAL_VERTS; ++u) {
+      const int64_t i = i0 + u * nthreads;
+      reached[u] = i < nlocal && i != root && (use_pack ? pack[i] != VAL_NONE : pred_of(pred[i]) != -1);
+      ok[u] = i < nlocal && valid[i];
+    }
+#pragma unroll
+    for (int u = 0; u < VAL_VERTS; ++u) missing += reached[u] && !ok[u];
   }
   warp_add(&err[VE_MISSING], missing);
 }
@@ -256,7 +285,7 @@ extern "C" int g500_validate(g500_graph* g, const g500_packed_edge* edges, int64
   val_root_kernel<<<1, 1, 0, s>>>(d_pred, root, nlocal, d_err);
   val_vertex_kernel<<<grid, 256, 0, s>>>(d_pred, nlocal, nglobal, root, d_pack, d_err);
   if (m > 0) val_edge_kernel<<<grid, 256, 0, s>>>(d_edges, m, d_pred, d_pack, nlocal, d_valid, d_err);
-  val_parent_kernel<<<grid, 256, 0, s>>>(d_pred, nlocal, root, d_valid, d_err);
+  val_parent_kernel<<<grid, 256, 0, s>>>(d_pred, d_pack, nlocal, root, d_valid, d_err);
   e = cudaGetLastError();
   unsigned long long h[VE_N];
   if (e == cudaSuccess) e = cudaMemcpyAsync(h, d_err, sizeof(h), cudaMemcpyDeviceToHost, s);
@@ -365,7 +394,7 @@ extern "C" int g500_validate_noalloc(const g500_packed_edge* dev_edges, int64_t 
   val_vertex_kernel<<<grid, 256, 0, s>>>(dev_pred, nlocalverts, nglobalverts, root, nullptr, sc.err);
   if (num_edges > 0)
     val_edge_kernel<<<grid, 256, 0, s>>>(dev_edges, num_edges, dev_pred, nullptr, nlocalverts, sc.valid, sc.err);
-  val_parent_kernel<<<grid, 256, 0, s>>>(dev_pred, nlocalverts, root, sc.valid, sc.err);
+  val_parent_kernel<<<grid, 256, 0, s>>>(dev_pred, nullptr, nlocalverts, root, sc.valid, sc.err);
   G500_CUDA(cudaGetLastError());
   unsigned long long h[VE_N];
   G500_CUDA(cudaMemcpyAsync(h, sc.err, sizeof(h), cudaMemcpyDeviceToHost, s));

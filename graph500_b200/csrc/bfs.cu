@@ -1399,14 +1399,16 @@ extern "C" int g500_bfs_run(g500_bfs* b, int64_t root, int64_t* pred, int pred_o
                                         0, s));
   G500_TRY(launch_deferred_pred(p, s));
   G500_CUDA(cudaEventRecord(b->ev1, s));
+  bool packed = false;
   if (!pred_on_device) {
-    bool packed = false;
     G500_TRY(pred_to_host_packed(b, pred, s, &packed));
     if (!packed) G500_CUDA(cudaMemcpyAsync(pred, b->d_pred, sizeof(int64_t) * g->nolv, cudaMemcpyDeviceToHost, s));
   }
   // last, since a copy to pageable memory waits for the run (pinned memory for it would cost 2 ms per handle)
-  G500_CUDA(cudaMemcpyAsync(b->h_ctl, b->d_ctl, sizeof(BfsCtl), cudaMemcpyDeviceToHost, s));
-  G500_CUDA(cudaStreamSynchronize(s));
+  if (!packed) {
+    G500_CUDA(cudaMemcpyAsync(b->h_ctl, b->d_ctl, sizeof(BfsCtl), cudaMemcpyDeviceToHost, s));
+    G500_CUDA(cudaStreamSynchronize(s));
+  }
   b->last_root = root;
   const BfsCtl& c = *b->h_ctl;
   check_ctl(b);

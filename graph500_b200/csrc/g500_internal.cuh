@@ -232,10 +232,9 @@ struct g500_bfs {
   uint8_t* last_levels_dst = nullptr;  // levels destination of the run in flight (a rerun writes it again)
   // a host pred crosses PCIe as packed 32-bit entries, expanded by host threads
   int pack_host_off = 0;
-  uint32_t* d_pack = nullptr;        // [nolv]
-  unsigned* d_pack_ovf = nullptr;
-  uint32_t* h_pack = nullptr;        // pinned [nolv + 64]
-  cudaEvent_t ev_chunk[8] = {};
+  void* d_pack_state = nullptr;
+  uint32_t* h_pack = nullptr;        // pinned [nolv], then the chunks' marks and the control block
+  uint32_t pack_run = 0;
   g500::PredExpander* expander = nullptr;
   uint32_t* d_vis[2] = {nullptr, nullptr};
   TdItem* d_queue[2] = {nullptr, nullptr};
@@ -262,7 +261,7 @@ int bfs_complete(g500_bfs* b, int64_t* reached, int64_t* nedge);
 // Copy the run's pred (b->d_pred) to host_pred as packed entries, expanded by
 // host threads chunk by chunk; *packed = false when the graph or the run
 // does not fit the packed form (the caller then copies the int64 entries).
-// Enqueued on s after the run; returns when host_pred is complete.
+// Enqueued on s after the run; returns when host_pred and b->h_ctl are complete.
 int pred_to_host_packed(g500_bfs* b, int64_t* host_pred, cudaStream_t s, bool* packed);
 void pred_expander_free(g500_bfs* b);
 

@@ -1,13 +1,16 @@
 // pred to a pageable host buffer for g500_bfs_run (the reference's driver
-// allocates pred with plain host memory, main.cc:74-75): the int64 entries
-// cross PCIe as 32-bit packed entries into a pinned staging buffer, in
-// chunks, and host threads expand each chunk into the caller's array while
-// the next one is still being copied.  The runtime's own pageable copy goes
-// through its staging buffers at about half the pinned rate (SCALE 22: 1.96
-// ms for the 34 MB pred against 0.92 ms this way, 0.83 ms by DMA into pinned
-// memory, which stays the path for a pinned pred).  The caller's array holds
-// the same int64 values either way (bfs.hpp:1203, :2470 encoding: parent |
-// level << 48, -1 unreached).
+// allocates pred with plain host memory, main.cc:74-75): a kernel packs the
+// int64 entries into 32 bits and stores them over PCIe into a pinned staging
+// buffer itself, in chunks, marking each when it is complete; host threads,
+// already waiting, expand a chunk into the caller's array while the next ones
+// cross.  The runtime's own pageable copy goes through its staging buffers at
+// about half the pinned rate, and a pack kernel followed by one copy and one
+// event per chunk left the link idle between copies and the threads asleep until
+// the first: 470 -> 390 us a call at SCALE 21, 290 -> 125 at SCALE 16, the search
+// included.  A pinned
+// pred keeps its single DMA copy.  The caller's array holds the same int64
+// values either way (bfs.hpp:1203, :2470 encoding: parent | level << 48, -1
+// unreached).
 //
 // Packed entry: parent original id in the low PACK_BITS bits, the level
 // above it; 0xFFFFFFFF = unreached.  Graphs with more than 2^PACK_BITS ids,
@@ -15,6 +18,8 @@
 #include "g500_internal.cuh"
 
 #include <algorithm>
+#include <atomic>
+#include <chrono>
 #include <condition_variable>
 #include <mutex>
 #include <thread>
@@ -26,40 +31,87 @@ namespace {
 constexpr int PACK_BITS = 27;
 constexpr uint32_t PACK_UNREACHED = 0xFFFFFFFFu;
 constexpr int PACK_MAX_LEVEL = 30;  // level 31 with an all-ones parent would read as unreached
-constexpr int PRED_CHUNKS = 8;
+// Chunks of at least 512 KB of packed entries (a chunk's fences and mark cost
+// about 5 us: with 16 chunks whatever the size a SCALE 18 call took 200 us
+// instead of 153), at most 16.
+constexpr int PRED_CHUNKS = 16;
+constexpr int64_t CHUNK_ENTRIES = 1 << 17;
+inline int chunks_for(int64_t n) {
+  int c = 1;
+  while (c < PRED_CHUNKS && n / (2 * c) >= CHUNK_ENTRIES) c *= 2;
+  return c;
+}
+constexpr int PACK_GROUPS = 2;     // groups of blocks, on alternate chunks: one packs while the other's stores drain
+constexpr int PACK_BLOCKS = 64;    // blocks per group
+constexpr int PACK_THREADS = 256;
 
-__global__ void __launch_bounds__(256) pack_pred_kernel(const int64_t* __restrict__ pred, int64_t n,
-                                                        uint32_t* __restrict__ out, unsigned* overflow) {
-  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
-  bool bad = false;
-  for (int64_t i = 2 * tid; i < n; i += 2 * nthreads) {  // n is even (a multiple of 65536)
-    const longlong2 v = __ldcs(reinterpret_cast<const longlong2*>(pred + i));
-    uint32_t e[2];
-    const long long x[2] = {v.x, v.y};
+// Device state of the packing: blocks that have finished a chunk, and whether
+// any entry did not fit.  Left clear by every run but one with such an entry.
+struct PackState {
+  unsigned done[PRED_CHUNKS];
+  unsigned bad;
+};
+
+// The pinned tail behind the packed entries.
+struct PackTail {
+  volatile uint32_t ready[PRED_CHUNKS];  // run number << 1 | an entry so far did not fit
+  BfsCtl ctl;                            // the run's control block
+};
+
+// Chunk c holds entries [c, c + 1) * n / nchunks (n is a multiple of 65536).
+// A chunk is marked by the last block of its group, after every block's stores
+// have reached host memory (system-wide fences).
+__global__ void __launch_bounds__(PACK_THREADS) pack_to_host_kernel(const int64_t* __restrict__ pred, int64_t n,
+                                                                    int nchunks, uint32_t* __restrict__ out, PackState* st,
+                                                                    volatile uint32_t* ready, uint32_t run) {
+  const int group = blockIdx.x % PACK_GROUPS;
+  const int64_t rank = blockIdx.x / PACK_GROUPS;
+  const int64_t len = n / nchunks;
+  for (int c = group; c < nchunks; c += PACK_GROUPS) {
+    bool bad = false;
+    for (int64_t i = c * len + (rank * PACK_THREADS + threadIdx.x) * 4; i < (c + 1) * len;
+         i += (int64_t)PACK_BLOCKS * PACK_THREADS * 4) {
+      const longlong2 a = __ldcs(reinterpret_cast<const longlong2*>(pred + i));
+      const longlong2 b = __ldcs(reinterpret_cast<const longlong2*>(pred + i + 2));
+      const long long x[4] = {a.x, a.y, b.x, b.y};
+      uint32_t e[4];
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      if (x[k] == -1) {
-        e[k] = PACK_UNREACHED;
-      } else {
-        const uint64_t parent = (uint64_t)x[k] & ((1ull << 48) - 1);
-        const uint64_t level = (uint64_t)x[k] >> 48;
-        bad |= parent >= (1ull << PACK_BITS) || level > (uint64_t)PACK_MAX_LEVEL;
-        e[k] = (uint32_t)parent | ((uint32_t)level << PACK_BITS);
+      for (int k = 0; k < 4; ++k) {
+        if (x[k] == -1) {
+          e[k] = PACK_UNREACHED;
+        } else {
+          const uint64_t parent = (uint64_t)x[k] & ((1ull << 48) - 1);
+          const uint64_t level = (uint64_t)x[k] >> 48;
+          bad |= parent >= (1ull << PACK_BITS) || level > (uint64_t)PACK_MAX_LEVEL;
+          e[k] = (uint32_t)parent | ((uint32_t)level << PACK_BITS);
+        }
       }
+      *reinterpret_cast<uint4*>(out + i) = make_uint4(e[0], e[1], e[2], e[3]);
     }
-    __stcs(reinterpret_cast<uint2*>(out + i), make_uint2(e[0], e[1]));
+    if (bad) atomicOr(&st->bad, 1u);
+    __threadfence_system();
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(&st->done[c], 1u) + 1 == PACK_BLOCKS) {
+      __threadfence_system();
+      st->done[c] = 0;
+      ready[c] = run << 1 | (atomicOr(&st->bad, 0u) ? 1u : 0u);
+    }
   }
-  if (bad) atomicOr(overflow, 1u);
+}
+
+inline void cpu_pause() {
+#if defined(__x86_64__) || defined(__i386__)
+  __builtin_ia32_pause();
+#endif
 }
 
 }  // namespace
 
-// Host threads that expand the chunks: each waits for a chunk's copy event
-// and expands its slice of it, so one wake-up per run serves every chunk.
+// Host threads that expand the chunks: each waits for a chunk's mark and
+// expands its slice of it, so one wake-up per run serves every chunk.
 class PredExpander {
  public:
-  PredExpander(int device, int nthreads) : device_(device), n_(nthreads) {
+  explicit PredExpander(int nthreads) : n_(nthreads) {
     for (int t = 1; t < nthreads; ++t) th_.emplace_back([this, t] { loop(t); });
   }
   ~PredExpander() {
@@ -71,28 +123,32 @@ class PredExpander {
     for (auto& t : th_) t.join();
   }
 
-  // expand src[0, n) into dst; chunk k = [bounds[k], bounds[k+1]) is ready
-  // once ev[k] has completed
-  void run(const uint32_t* src, int64_t* dst, const int64_t* bounds, cudaEvent_t* ev, int nchunks) {
+  // Expand src[0, n) into dst, chunk by chunk as run `run` marks them; the work
+  // it waits for is on stream s.  False if s ended without marking them all
+  // (nothing is waited for any more then).
+  bool run(const uint32_t* src, int64_t* dst, int64_t n, const volatile uint32_t* ready, uint32_t run,
+           cudaStream_t s) {
     {
       std::lock_guard<std::mutex> lk(mu_);
       src_ = src;
       dst_ = dst;
-      bounds_ = bounds;
-      ev_ = ev;
-      nchunks_ = nchunks;
+      nchunks_ = chunks_for(n);
+      len_ = n / nchunks_;
+      ready_ = ready;
+      run_ = run;
+      gave_up_.store(false);
       pending_ = n_ - 1;
       ++gen_;
     }
     cv_.notify_all();
-    work(0);
+    work(0, s);
     std::unique_lock<std::mutex> lk(mu_);
     cv_done_.wait(lk, [&] { return pending_ == 0; });
+    return !gave_up_.load();
   }
 
  private:
   void loop(int t) {
-    cudaSetDevice(device_);
     uint64_t seen = 0;
     for (;;) {
       {
@@ -101,7 +157,7 @@ class PredExpander {
         if (stop_) return;
         seen = gen_;
       }
-      work(t);
+      work(t, nullptr);
       {
         std::lock_guard<std::mutex> lk(mu_);
         --pending_;
@@ -110,44 +166,75 @@ class PredExpander {
     }
   }
 
-  void work(int t) {
+  // Thread 0 watches the stream: once its work has ended, in whatever way, a
+  // chunk that is not marked never will be, and every thread gives up.
+  bool wait_for(int c, int t, cudaStream_t s) {
+    for (uint32_t spins = 1;; ++spins) {
+      if ((ready_[c] >> 1) == run_) break;
+      if (gave_up_.load(std::memory_order_relaxed)) return false;
+      if (t == 0 && (spins & 0xFFF) == 0 && ended(s) && (ready_[c] >> 1) != run_) {
+        gave_up_.store(true);
+        return false;
+      }
+      cpu_pause();
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    return true;
+  }
+
+  // The stream's work is over: complete, or failing for some seconds (a query
+  // may also be refused for a while, as during another thread's capture).
+  bool ended(cudaStream_t s) {
+    const cudaError_t e = cudaStreamQuery(s);
+    if (e == cudaSuccess) return true;
+    if (e == cudaErrorNotReady) {
+      failing_ = false;
+      return false;
+    }
+    cudaGetLastError();
+    const auto now = std::chrono::steady_clock::now();
+    if (!failing_) since_ = now;
+    failing_ = true;
+    return now - since_ > std::chrono::seconds(5);
+  }
+
+  void work(int t, cudaStream_t s) {
     for (int k = 0; k < nchunks_; ++k) {
-      const int64_t b = bounds_[k], len = bounds_[k + 1] - b;
-      const int64_t lo = b + len * t / n_, hi = b + len * (t + 1) / n_;
-      cudaEventSynchronize(ev_[k]);
-      const uint32_t* s = src_;
+      const int64_t b = len_ * k;
+      const int64_t lo = b + len_ * t / n_, hi = b + len_ * (t + 1) / n_;
+      if (!wait_for(k, t, s)) return;
+      const uint32_t* src = src_;
       int64_t* d = dst_;
       for (int64_t i = lo; i < hi; ++i) {
-        const uint32_t e = s[i];
+        const uint32_t e = src[i];
         d[i] = e == PACK_UNREACHED ? -1 : (int64_t)(e & ((1u << PACK_BITS) - 1u)) | ((int64_t)(e >> PACK_BITS) << 48);
       }
     }
   }
 
-  int device_ = 0, n_ = 1;
+  int n_ = 1;
+  bool failing_ = false;  // thread 0 only
+  std::chrono::steady_clock::time_point since_;
   std::vector<std::thread> th_;
   std::mutex mu_;
   std::condition_variable cv_, cv_done_;
+  std::atomic<bool> gave_up_{false};
   bool stop_ = false;
   uint64_t gen_ = 0;
   int pending_ = 0;
   const uint32_t* src_ = nullptr;
   int64_t* dst_ = nullptr;
-  const int64_t* bounds_ = nullptr;
-  cudaEvent_t* ev_ = nullptr;
-  int nchunks_ = 0;
+  int64_t len_ = 0;
+  int nchunks_ = 1;
+  const volatile uint32_t* ready_ = nullptr;
+  uint32_t run_ = 0;
 };
 
 void pred_expander_free(g500_bfs* b) {
   delete b->expander;
   b->expander = nullptr;
-  for (auto& e : b->ev_chunk)
-    if (e) {
-      cudaEventDestroy(e);
-      e = nullptr;
-    }
-  dev_free(b->d_pack);
-  dev_free(b->d_pack_ovf);
+  dev_free(b->d_pack_state);
+  b->d_pack_state = nullptr;
   if (b->h_pack) cudaFreeHost(b->h_pack);
   b->h_pack = nullptr;
 }
@@ -156,46 +243,41 @@ int pred_to_host_packed(g500_bfs* b, int64_t* host_pred, cudaStream_t s, bool* p
   g500_graph* g = b->g;
   *packed = false;
   const int64_t n = g->nolv;
-  if (n > (1ll << PACK_BITS) || n % 2 != 0 || b->pack_host_off) return G500_OK;
+  if (n > (1ll << PACK_BITS) || n % (4 * PRED_CHUNKS) != 0 || b->pack_host_off) return G500_OK;
   cudaPointerAttributes attr;
   if (cudaPointerGetAttributes(&attr, host_pred) != cudaSuccess) {
     cudaGetLastError();  // not a pointer the runtime knows: pageable
     attr.type = cudaMemoryTypeUnregistered;
   }
   if (attr.type != cudaMemoryTypeUnregistered) return G500_OK;  // pinned (or device): one DMA copy is faster
-  if (!b->d_pack) {
-    G500_TRY(dev_alloc_n(&b->d_pack, n, "packed pred"));
-    G500_TRY(dev_alloc_n(&b->d_pack_ovf, 1, "packed pred overflow flag"));
-    // the overflow flag lands after the entries
-    G500_CUDA(cudaHostAlloc(&b->h_pack, sizeof(uint32_t) * (size_t)(n + 64), cudaHostAllocDefault));
-    for (auto& e : b->ev_chunk) G500_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  if (!b->expander) {
+    void* st = b->d_pack_state;
+    if (!st) G500_TRY(dev_alloc(&st, sizeof(PackState), "pred packing state"));
+    b->d_pack_state = st;
+    G500_CUDA(cudaMemsetAsync(st, 0, sizeof(PackState), s));
+    if (!b->h_pack) {
+      G500_CUDA(cudaHostAlloc(&b->h_pack, sizeof(uint32_t) * (size_t)n + sizeof(PackTail), cudaHostAllocDefault));
+      memset(b->h_pack + n, 0, sizeof(PackTail));
+    }
     const int hw = (int)std::thread::hardware_concurrency();
-    b->expander = new PredExpander(g->device, std::max(1, std::min(hw > 0 ? hw : 1, 16)));
+    b->expander = new PredExpander(std::max(1, std::min(hw > 0 ? hw : 1, 16)));
   }
-  G500_CUDA(cudaMemsetAsync(b->d_pack_ovf, 0, sizeof(unsigned), s));
-  const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(n / 2, 256), (int64_t)num_sms() * 8);
-  pack_pred_kernel<<<grid, 256, 0, s>>>(b->d_pred, n, b->d_pack, b->d_pack_ovf);
+  PackState* st = static_cast<PackState*>(b->d_pack_state);
+  PackTail* tail = reinterpret_cast<PackTail*>(b->h_pack + n);  // n is even: 8-byte aligned
+  G500_CUDA(cudaMemcpyAsync(&tail->ctl, b->d_ctl, sizeof(BfsCtl), cudaMemcpyDeviceToHost, s));
+  const uint32_t run = ++b->pack_run & 0x7FFFFFFFu;
+  pack_to_host_kernel<<<PACK_GROUPS * PACK_BLOCKS, PACK_THREADS, 0, s>>>(b->d_pred, n, chunks_for(n), b->h_pack, st, tail->ready, run);
   G500_CUDA(cudaGetLastError());
-  volatile uint32_t* h_ovf = b->h_pack + n;
-  *h_ovf = 0;
-  G500_CUDA(cudaMemcpyAsync(b->h_pack + n, b->d_pack_ovf, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-  int64_t bounds[PRED_CHUNKS + 1];
-  for (int k = 0; k <= PRED_CHUNKS; ++k) bounds[k] = (n * k / PRED_CHUNKS) & ~(int64_t)63;
-  bounds[PRED_CHUNKS] = n;
-  for (int k = 0; k < PRED_CHUNKS; ++k) {
-    const int64_t lo = bounds[k], len = bounds[k + 1] - lo;
-    if (len > 0)
-      G500_CUDA(cudaMemcpyAsync(b->h_pack + lo, b->d_pack + lo, sizeof(uint32_t) * (size_t)len,
-                                cudaMemcpyDeviceToHost, s));
-    G500_CUDA(cudaEventRecord(b->ev_chunk[k], s));
-  }
-  // the flag arrived with the first chunk's event
-  G500_CUDA(cudaEventSynchronize(b->ev_chunk[0]));
-  if (*h_ovf) {  // a level or an id beyond the packed fields: the caller gets the int64 copy instead
-    G500_CUDA(cudaStreamSynchronize(s));
+  const bool complete = b->expander->run(b->h_pack, host_pred, n, tail->ready, run, s);
+  G500_CUDA(cudaStreamSynchronize(s));
+  if (!complete) return set_error(G500_E_DEVICE, "the packed pred did not arrive");
+  *b->h_ctl = tail->ctl;
+  bool bad = false;
+  for (int c = 0; c < chunks_for(n); ++c) bad |= tail->ready[c] & 1u;
+  if (bad) {  // a level or an id beyond the packed fields: the caller gets the int64 copy instead
+    G500_CUDA(cudaMemsetAsync(st, 0, sizeof(PackState), s));
     return G500_OK;
   }
-  b->expander->run(b->h_pack, host_pred, bounds, b->ev_chunk, PRED_CHUNKS);
   *packed = true;
   return G500_OK;
 }

@@ -413,3 +413,28 @@ def test_switch_back_to_top_down_keeps_levels(g500, oracle_mod, blocks):
         ok, evc, rep = oracle_mod.validate(edges, bfs.graph_.info.max_used_vertex + 1, len(pred), root, pred)
         assert ok and evc == st.nedge, rep
     bfs.close()
+
+
+@pytest.mark.parametrize("blocks64k", [1, 2, 3, 5, 8, 33])
+def test_packed_host_pred_chunks(g500, oracle_mod, blocks64k):
+    """Host pred arrays of every chunk count, at sizes that are odd multiples of 65536, against the device's own
+    entries; a run too deep for the packed entries in between falls back, and the next packs again."""
+    n = 65536 * blocks64k
+    rng = np.random.default_rng(blocks64k)
+    ids = rng.integers(0, min(n, 40000), (200000, 2))
+    path = np.stack([np.arange(n - 60, n - 1), np.arange(n - 59, n)], 1)  # 60 levels apart from the rest
+    ids = np.concatenate([ids, path])
+    edges = np.zeros(len(ids), g500.EDGE_DTYPE)
+    edges["v0_low"], edges["v1_low"] = ids[:, 0], ids[:, 1]
+    og = oracle_mod.Graph(edges, 0)
+    bfs = g500.BfsOnGPU(reorder_mode=0)
+    bfs.construct(edges)
+    bfs.prepare_bfs()
+    host = np.zeros(bfs.graph_.pred_size(), np.int64)
+    for root in (int(ids[0, 0]), n - 60, int(ids[1, 1])):
+        host[:] = 0x5A5A5A5A5A5A5A5A
+        st = bfs.run_bfs(root, host)
+        assert np.array_equal(g500.levels_from_pred(host), og.bfs_levels(root))
+        ok, evc, rep = oracle_mod.validate(edges, bfs.graph_.info.max_used_vertex + 1, len(host), root, host)
+        assert ok and evc == st.nedge, rep
+    bfs.close()

@@ -1,6 +1,6 @@
 // Batched multi-source BFS: up to 128 roots per call, W = 32/64/128 roots per
 // launch as one bit-lane each in W-bit masks per vertex (visited V, frontier
-// F, next N), with a uint8 level per (vertex, lane).  Each launch is one
+// F, next N), the levels as bit planes per 32 lanes.  Each launch is one
 // persistent cooperative kernel; every level is
 //
 //   pull   every vertex with unvisited lanes ORs its neighbours' frontier
@@ -9,16 +9,17 @@
 //   push   every frontier vertex ORs its mask into its neighbours' next masks
 //          (atomicOr into N, only the bits a neighbour still lacks),
 //
+// or both (lanes with a small frontier pushed first, the others pulled),
 // followed by settling the new lanes (V |= new; next F = new; levels): a
 // pulling row settles itself, the hub rows (split across warps) and every
-// row after a push settle in a pass of their own.  The frontier masks are
-// double-buffered by level parity.  Pull or push is chosen per level from
+// row after a push-only level settle in a pass of their own.  The frontier
+// masks are double-buffered by level parity.  Pull or push is chosen per level from
 // edge counts: pull when the new frontier's degree sum exceeds (degree sum of
 // vertices with unvisited lanes) / alpha.  On large graphs a push level with
 // a small frontier is sparse: it works on the vertices marked in frontier and
 // touched bitmaps instead of on every vertex (kernel argument SP).
-// Levels come out per root in original-id order through a shared-memory
-// transpose; the whole launch sequence is captured once as a CUDA graph and
+// Levels come out per root in original-id order through bit and byte
+// transposes in registers; the whole launch sequence is captured once as a CUDA graph and
 // replayed for every batch.
 //
 // The levels of each lane are exactly the BFS distances from its root, the
@@ -1049,9 +1050,10 @@ __global__ void __launch_bounds__(MS_THREADS, MS_MIN_BLOCKS) msbfs_kernel(MsPara
     la.fb = p.fb[level % 3];
     if (level == (int)MS_PLANE_LEVELS - 1)  // the upper planes, first written at the next level
       for (int64_t i = tid; i < p.nlv * NW; i += nthreads) p.L[p.nlv * NW + i] = make_uint4(0, 0, 0, 0);
-    // A level that would pull surveys the lanes' frontiers: lanes whose frontier degree sum is under 1/MS_SURVEY_DIV of the graph's entries are
-    // pushed at that level, the others pulled (a mixed level: both phases
-    // leave their finds in N and the apply pass settles every vertex).
+    // A level that would pull surveys the lanes' frontiers: lanes whose
+    // frontier degree sum is under 1/MS_SURVEY_DIV of the graph's entries are
+    // pushed first (a mixed level), the others pulled after a barrier, each row
+    // settling its finds with what was pushed to it.
     Mask<NW> qm, pm;  // lanes pushed, lanes pulled
 #pragma unroll
     for (int k = 0; k < NW; ++k) {

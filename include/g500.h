@@ -205,8 +205,10 @@ int g500_bfs_set_pred_mode(g500_bfs* b, int mode);
  * than 30 levels.  on = 1 (default) or 0 (always copy the int64 entries);
  * the values are the same. */
 int g500_bfs_set_host_pack(g500_bfs* b, int on);
-/* Blocks of the persistent kernel (0 = every co-resident block of the device);
- * fewer leave SMs to kernels of other handles running at the same time. */
+/* Blocks of the persistent kernel (0 = every co-resident block of the device;
+ * a new handle starts with that, or with one block per SM on graphs of at most
+ * 2^20 vertices with edges); fewer leave SMs to kernels of other handles
+ * running at the same time. */
 int g500_bfs_set_grid(g500_bfs* b, int blocks);
 
 /* Autotuner: time every (policy, alpha, beta) of a built-in grid on the given
@@ -303,7 +305,7 @@ typedef struct g500_msbfs_level {
                               lanes with a small frontier pushed, the others pulled */
   int64_t discovered;      /* new (vertex, lane) pairs */
   double device_ms;        /* the whole level */
-  double expand_ms;        /* its pull or push phase (the rest is the apply pass) */
+  double expand_ms;        /* its pull or push phase (the rest is the apply pass; all of it where rows settle as they pull) */
   int64_t rows_read;       /* counting runs: row (or hub chunk) offset reads of the level, else -1 */
   int64_t sectors;         /* counting runs: 32-byte adjacency sectors the level's examined entries span, else -1 */
 } g500_msbfs_level;
@@ -325,8 +327,10 @@ int g500_msbfs_wait(g500_msbfs* m, g500_msbfs_stats* stats);
 /* on != 0: every call that fits one launch also computes the per-root
  * statistics of g500_msbfs_root_stats on the device, in the same stream. */
 int g500_msbfs_set_root_stats(g500_msbfs* m, int on);
-/* Blocks per launch (0 = every co-resident block of the device).  Fewer
- * blocks leave SMs to launches of other handles running at the same time. */
+/* Blocks per launch (0 = every co-resident block of the device; a new handle
+ * starts with that, or with fewer on graphs of at most 2^20 vertices with
+ * edges).  Fewer blocks leave SMs to launches of other handles running at the
+ * same time. */
 int g500_msbfs_set_grid(g500_msbfs* m, int blocks);
 int g500_msbfs_get_grid(const g500_msbfs* m, int lane_width, int* blocks, int* max_blocks);
 /* Sparse levels: a push level whose last frontier has a degree sum of at most

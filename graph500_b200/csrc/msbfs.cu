@@ -1466,6 +1466,7 @@ struct g500_msbfs {
   unsigned grid_full[3] = {0, 0, 0};                  // the whole device's co-resident blocks
   int want_stats = 0;                                 // root statistics enqueued with every one-launch call
   int in_flight = 0, fl_batches = 0, fl_stats = 0, stats_valid = 0;
+  int run_width = 64;                                 // lane width of the last launch: the layout of V and L
   std::vector<int64_t> fl_roots, last_roots;
   std::chrono::steady_clock::time_point t_launch;
   cudaGraphExec_t graphs[3][4] = {};                  // [log2(W/32)][batch]
@@ -1730,7 +1731,7 @@ extern "C" int g500_msbfs_set_params(g500_msbfs* m, int lane_width, double alpha
 static int ms_enqueue_stats(g500_msbfs* m, int nroots, cudaStream_t s) {
   g500_graph* g = m->g;
   const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(std::max<int64_t>(g->nlv, 1), 256), num_sms() * 8);
-  const int W = m->lane_width;
+  const int W = m->run_width;
   if (W == 32) ms_stats_kernel<1><<<grid, 256, 0, s>>>(m->V, g->d_vis_init, g->d_endp, g->nlv, nroots, m->head, g->d_reorder, m->sums, m->stats_dev);
   else if (W == 64) ms_stats_kernel<2><<<grid, 256, 0, s>>>(m->V, g->d_vis_init, g->d_endp, g->nlv, nroots, m->head, g->d_reorder, m->sums, m->stats_dev);
   else ms_stats_kernel<4><<<grid, 256, 0, s>>>(m->V, g->d_vis_init, g->d_endp, g->nlv, nroots, m->head, g->d_reorder, m->sums, m->stats_dev);
@@ -1769,6 +1770,7 @@ static int ms_launch(g500_msbfs* m, const int64_t* roots, int nroots, uint8_t* l
   G500_CUDA(cudaSetDevice(g->device));
   m->t_launch = std::chrono::steady_clock::now();
   const int W = m->lane_width;
+  m->run_width = W;
   const int ni = nw_index(W);
   const int batches = (nroots + W - 1) / W;
   const bool levels_direct = levels && levels_on_device && ms_direct_row(m, levels);
@@ -1856,7 +1858,7 @@ static int ms_complete(g500_msbfs* m, g500_msbfs_stats* stats) {
     memset(stats, 0, sizeof(*stats));
     stats->device_ms = ms;
     stats->host_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - m->t_launch).count();
-    stats->lane_width = m->lane_width;
+    stats->lane_width = m->run_width;
     stats->batches = batches;
     for (int b = 0; b < batches; ++b) {
       stats->num_levels = std::max<int32_t>(stats->num_levels, (int32_t)m->h_ctl[b].num_levels);

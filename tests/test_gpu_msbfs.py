@@ -87,6 +87,25 @@ def test_msbfs_root_stats_match_validator(g500, oracle_mod, s13):
     ms.close()
 
 
+@pytest.mark.parametrize("ran,then", [(32, 64), (32, 128), (64, 32), (128, 64)])
+def test_msbfs_root_stats_keep_the_width_that_ran(g500, s13, ran, then):
+    """Root statistics and the run's lane width describe the launch that ran, whatever width is set after it:
+    after a run, and while a launch is in flight."""
+    g, og, roots, _ = s13
+    ms = g500.MultiSourceBFS(g, ran)
+    ms.run(roots[:20])
+    want = [a.tolist() for a in ms.root_stats(20)]
+    ms.run(roots[:20])
+    ms.set_params(then)
+    assert [a.tolist() for a in ms.root_stats(20)] == want
+    ms.set_params(ran)
+    ms.launch(roots[:20])
+    ms.set_params(then)
+    assert ms.wait().lane_width == ran
+    assert [a.tolist() for a in ms.root_stats(20)] == want
+    ms.close()
+
+
 def test_msbfs_matches_reference_fixture_levels(g500):
     rec, arr = load_golden(18, 2)
     g = g500.Graph2DCSR.generate(18, 16, 2)

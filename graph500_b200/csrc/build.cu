@@ -470,7 +470,7 @@ int graph_destroy_internal(g500_graph* g) {
   cudaSetDevice(g->device);
   if (g->stream) cudaStreamSynchronize(g->stream);
   dev_free(g->d_maps);
-  dev_free(g->d_val);
+  dev_free(g->d_val.load());
   dev_free(g->d_cols);
   if (g->owns_edges) dev_free(g->d_edges);
   if (g->stream) cudaStreamDestroy(g->stream);

@@ -5,6 +5,7 @@
 #include <stdint.h>
 #include <stdarg.h>
 #include <stdio.h>
+#include <atomic>
 #include <string>
 #include <vector>
 
@@ -133,7 +134,7 @@ struct g500_graph {
   double gen_seconds = 0, build_seconds = 0;
 
   void* d_maps = nullptr;           // the allocation of every array below but cols and edges
-  void* d_val = nullptr;            // the validator's scratch, kept once a call has needed it
+  std::atomic<void*> d_val{nullptr};  // the validator's scratch, kept once a call has needed it (null while one uses it)
   uint64_t* d_offsets = nullptr;    // [nlv + 1]
   uint32_t* d_cols = nullptr;       // [nge]   reordered targets, ascending per row
   uint32_t* d_first = nullptr;      // [nlv]   first (smallest) neighbour (| FIRST_MORE) or NO_VERTEX

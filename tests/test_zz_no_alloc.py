@@ -122,3 +122,37 @@ def test_packed_and_unpacked_validation_report_alike(g500, planted, skip, drop):
     if planted not in ("none",):
         assert not ok.value
     bfs.close()
+
+
+def test_validations_of_one_graph_from_several_threads(g500):
+    """Calls on one graph from several threads each report their own result: half validate a right pred, half
+    one with two levels planted wrong, and every call's counts are those of the same call alone."""
+    import threading
+
+    bfs = g500.BfsOnGPU(reorder_mode=2)
+    bfs.construct(g500.EdgeList(None, 14, 16))
+    bfs.prepare_bfs()
+    g = bfs.graph_
+    root = int(g500.find_roots(g, 1)[0])
+    good = np.zeros(g.pred_size(), np.int64)
+    bfs.run_bfs(root, good)
+    bad = good.copy()
+    reached = np.nonzero((good != -1) & (np.arange(len(good)) != root))[0]
+    for v in reached[[len(reached) // 3, len(reached) // 2]]:
+        bad[v] += 2 << 48
+    alone = [g500.validate_bfs_result(g, root, p) for p in (good, bad)]
+    assert alone[0][0] and not alone[1][0]
+    got = [[] for _ in range(8)]
+
+    def work(i):
+        for _ in range(40):
+            got[i].append(g500.validate_bfs_result(g, root, (good, bad)[i % 2]))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(got))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for i, results in enumerate(got):
+        assert results == [alone[i % 2]] * 40, i
+    bfs.close()

@@ -565,7 +565,7 @@ extern "C" int g500_graph_info_get(const g500_graph* g, g500_graph_info* info) {
   info->num_global_edges = g->nge;
   info->max_used_vertex = g->max_used_vertex;
   info->num_input_edges = g->num_edges;
-  info->device_bytes = g->device_bytes;
+  info->device_bytes = g->device_bytes + g->val_bytes.load();
   info->reorder_mode = g->reorder_mode;
   info->device = g->device;
   return G500_OK;

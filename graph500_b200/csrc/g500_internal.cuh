@@ -135,6 +135,7 @@ struct g500_graph {
 
   void* d_maps = nullptr;           // the allocation of every array below but cols and edges
   std::atomic<void*> d_val{nullptr};  // the validator's scratch, kept once a call has needed it (null while one uses it)
+  std::atomic<int64_t> val_bytes{0};  // its size
   uint64_t* d_offsets = nullptr;    // [nlv + 1]
   uint32_t* d_cols = nullptr;       // [nge]   reordered targets, ascending per row
   uint32_t* d_first = nullptr;      // [nlv]   first (smallest) neighbour (| FIRST_MORE) or NO_VERTEX

@@ -227,9 +227,13 @@ __global__ void __launch_bounds__(256) val_parent_kernel(const int64_t* __restri
 struct KeptScratch {
   g500_graph* g;
   void* p;
+  size_t bytes;
+  bool keep = true;
   ~KeptScratch() {
     void* none = nullptr;
-    if (p && !g->d_val.compare_exchange_strong(none, p)) dev_free(p);
+    if (!p) return;
+    if (keep && g->d_val.compare_exchange_strong(none, p)) g->val_bytes.store((int64_t)bytes);
+    else dev_free(p);
   }
 };
 
@@ -284,12 +288,17 @@ extern "C" int g500_validate(g500_graph* g, const g500_packed_edge* edges, int64
   Slab scratch;
   scratch.add(&d_err, VE_N);
   scratch.add(&d_valid, nlocal);
+  Slab small = scratch;
   uint32_t* d_pack = nullptr;  // packed entries, where the ids allow them
   const bool can_pack = nlocal <= (int64_t(1) << VAL_SHIFT);
   if (can_pack) scratch.add(&d_pack, nlocal);
-  KeptScratch kept{g, g->d_val.exchange(nullptr)};
+  KeptScratch kept{g, g->d_val.exchange(nullptr), scratch.bytes};
   if (kept.p) scratch.place(kept.p);
   else st = scratch.alloc(&kept.p, "validation scratch");
+  if (st == G500_E_NOMEM && can_pack) {  // a fifth of the memory does without packed entries, for this call
+    st = small.alloc(&kept.p, "validation scratch");
+    kept.keep = false;
+  }
   if (st != G500_OK) { cleanup(); return st; }
   cudaError_t e = cudaMemsetAsync(d_err, 0, sizeof(unsigned long long) * VE_N, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_valid, 0, (size_t)nlocal, s);

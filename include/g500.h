@@ -58,7 +58,7 @@ typedef struct g500_graph_info {
   int64_t num_global_edges;      /* directed CSR entries after dedup (:1438-1441) */
   int64_t max_used_vertex;       /* largest original id with an edge (benchmark_helper.hpp:510) */
   int64_t num_input_edges;       /* length of the resident edge list (0 if not kept) */
-  int64_t device_bytes;          /* device memory held by the graph */
+  int64_t device_bytes;          /* device memory held by the graph (with the validator's scratch once it has one) */
   int32_t reorder_mode;          /* VERTEX_REORDERING 0/1/2 (parameters.h:37-41) */
   int32_t device;
 } g500_graph_info;
@@ -250,7 +250,10 @@ typedef struct g500_validate_report {
 /* validate_bfs_result (validate.hpp:1008-1019) with nglobalverts =
  * max_used_vertex + 1 and nlocalverts = pred_size, as main.cc:129-133 calls
  * it.  edges == NULL uses the graph's resident edge list.  *ok = 1 when the
- * result is valid; *edge_visit_count = the traversed-edge count TEPS uses. */
+ * result is valid; *edge_visit_count = the traversed-edge count TEPS uses.
+ * The first call allocates 5 bytes of scratch per original id (1 above 2^27
+ * ids), which the graph then holds and counts in device_bytes; where only 1
+ * byte per id is free, a call does with that and holds nothing. */
 int g500_validate(g500_graph* g, const g500_packed_edge* edges, int64_t num_edges,
                   int edges_on_device, int64_t root, const int64_t* pred, int pred_on_device,
                   int64_t* edge_visit_count, int* ok, g500_validate_report* report);

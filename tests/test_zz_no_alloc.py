@@ -156,3 +156,50 @@ def test_validations_of_one_graph_from_several_threads(g500):
     for i, results in enumerate(got):
         assert results == [alone[i % 2]] * 40, i
     bfs.close()
+
+
+def test_validation_scratch_is_reported_and_not_needed_whole(g500):
+    """With room for the flags but not for the packed entries a validation still runs, and keeps nothing; with
+    room it keeps its scratch and the graph's device_bytes say so."""
+    import torch
+
+    warm = g500.Graph2DCSR.generate(10)  # the kernels are loaded before memory runs short
+    g500.validate_bfs_result(warm, 0, np.full(warm.pred_size(), -1, np.int64))
+    warm.close()
+    bfs = g500.BfsOnGPU(reorder_mode=2)
+    bfs.construct(g500.EdgeList(None, 22, 1))
+    bfs.prepare_bfs()
+    g = bfs.graph_
+    n = g.pred_size()
+    root = int(g500.find_roots(g, 1)[0])
+    pred = torch.empty(n, dtype=torch.int64, device="cuda")
+    bfs.run_bfs(root, pred)
+    torch.cuda.synchronize()
+
+    def held():
+        info = g500.GraphInfo()
+        g500.check(g500.lib().g500_graph_info_get(g.h, C.byref(info)))
+        return info.device_bytes
+
+    def fill(size, out):
+        try:
+            while True:
+                out.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+        except torch.OutOfMemoryError:
+            pass
+
+    before, full = held(), []
+    spare = torch.empty(14 << 20, dtype=torch.uint8, device="cuda")  # the flags take 4.2 MB, the rest 17
+    try:
+        for size in (1 << 30, 16 << 20, 1 << 20):
+            fill(size, full)
+        del spare
+        torch.cuda.empty_cache()
+        got = g500.validate_bfs_result(g, root, pred)
+    finally:
+        full.clear()
+        torch.cuda.empty_cache()
+    assert held() == before
+    assert got == g500.validate_bfs_result(g, root, pred) and got[0]
+    assert before + 5 * n <= held() <= before + 5 * n + 4096
+    bfs.close()

@@ -308,7 +308,6 @@ int graph_alloc_maps(g500_graph* g) {
   m.add(&g->d_offsets, g->nlv + 1);
   m.add(&g->d_first, g->nlv);
   m.add(&g->d_vis_init, g->nlv / 32);
-  m.add(&g->d_has_edge, g->nolv / 32);
   return m.alloc(&g->d_maps, "reorder maps, row offsets and bitmaps");
 }
 
@@ -343,11 +342,12 @@ static int build_from_device_edges(g500_graph* g, const g500_packed_edge* d_edge
   const int64_t nolv = g->nolv;
 
   // degrees
-  uint32_t *deg = nullptr, *sl = nullptr;
+  uint32_t *deg = nullptr, *sl = nullptr, *has_edge = nullptr;
   uint64_t *k = nullptr, *k2 = nullptr;
   Slab verts;
   verts.add(&deg, nolv);
   verts.add(&sl, nolv);
+  verts.add(&has_edge, nolv / 32);
   if (g->reorder_mode != 0) {
     verts.add(&k, nolv);
     verts.add(&k2, nolv);
@@ -387,8 +387,12 @@ static int build_from_device_edges(g500_graph* g, const g500_packed_edge* d_edge
   G500_CUDA(cudaGetLastError());
   endp_kernel<<<grid_for(nolv), 256, 0, s>>>(deg, sl, g->d_invert, nolv, g->d_endp);
   G500_CUDA(cudaGetLastError());
-  has_edge_orig_kernel<<<grid_for(nolv), 256, 0, s>>>(deg, nolv, g->d_has_edge);
+  // host bitmap of has_edge over original ids
+  has_edge_orig_kernel<<<grid_for(nolv), 256, 0, s>>>(deg, nolv, has_edge);
   G500_CUDA(cudaGetLastError());
+  g->h_has_edge_orig.assign((size_t)(nolv / 32), 0u);
+  G500_CUDA(cudaMemcpyAsync(g->h_has_edge_orig.data(), has_edge, sizeof(uint32_t) * (nolv / 32),
+                            cudaMemcpyDeviceToHost, s));
 
   // CSR: keys for both directions (over the degrees' memory), sort, drop duplicates
   uint64_t* sorted = nullptr;
@@ -427,10 +431,6 @@ static int build_from_device_edges(g500_graph* g, const g500_packed_edge* d_edge
                                                      g->d_first, g->d_vis_init);
     G500_CUDA(cudaGetLastError());
   }
-  // host bitmap of has_edge over original ids
-  g->h_has_edge_orig.assign((size_t)(nolv / 32), 0u);
-  G500_CUDA(cudaMemcpyAsync(g->h_has_edge_orig.data(), g->d_has_edge, sizeof(uint32_t) * (nolv / 32),
-                            cudaMemcpyDeviceToHost, s));
   G500_CUDA(cudaStreamSynchronize(s));
 
   // find_max_used_vertex (benchmark_helper.hpp:510-528) on the host bitmap

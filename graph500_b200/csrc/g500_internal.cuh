@@ -144,7 +144,6 @@ struct g500_graph {
   uint32_t* d_invert = nullptr;     // [nolv]  reordered -> original
   uint32_t* d_vis_init = nullptr;   // [nlv/32] ~has_edge in reordered space
   uint32_t* d_endp = nullptr;       // [nolv]  input endpoint occurrences per reordered vertex
-  uint32_t* d_has_edge = nullptr;   // [nolv/32] has-edge bitmap over original ids (construction)
   g500_packed_edge* d_edges = nullptr;  // resident input edge list (optional)
   int64_t num_edges = 0;
   bool owns_edges = false;

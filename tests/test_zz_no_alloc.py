@@ -203,3 +203,22 @@ def test_validation_scratch_is_reported_and_not_needed_whole(g500):
     assert got == g500.validate_bfs_result(g, root, pred) and got[0]
     assert before + 5 * n <= held() <= before + 5 * n + 4096
     bfs.close()
+
+
+@pytest.mark.parametrize("validated", [False, True])
+def test_device_bytes_is_what_a_graph_holds(g500, validated):
+    """device_bytes against the memory that destroying the graph gives back: within the 2 MB granularity of its
+    allocations (maps, adjacency, edge list, validator's scratch)."""
+    import torch
+
+    g = g500.Graph2DCSR.generate(26, 1)
+    if validated:
+        root = int(g500.find_roots(g, 1)[0])
+        g500.validate_bfs_result(g, root, torch.full((g.pred_size(),), -1, dtype=torch.int64, device="cuda"))
+    info = g500.GraphInfo()
+    g500.check(g500.lib().g500_graph_info_get(g.h, C.byref(info)))
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    g.close()
+    held = torch.cuda.mem_get_info()[0] - free
+    assert info.device_bytes <= held <= info.device_bytes + (4 << 21)

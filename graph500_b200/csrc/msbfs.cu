@@ -1303,11 +1303,12 @@ __global__ void __launch_bounds__(TR_BLOCK, 4) ms_transpose_kernel(const uint4* 
   __syncthreads();
   if (threadIdx.x == 0) last = atomicAdd(&ctl->out_blocks, 1u) + 1 == gridDim.x;
   __syncthreads();
-  if (last)
-    for (int i = threadIdx.x; i < nroots; i += TR_BLOCK) {
-      if (rows[0][i]) rows[0][i][head->roots[i]] = 0;
-      if (rows[1][i]) rows[1][i][head->roots[i]] = 0;
-    }
+  if (!last) return;
+  __threadfence();  // these bytes lie in words other blocks have written
+  for (int i = threadIdx.x; i < nroots; i += TR_BLOCK) {
+    if (rows[0][i]) rows[0][i][head->roots[i]] = 0;
+    if (rows[1][i]) rows[1][i][head->roots[i]] = 0;
+  }
 }
 
 __global__ void ms_degree_kernel(const uint64_t* __restrict__ off, int64_t nlv, uint32_t* __restrict__ deg) {

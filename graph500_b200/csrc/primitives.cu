@@ -25,6 +25,7 @@ int set_error(int code, const char* fmt, ...) {
 
 int cuda_error(cudaError_t e, const char* what, const char* file, int line) {
   int code = (e == cudaErrorMemoryAllocation) ? G500_E_NOMEM : G500_E_DEVICE;
+  cudaGetLastError();  // a refused call is reported here, not by the next launch's check as well
   return set_error(code, "%s failed: %s (%s:%d)", what, cudaGetErrorString(e), file, line);
 }
 

@@ -21,3 +21,11 @@ def test_barrier_wait_runs_out_and_context_recovers(g500):
     bfs.run_bfs(root, pred)
     assert g500.validate_bfs_result(bfs.graph_, root, pred)[0]
     bfs.close()
+
+
+def test_a_refused_cuda_call_does_not_fail_the_next_one(g500):
+    """An error that CUDA returned to one call (a device that does not exist) is that call's alone."""
+    with pytest.raises(g500.G500Error) as ei:
+        g500.Graph2DCSR.generate(10, device=99)
+    assert ei.value.code == g500.G500_E_DEVICE
+    g500.Graph2DCSR.generate(10).close()

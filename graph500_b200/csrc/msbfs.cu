@@ -27,6 +27,9 @@
 #include "g500_internal.cuh"
 #include "device_common.cuh"
 
+#include <cuda.h>
+#include <cudaTypedefs.h>
+
 #include <algorithm>
 #include <chrono>
 
@@ -1742,15 +1745,36 @@ static int ms_enqueue_stats(g500_msbfs* m, int nroots, cudaStream_t s) {
   return G500_OK;
 }
 
-// Whether the output pass can write a level row at p itself.
-static bool ms_direct_row(const g500_msbfs* m, const void* p) {
+// The end of the device allocation that p lies in, or null.
+static const uint8_t* allocation_end(const void* p) {
+  static const PFN_cuMemGetAddressRange_v3020 get_range = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &found) != cudaSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return reinterpret_cast<PFN_cuMemGetAddressRange_v3020>(f);
+  }();
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  if (!get_range || get_range(&base, &size, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS) return nullptr;
+  return reinterpret_cast<const uint8_t*>(base) + size;
+}
+
+// Whether the output pass can write `bytes` of level rows at p itself.  Memory
+// that ends earlier is left to a copy, which the runtime refuses: the pass
+// would write past its end.
+static bool ms_direct_rows(const g500_msbfs* m, const uint8_t* p, int64_t bytes) {
   if (reinterpret_cast<uintptr_t>(p) & 3) return false;
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  return a.type == cudaMemoryTypeDevice && a.device == m->g->device;
+  if (a.type != cudaMemoryTypeDevice || a.device != m->g->device) return false;
+  const uint8_t* end = allocation_end(p);
+  return end && end - p >= bytes;
 }
 
 // Enqueue a whole call (every launch, the optional level copy, the control
@@ -1774,7 +1798,7 @@ static int ms_launch(g500_msbfs* m, const int64_t* roots, int nroots, uint8_t* l
   m->run_width = W;
   const int ni = nw_index(W);
   const int batches = (nroots + W - 1) / W;
-  const bool levels_direct = levels && levels_on_device && ms_direct_row(m, levels);
+  const bool levels_direct = levels && levels_on_device && ms_direct_rows(m, levels, (int64_t)nroots * g->nolv);
   bool copied[MS_MAX_LANES];  // root_dsts: the row is copied after the launch
   for (int b = 0; b < 4; ++b) {
     MsHead& h = m->staging[b];
@@ -1787,7 +1811,7 @@ static int ms_launch(g500_msbfs* m, const int64_t* roots, int nroots, uint8_t* l
       h.row[0][i] = own;
       h.row[1][i] = levels_direct ? levels + (int64_t)r * g->nolv : nullptr;
       if (root_dsts) {
-        copied[r] = root_dsts[r] && !ms_direct_row(m, root_dsts[r]);
+        copied[r] = root_dsts[r] && !ms_direct_rows(m, root_dsts[r], g->nolv);
         if (!copied[r]) h.row[0][i] = root_dsts[r];
       }
     }

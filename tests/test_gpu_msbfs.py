@@ -1,6 +1,8 @@
 """Batched multi-source BFS vs the oracle: per-root uint8 levels are the BFS
 distances (255 = unreached), bit-exact, for every lane width, with and without
 the CUDA graph, under push-only and pull-only level schedules."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -247,6 +249,32 @@ def test_msbfs_levels_into_device_memory(g500, s13, offset, lanes, n):
         assert (got[:offset] == 77).all() and (got[offset + size:] == 77).all()
         assert np.array_equal(ms.device_levels(n).cpu().numpy(), got[offset:offset + size].reshape(n, -1))
     ms.close()
+
+
+@pytest.mark.parametrize("spare", [0, 1])
+def test_msbfs_refuses_device_memory_shorter_than_its_rows(g500, spare):
+    """A device allocation that ends inside the rows is refused by the call (the output pass must not write past
+    it); one of exactly their size is written, and the handle works on."""
+    import torch
+    g = g500.Graph2DCSR.generate(18, 4)
+    roots = g500.find_roots(g, 48)  # 48 * 2^18 bytes: 12 MB, a torch allocation of its own
+    ms = g500.MultiSourceBFS(g, 64)
+    want = ms.levels(roots)
+    torch.cuda.empty_cache()
+    buf = torch.full((len(roots) * g.pred_size(),), 77, dtype=torch.uint8, device="cuda")
+    n = len(roots) + spare * 16
+    rr = np.resize(roots, n)
+    L, p = g500.lib(), g500.MsStats()
+    rc = L.g500_msbfs_run(ms.h, rr.ctypes.data, n, buf.data_ptr(), 1, C.byref(p))
+    torch.cuda.synchronize()
+    if spare:
+        assert rc == g500.G500_E_DEVICE and b"invalid argument" in L.g500_last_error()
+        assert (buf == 77).all()
+    else:
+        assert rc == g500.G500_OK and np.array_equal(buf.cpu().numpy().reshape(want.shape), want)
+    assert np.array_equal(ms.levels(roots), want)
+    ms.close()
+    g.close()
 
 
 @pytest.mark.parametrize("lane_width", [32, 64, 128])

@@ -1037,7 +1037,7 @@ static int bfs_free(g500_bfs* b) {
   dev_free(b->d_levels);
   dev_free(b->d_overflow);
   if (b->ev_done) cudaEventDestroy(b->ev_done);
-  if (b->h_ctl != &b->host_ctl) cudaFreeHost(b->h_ctl);
+  pinned_slot_free(b->g->device, b->h_ctl);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
   if (b->own_stream) cudaStreamDestroy(b->own_stream);
@@ -1164,7 +1164,10 @@ extern "C" int g500_bfs_create(g500_graph* g, g500_bfs** out) {
     chk(cudaGetLastError(), "endpoint counts per bitmap word");
     chk(cudaStreamSynchronize(b->own_stream), "endpoint counts per bitmap word");
   }
-  b->h_ctl = &b->host_ctl;
+  void* h_ctl = nullptr;
+  if (st == G500_OK) st = pinned_slot(g->device, &h_ctl, "host copy of the control block");
+  b->h_ctl = static_cast<BfsCtl*>(h_ctl);
+  if (st == G500_OK) memset(h_ctl, 0, sizeof(BfsCtl));
   if (st == G500_OK) chk(cudaMemset(b->d_ctl, 0, sizeof(BfsCtl)), "cudaMemset");
   chk(cudaEventCreate(&b->ev0), "cudaEventCreate");
   chk(cudaEventCreate(&b->ev1), "cudaEventCreate");
@@ -1211,12 +1214,6 @@ int bfs_launch_levels(g500_bfs* b, int64_t root, uint8_t* levels_dst) {
   if (!b->d_levels) G500_TRY(dev_alloc_n(&b->d_levels, std::max<int64_t>(g->nolv, 1), "levels"));
   if (!b->d_overflow) G500_TRY(dev_alloc_n(&b->d_overflow, 1, "level overflow flag"));
   if (!b->ev_done) G500_CUDA(cudaEventCreateWithFlags(&b->ev_done, cudaEventDisableTiming));
-  if (b->h_ctl == &b->host_ctl) {  // an asynchronous copy needs pinned memory
-    BfsCtl* pinned = nullptr;
-    G500_CUDA(cudaHostAlloc(&pinned, sizeof(BfsCtl), cudaHostAllocDefault));
-    *pinned = b->host_ctl;
-    b->h_ctl = pinned;
-  }
   cudaStream_t s = b->stream;
   RunParams p;
   G500_TRY(make_params(b, root, b->d_pred, &p));
@@ -1404,7 +1401,6 @@ extern "C" int g500_bfs_run(g500_bfs* b, int64_t root, int64_t* pred, int pred_o
     G500_TRY(pred_to_host_packed(b, pred, s, &packed));
     if (!packed) G500_CUDA(cudaMemcpyAsync(pred, b->d_pred, sizeof(int64_t) * g->nolv, cudaMemcpyDeviceToHost, s));
   }
-  // last, since a copy to pageable memory waits for the run (pinned memory for it would cost 2 ms per handle)
   if (!packed) {
     G500_CUDA(cudaMemcpyAsync(b->h_ctl, b->d_ctl, sizeof(BfsCtl), cudaMemcpyDeviceToHost, s));
     G500_CUDA(cudaStreamSynchronize(s));

@@ -59,6 +59,12 @@ int dev_alloc_n(T** p, int64_t n, const char* what) {
 }
 void dev_free(void* p);
 
+// A small piece (at most PINNED_SLOT bytes) of pinned host memory for `device`,
+// the current one, and back.
+constexpr size_t PINNED_SLOT = 512;
+int pinned_slot(int device, void** p, const char* what);
+void pinned_slot_free(int device, void* p);
+
 // Several arrays cut from one device allocation.  A cudaMalloc costs about 0.4
 // ms and a cudaFree 0.3 ms whatever their size below 256 MB, which for the two
 // dozen arrays of a graph's construction was half of its time at SCALE 22.
@@ -204,6 +210,8 @@ struct LevelRecord {
   unsigned long long t_ns;      // %globaltimer when the level's last barrier completed
 };
 
+static_assert(sizeof(BfsCtl) <= g500::PINNED_SLOT, "the host copy's place");
+
 constexpr int MAX_LEVELS = 0xFFFE;
 
 namespace g500 {
@@ -234,15 +242,14 @@ struct g500_bfs {
   // a host pred crosses PCIe as packed 32-bit entries, expanded by host threads
   int pack_host_off = 0;
   void* d_pack_state = nullptr;
-  uint32_t* h_pack = nullptr;        // pinned [nolv], then the chunks' marks and the control block
+  uint32_t* h_pack = nullptr;        // pinned [nolv], then the chunks' marks
   uint32_t pack_run = 0;
   g500::PredExpander* expander = nullptr;
   uint32_t* d_vis[2] = {nullptr, nullptr};
   TdItem* d_queue[2] = {nullptr, nullptr};
   int64_t queue_cap = 0;
   BfsCtl* d_ctl = nullptr;
-  BfsCtl* h_ctl = nullptr;           // copy after each run: &host_ctl, or pinned once a run was asynchronous
-  BfsCtl host_ctl = {};
+  BfsCtl* h_ctl = nullptr;           // pinned copy after each run
   int ctl_ready = 0;                 // d_ctl is as a run needs it (see prepare_ctl)
   LevelRecord* d_rec = nullptr;      // [MAX_LEVELS]
   TdItem* d_big = nullptr;           // [BIG_ROWS] long frontier rows, listed whole

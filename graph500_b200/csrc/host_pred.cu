@@ -52,10 +52,9 @@ struct PackState {
   unsigned bad;
 };
 
-// The pinned tail behind the packed entries.
+// The chunks' marks, in pinned memory behind the packed entries.
 struct PackTail {
   volatile uint32_t ready[PRED_CHUNKS];  // run number << 1 | an entry so far did not fit
-  BfsCtl ctl;                            // the run's control block
 };
 
 // Chunk c holds entries [c, c + 1) * n / nchunks (n is a multiple of 65536).
@@ -263,15 +262,14 @@ int pred_to_host_packed(g500_bfs* b, int64_t* host_pred, cudaStream_t s, bool* p
     b->expander = new PredExpander(std::max(1, std::min(hw > 0 ? hw : 1, 16)));
   }
   PackState* st = static_cast<PackState*>(b->d_pack_state);
-  PackTail* tail = reinterpret_cast<PackTail*>(b->h_pack + n);  // n is even: 8-byte aligned
-  G500_CUDA(cudaMemcpyAsync(&tail->ctl, b->d_ctl, sizeof(BfsCtl), cudaMemcpyDeviceToHost, s));
+  PackTail* tail = reinterpret_cast<PackTail*>(b->h_pack + n);
+  G500_CUDA(cudaMemcpyAsync(b->h_ctl, b->d_ctl, sizeof(BfsCtl), cudaMemcpyDeviceToHost, s));
   const uint32_t run = ++b->pack_run & 0x7FFFFFFFu;
   pack_to_host_kernel<<<PACK_GROUPS * PACK_BLOCKS, PACK_THREADS, 0, s>>>(b->d_pred, n, chunks_for(n), b->h_pack, st, tail->ready, run);
   G500_CUDA(cudaGetLastError());
   const bool complete = b->expander->run(b->h_pack, host_pred, n, tail->ready, run, s);
   G500_CUDA(cudaStreamSynchronize(s));
   if (!complete) return set_error(G500_E_DEVICE, "the packed pred did not arrive");
-  *b->h_ctl = tail->ctl;
   bool bad = false;
   for (int c = 0; c < chunks_for(n); ++c) bad |= tail->ready[c] & 1u;
   if (bad) {  // a level or an id beyond the packed fields: the caller gets the int64 copy instead

@@ -438,3 +438,57 @@ def test_packed_host_pred_chunks(g500, oracle_mod, blocks64k):
         ok, evc, rep = oracle_mod.validate(edges, bfs.graph_.info.max_used_vertex + 1, len(host), root, host)
         assert ok and evc == st.nedge, rep
     bfs.close()
+
+
+def test_many_handles_at_once(g500):
+    """More BFS handles than share a page of pinned memory (128), run in turn, given back in mixed order and from
+    several threads, and made again: each keeps its own counts."""
+    import threading
+
+    graphs = [g500.Graph2DCSR.generate(10, 16, 2, 0, 2 + i, 3) for i in range(3)]
+    roots = [int(g500.find_roots(g, 1)[0]) for g in graphs]
+
+    def make(k):
+        bfs = g500.BfsOnGPU(reorder_mode=2)
+        bfs.graph_ = graphs[k % 3]
+        bfs.prepare_bfs()
+        return bfs
+
+    def counts(bfs, k, pred):
+        st = bfs.run_bfs(roots[k % 3], pred)
+        return st.reached, st.nedge, st.num_levels, [lv["discovered"] for lv in bfs.level_stats()]
+
+    want = []
+    for k in range(3):
+        bfs = make(k)
+        want.append(counts(bfs, k, np.zeros(graphs[k].pred_size(), np.int64)))
+        bfs.end_bfs()
+    handles = [make(k) for k in range(140)]
+    pred = np.zeros(graphs[0].pred_size(), np.int64)
+    for _ in range(2):
+        for k, bfs in enumerate(handles):
+            assert counts(bfs, k, pred) == want[k % 3], k
+        for k in range(0, 140, 3):
+            handles[k].end_bfs()
+        for k in range(0, 140, 3):
+            handles[k] = make(k)
+    for bfs in handles:
+        bfs.end_bfs()
+    failed = []
+
+    def work(i):
+        own = np.zeros(graphs[0].pred_size(), np.int64)
+        for _ in range(20):
+            bfs = make(i)
+            if counts(bfs, i, own) != want[i]:
+                failed.append(i)
+            bfs.end_bfs()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
+    for g in graphs:
+        g.close()

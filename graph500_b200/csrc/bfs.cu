@@ -745,7 +745,7 @@ __device__ __forceinline__ void write_record(LevelRecord* rec, int level, bool t
   rec[level - 1] = r;
 }
 
-template <int DEF>
+template <int DEF, bool LISTS>
 __global__ void __launch_bounds__(BFS_THREADS, BFS_MIN_BLOCKS) bfs_persistent_kernel(RunParams p) {
   __shared__ unsigned long long sh_cnt[C_NUM];
   __shared__ unsigned long long sh_acc[C_NUM];
@@ -809,8 +809,6 @@ __global__ void __launch_bounds__(BFS_THREADS, BFS_MIN_BLOCKS) bfs_persistent_ke
   bool forward = true, growing = true;
   bool bu_before = false;  // the last level was bottom-up
   int listed_levels = -1;  // bottom-up levels run from the lists (-1: there are none)
-  const bool lists_pay = p.policy == G500_DIR_REFERENCE && p.nwords >= BU_LIST_WORDS * gwarp_count() &&
-                         (double)p.ngv / p.beta < (double)(BU_LIST * gwarp_count());
   int64_t qn = root_items, prev_nq = 0, visited = 1, carried = 0, nbig = 0;
   unsigned td_levels = 0;
   int64_t mu = (int64_t)(p.off[p.nlv] - root_deg);  // degree sum of unvisited vertices (edge policy)
@@ -844,14 +842,14 @@ __global__ void __launch_bounds__(BFS_THREADS, BFS_MIN_BLOCKS) bfs_persistent_ke
       listed = sh_cnt[C_QITEMS];
       mf = sh_cnt[C_MF];
     } else {
-      if (listed_levels >= 0) {
+      if (LISTS && listed_levels >= 0) {
         bu_list_level<DEF>(p, p.vis[cur_vis], p.vis[cur_vis ^ 1], listed_levels == 0, lists, sh_acc, lvl);
       } else {
         bu_level<DEF>(p, p.vis[cur_vis], p.vis[cur_vis ^ 1], sh_acc, lvl);
-        if (bu_before && lists_pay) bu_collect(p, p.vis[cur_vis ^ 1], lists, sh_acc);
+        if (LISTS && bu_before) bu_collect(p, p.vis[cur_vis ^ 1], lists, sh_acc);
       }
       if (!grid_sync_sum<C_NUM>(cnt, &ctl->bar, sh_acc, sh_cnt)) return;
-      if (listed_levels >= 0 || (bu_before && lists_pay && sh_cnt[C_BIG] == 0)) ++listed_levels;
+      if (LISTS && (listed_levels >= 0 || (bu_before && sh_cnt[C_BIG] == 0))) ++listed_levels;
       if (tid == 0) t_mid = globaltimer();
       ++phase;
       disc = sh_cnt[C_DISC];
@@ -1055,10 +1053,20 @@ static int launch_deferred_pred(const RunParams& p, cudaStream_t s) {
   return G500_OK;
 }
 
-static const void* bfs_kernel_for(int deferred) {
-  if (deferred == 2) return (const void*)bfs_persistent_kernel<2>;
-  if (deferred == 1) return (const void*)bfs_persistent_kernel<1>;
-  return (const void*)bfs_persistent_kernel<0>;
+// Whether late bottom-up levels run from lists (see bu_collect).  A kernel of its
+// own: with the lists' code in every search, one without them took 1 us longer
+// at SCALE 22.
+static bool lists_pay(const RunParams& p, unsigned grid) {
+  const int64_t warps = (int64_t)grid * (BFS_THREADS / 32);
+  return p.policy == G500_DIR_REFERENCE && p.nwords >= BU_LIST_WORDS * warps &&
+         (double)p.ngv / p.beta < (double)(BU_LIST * warps);
+}
+
+static const void* bfs_kernel_for(const RunParams& p, unsigned grid) {
+  const bool lists = lists_pay(p, grid);
+  if (p.deferred == 2) return lists ? (const void*)bfs_persistent_kernel<2, true> : (const void*)bfs_persistent_kernel<2, false>;
+  if (p.deferred == 1) return lists ? (const void*)bfs_persistent_kernel<1, true> : (const void*)bfs_persistent_kernel<1, false>;
+  return lists ? (const void*)bfs_persistent_kernel<0, true> : (const void*)bfs_persistent_kernel<0, false>;
 }
 
 // The kernel's parameters for one run from `root` writing pred to `pred`.
@@ -1173,7 +1181,7 @@ extern "C" int g500_bfs_create(g500_graph* g, g500_bfs** out) {
   chk(cudaEventCreate(&b->ev1), "cudaEventCreate");
   if (st == G500_OK) {
     int per_sm = 0;
-    chk(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bfs_persistent_kernel<2>, BFS_THREADS, 0),
+    chk(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bfs_persistent_kernel<2, true>, BFS_THREADS, 0),
         "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
     int coop = 0;
     chk(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, g->device), "cudaDeviceGetAttribute");
@@ -1221,7 +1229,7 @@ int bfs_launch_levels(g500_bfs* b, int64_t root, uint8_t* levels_dst) {
   void* args[] = {&p};
   G500_TRY(prepare_ctl(b, s));
   G500_CUDA(cudaMemsetAsync(b->d_overflow, 0, sizeof(unsigned), s));
-  G500_CUDA(cudaLaunchCooperativeKernel(bfs_kernel_for(p.deferred), dim3(b->grid), dim3(BFS_THREADS), args,
+  G500_CUDA(cudaLaunchCooperativeKernel(bfs_kernel_for(p, b->grid), dim3(b->grid), dim3(BFS_THREADS), args,
                                         0, s));
   G500_TRY(launch_deferred_pred(p, s));
   const unsigned lg = (unsigned)std::min<int64_t>(ceil_div(g->nolv, 256), num_sms() * 8);
@@ -1392,7 +1400,7 @@ extern "C" int g500_bfs_run(g500_bfs* b, int64_t root, int64_t* pred, int pred_o
   void* args[] = {&p};
   G500_TRY(prepare_ctl(b, s));
   G500_CUDA(cudaEventRecord(b->ev0, s));
-  G500_CUDA(cudaLaunchCooperativeKernel(bfs_kernel_for(p.deferred), dim3(b->grid), dim3(BFS_THREADS), args,
+  G500_CUDA(cudaLaunchCooperativeKernel(bfs_kernel_for(p, b->grid), dim3(b->grid), dim3(BFS_THREADS), args,
                                         0, s));
   G500_TRY(launch_deferred_pred(p, s));
   G500_CUDA(cudaEventRecord(b->ev1, s));

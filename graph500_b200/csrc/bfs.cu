@@ -781,7 +781,10 @@ __global__ void __launch_bounds__(BFS_THREADS, BFS_MIN_BLOCKS) bfs_persistent_ke
     if (has_edges && tid == 0) put_deferred<DEF>(p, root_r, (uint32_t)p.root, 0);
   if (blockIdx.x == 0 && threadIdx.x < 3 * C_NUM) (&ctl->cnt[0][0])[threadIdx.x] = 0;
   if (blockIdx.x == 0 && threadIdx.x < 3 * P_NUM) (&ctl->pos[0][0])[threadIdx.x] = 0;
-  if (tid == 0) ctl->edges2 = 0;
+  if (tid == 0) {
+    ctl->edges2 = 0;
+    ctl->list_levels = 0;
+  }
 
   // first_expand (bfs.hpp:477-518): the root's row becomes the first queue
   for (int64_t c = tid; c < root_items; c += nthreads) {
@@ -844,6 +847,7 @@ __global__ void __launch_bounds__(BFS_THREADS, BFS_MIN_BLOCKS) bfs_persistent_ke
     } else {
       if (LISTS && listed_levels >= 0) {
         bu_list_level<DEF>(p, p.vis[cur_vis], p.vis[cur_vis ^ 1], listed_levels == 0, lists, sh_acc, lvl);
+        if (tid == 0) ++ctl->list_levels;
       } else {
         bu_level<DEF>(p, p.vis[cur_vis], p.vis[cur_vis ^ 1], sh_acc, lvl);
         if (LISTS && bu_before) bu_collect(p, p.vis[cur_vis ^ 1], lists, sh_acc);
@@ -1473,6 +1477,12 @@ extern "C" int g500_bfs_level_stats(const g500_bfs* b, g500_level_stats* out, in
     o.device_ms_tail = r.t_mid_ns ? (double)(r.t_ns - r.t_mid_ns) * 1e-6 : 0.0;
     prev = r.t_ns;
   }
+  return G500_OK;
+}
+
+extern "C" int g500_selftest_bfs_list_levels(const g500_bfs* b, int* levels) {
+  if (!b || !levels) return set_error(G500_E_INVAL, "null argument");
+  *levels = (int)b->h_ctl->list_levels;
   return G500_OK;
 }
 

@@ -198,6 +198,7 @@ struct BfsCtl {
   unsigned long long reached;   // reached vertices
   unsigned long long edges2;    // 2 * nedge (runs that ask for it)
   unsigned td_levels;           // levels run top-down
+  unsigned list_levels;         // bottom-up levels run from the warps' lists
   unsigned pad_overflow;        // host copy of the levels-overflow flag of an asynchronous run
 };
 

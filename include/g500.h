@@ -489,6 +489,10 @@ int g500_part_destroy(g500_part* p);
  * end with the others giving up (*timed_out = 1) and leave the context usable
  * for a following launch (*recovered = 1).  Causes no fault. */
 int g500_selftest_barrier_timeout(int device, int* timed_out, int* recovered);
+/* Levels of the last run that worked from the warps' lists of unvisited
+ * vertices instead of the visited bitmap (late bottom-up levels of large
+ * graphs; their results and counters are those of any bottom-up level). */
+int g500_selftest_bfs_list_levels(const g500_bfs* b, int* levels);
 
 /* Validation that allocates nothing, for callers that cannot call cudaMalloc
  * (a host framework owning all device memory through its own arena or caching

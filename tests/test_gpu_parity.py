@@ -4,6 +4,7 @@ Bit-exact for everything: edges, CSR, reorder maps, roots, levels; parents
 are accepted iff both the device validator and the oracle's restatement of
 validate.hpp accept them.
 """
+import ctypes as C
 import hashlib
 
 import numpy as np
@@ -357,7 +358,7 @@ def test_listed_bottom_up_levels(g500, oracle_mod, pred_mode, pendants):
     """A star (which turns the search bottom-up) with a caterpillar of 60 spine vertices on one leaf: dozens of
     late bottom-up levels over rows of 1 to 92 entries.  One or two blocks have enough words per warp to run
     them from their lists (90 pendants overflow the lists at first), the whole device does not: levels and
-    per-level counters must be the same."""
+    per-level counters must be the same.  The other direction policy uses no lists."""
     leaves, spine = 60000, 60
     pairs = [(0, i) for i in range(1, leaves + 1)]
     base, pend = leaves + 1, leaves + 1 + spine
@@ -383,6 +384,13 @@ def test_listed_bottom_up_levels(g500, oracle_mod, pred_mode, pendants):
         assert sum(not lv[0] for lv in got) == st.bu_levels > spine and len(got) == st.num_levels
         want = want or got
         assert got == want, blocks
+        n = C.c_int()
+        g500.check(g500.lib().g500_selftest_bfs_list_levels(bfs.h, C.byref(n)))
+        assert 0 < n.value < st.bu_levels if blocks else n.value == 0, (blocks, n.value)
+    bfs.set_params(2000.0, 1e9, True, g500.DIR_EDGES)
+    bfs.run_bfs(77, pred)
+    g500.check(g500.lib().g500_selftest_bfs_list_levels(bfs.h, C.byref(n)))
+    assert n.value == 0 and np.array_equal(g500.levels_from_pred(pred), og.bfs_levels(77))
     bfs.close()
 
 

@@ -423,11 +423,12 @@ def test_switch_back_to_top_down_keeps_levels(g500, oracle_mod, blocks):
     bfs.close()
 
 
-@pytest.mark.parametrize("blocks64k", [1, 2, 3, 5, 8, 33])
-def test_packed_host_pred_chunks(g500, oracle_mod, blocks64k):
-    """Host pred arrays of every chunk count, at sizes that are odd multiples of 65536, against the device's own
-    entries; a run too deep for the packed entries in between falls back, and the next packs again."""
-    n = 65536 * blocks64k
+@pytest.mark.parametrize("blocks64k,ids_used", [(1, 1), (2, 2), (4, 4), (8, 8), (16, 16), (32, 32), (4, 3), (8, 5), (64, 33)])
+def test_packed_host_pred_chunks(g500, oracle_mod, blocks64k, ids_used):
+    """Host pred arrays of every chunk count (1, 1, 2, 4, 8 and 16 chunks for 2^16 to 2^21 entries, a power of two
+    whatever the largest id), with ids up to their end or to somewhere inside, against the oracle's levels; a run
+    too deep for the packed entries in between falls back, and the next packs again."""
+    n = 65536 * ids_used
     rng = np.random.default_rng(blocks64k)
     ids = rng.integers(0, min(n, 40000), (200000, 2))
     path = np.stack([np.arange(n - 60, n - 1), np.arange(n - 59, n)], 1)  # 60 levels apart from the rest
@@ -439,6 +440,7 @@ def test_packed_host_pred_chunks(g500, oracle_mod, blocks64k):
     bfs.construct(edges)
     bfs.prepare_bfs()
     host = np.zeros(bfs.graph_.pred_size(), np.int64)
+    assert len(host) == 65536 * blocks64k
     for root in (int(ids[0, 0]), n - 60, int(ids[1, 1])):
         host[:] = 0x5A5A5A5A5A5A5A5A
         st = bfs.run_bfs(root, host)

@@ -16,21 +16,14 @@
 // above it; 0xFFFFFFFF = unreached.  Graphs with more than 2^PACK_BITS ids,
 // and runs with a level of 31 or more, copy the int64 entries instead.
 #include "g500_internal.cuh"
+#include "pred_expander.h"
 
 #include <algorithm>
-#include <atomic>
-#include <chrono>
-#include <condition_variable>
-#include <mutex>
-#include <thread>
 #include <vector>
 
 namespace g500 {
 namespace {
 
-constexpr int PACK_BITS = 27;
-constexpr uint32_t PACK_UNREACHED = 0xFFFFFFFFu;
-constexpr int PACK_MAX_LEVEL = 30;  // level 31 with an all-ones parent would read as unreached
 // Chunks of at least 512 KB of packed entries (a chunk's fences and mark cost
 // about 5 us: with 16 chunks whatever the size a SCALE 18 call took 200 us
 // instead of 153), at most 16.
@@ -98,136 +91,7 @@ __global__ void __launch_bounds__(PACK_THREADS) pack_to_host_kernel(const int64_
   }
 }
 
-inline void cpu_pause() {
-#if defined(__x86_64__) || defined(__i386__)
-  __builtin_ia32_pause();
-#endif
-}
-
 }  // namespace
-
-// Host threads that expand the chunks: each waits for a chunk's mark and
-// expands its slice of it, so one wake-up per run serves every chunk.
-class PredExpander {
- public:
-  explicit PredExpander(int nthreads) : n_(nthreads) {
-    for (int t = 1; t < nthreads; ++t) th_.emplace_back([this, t] { loop(t); });
-  }
-  ~PredExpander() {
-    {
-      std::lock_guard<std::mutex> lk(mu_);
-      stop_ = true;
-    }
-    cv_.notify_all();
-    for (auto& t : th_) t.join();
-  }
-
-  // Expand src[0, n) into dst, chunk by chunk as run `run` marks them; the work
-  // it waits for is on stream s.  False if s ended without marking them all
-  // (nothing is waited for any more then).
-  bool run(const uint32_t* src, int64_t* dst, int64_t n, const volatile uint32_t* ready, uint32_t run,
-           cudaStream_t s) {
-    {
-      std::lock_guard<std::mutex> lk(mu_);
-      src_ = src;
-      dst_ = dst;
-      nchunks_ = chunks_for(n);
-      len_ = n / nchunks_;
-      ready_ = ready;
-      run_ = run;
-      gave_up_.store(false);
-      pending_ = n_ - 1;
-      ++gen_;
-    }
-    cv_.notify_all();
-    work(0, s);
-    std::unique_lock<std::mutex> lk(mu_);
-    cv_done_.wait(lk, [&] { return pending_ == 0; });
-    return !gave_up_.load();
-  }
-
- private:
-  void loop(int t) {
-    uint64_t seen = 0;
-    for (;;) {
-      {
-        std::unique_lock<std::mutex> lk(mu_);
-        cv_.wait(lk, [&] { return stop_ || gen_ != seen; });
-        if (stop_) return;
-        seen = gen_;
-      }
-      work(t, nullptr);
-      {
-        std::lock_guard<std::mutex> lk(mu_);
-        --pending_;
-      }
-      cv_done_.notify_one();
-    }
-  }
-
-  // Thread 0 watches the stream: once its work has ended, in whatever way, a
-  // chunk that is not marked never will be, and every thread gives up.
-  bool wait_for(int c, int t, cudaStream_t s) {
-    for (uint32_t spins = 1;; ++spins) {
-      if ((ready_[c] >> 1) == run_) break;
-      if (gave_up_.load(std::memory_order_relaxed)) return false;
-      if (t == 0 && (spins & 0xFFF) == 0 && ended(s) && (ready_[c] >> 1) != run_) {
-        gave_up_.store(true);
-        return false;
-      }
-      cpu_pause();
-    }
-    std::atomic_thread_fence(std::memory_order_acquire);
-    return true;
-  }
-
-  // The stream's work is over: complete, or failing for some seconds (a query
-  // may also be refused for a while, as during another thread's capture).
-  bool ended(cudaStream_t s) {
-    const cudaError_t e = cudaStreamQuery(s);
-    if (e == cudaSuccess) return true;
-    if (e == cudaErrorNotReady) {
-      failing_ = false;
-      return false;
-    }
-    cudaGetLastError();
-    const auto now = std::chrono::steady_clock::now();
-    if (!failing_) since_ = now;
-    failing_ = true;
-    return now - since_ > std::chrono::seconds(5);
-  }
-
-  void work(int t, cudaStream_t s) {
-    for (int k = 0; k < nchunks_; ++k) {
-      const int64_t b = len_ * k;
-      const int64_t lo = b + len_ * t / n_, hi = b + len_ * (t + 1) / n_;
-      if (!wait_for(k, t, s)) return;
-      const uint32_t* src = src_;
-      int64_t* d = dst_;
-      for (int64_t i = lo; i < hi; ++i) {
-        const uint32_t e = src[i];
-        d[i] = e == PACK_UNREACHED ? -1 : (int64_t)(e & ((1u << PACK_BITS) - 1u)) | ((int64_t)(e >> PACK_BITS) << 48);
-      }
-    }
-  }
-
-  int n_ = 1;
-  bool failing_ = false;  // thread 0 only
-  std::chrono::steady_clock::time_point since_;
-  std::vector<std::thread> th_;
-  std::mutex mu_;
-  std::condition_variable cv_, cv_done_;
-  std::atomic<bool> gave_up_{false};
-  bool stop_ = false;
-  uint64_t gen_ = 0;
-  int pending_ = 0;
-  const uint32_t* src_ = nullptr;
-  int64_t* dst_ = nullptr;
-  int64_t len_ = 0;
-  int nchunks_ = 1;
-  const volatile uint32_t* ready_ = nullptr;
-  uint32_t run_ = 0;
-};
 
 void pred_expander_free(g500_bfs* b) {
   delete b->expander;
@@ -267,7 +131,14 @@ int pred_to_host_packed(g500_bfs* b, int64_t* host_pred, cudaStream_t s, bool* p
   const uint32_t run = ++b->pack_run & 0x7FFFFFFFu;
   pack_to_host_kernel<<<PACK_GROUPS * PACK_BLOCKS, PACK_THREADS, 0, s>>>(b->d_pred, n, chunks_for(n), b->h_pack, st, tail->ready, run);
   G500_CUDA(cudaGetLastError());
-  const bool complete = b->expander->run(b->h_pack, host_pred, n, tail->ready, run, s);
+  const auto state = [s] {
+    const cudaError_t e = cudaStreamQuery(s);
+    if (e == cudaSuccess) return WorkState::complete;
+    if (e == cudaErrorNotReady) return WorkState::running;
+    cudaGetLastError();
+    return WorkState::refused;
+  };
+  const bool complete = b->expander->run(b->h_pack, host_pred, n, chunks_for(n), tail->ready, run, state);
   G500_CUDA(cudaStreamSynchronize(s));
   if (!complete) return set_error(G500_E_DEVICE, "the packed pred did not arrive");
   bool bad = false;

@@ -1,0 +1,88 @@
+// The host side of a packed pred's arrival (graph500_b200/csrc/pred_expander.h)
+// without a GPU: the marks and the state of the work come from this program.
+// One check per argument; prints "ok" or what was wrong.
+#include "pred_expander.h"
+
+#include <stdio.h>
+#include <string.h>
+
+#include <algorithm>
+#include <string>
+
+using namespace g500;
+using std::chrono::milliseconds;
+
+namespace {
+
+constexpr int64_t N = 1 << 16;
+constexpr int CHUNKS = 16;
+
+struct Fixture {
+  std::vector<uint32_t> src = std::vector<uint32_t>(N);
+  std::vector<int64_t> dst = std::vector<int64_t>(N, 0x5A5A5A5A5A5A5A5A);
+  volatile uint32_t ready[CHUNKS] = {};
+  Fixture() {
+    for (int64_t i = 0; i < N; ++i)
+      src[(size_t)i] = i % 7 == 0 ? PACK_UNREACHED : (uint32_t)(i * 2654435761u) % (31u << PACK_BITS);
+  }
+  void mark(int c, uint32_t run, bool bad = false) {
+    std::atomic_thread_fence(std::memory_order_release);
+    ready[c] = run << 1 | (bad ? 1u : 0u);
+  }
+  void mark_all(uint32_t run) {
+    for (int c = 0; c < CHUNKS; ++c) mark(c, run);
+  }
+  bool expanded(int64_t b, int64_t e) const {
+    for (int64_t i = b; i < e; ++i) {
+      const uint32_t p = src[(size_t)i];
+      const int64_t want = p == PACK_UNREACHED ? -1 : (int64_t)(p % (1u << PACK_BITS)) + ((int64_t)(p >> PACK_BITS) << 48);
+      if (dst[(size_t)i] != want) return false;
+    }
+    return true;
+  }
+};
+
+std::string entries() {
+  for (int threads : {1, 3, 16}) {
+    Fixture f;
+    PredExpander x(threads);
+    for (uint32_t run = 1; run <= 20; ++run) {
+      std::fill(f.dst.begin(), f.dst.end(), 7);
+      std::thread marks([&] {
+        for (int c = CHUNKS - 1; c >= 0; --c) f.mark((c + (int)run) % CHUNKS, run);  // in any order
+      });
+      const bool done = x.run(f.src.data(), f.dst.data(), N, CHUNKS, f.ready, run, [] { return WorkState::running; });
+      marks.join();
+      if (!done || !f.expanded(0, N)) return "run " + std::to_string(run) + " with " + std::to_string(threads) + " threads";
+    }
+  }
+  return "ok";
+}
+
+// work that ends without marking every chunk ends the wait
+std::string unmarked() {
+  Fixture f;
+  PredExpander x(4);
+  f.mark(0, 1);
+  if (x.run(f.src.data(), f.dst.data(), N, CHUNKS, f.ready, 1, [] { return WorkState::complete; })) return "complete";
+  PredExpander y(4, milliseconds(20));
+  f.mark(0, 2);
+  if (y.run(f.src.data(), f.dst.data(), N, CHUNKS, f.ready, 2, [] { return WorkState::refused; })) return "refused";
+  return "ok";
+}
+
+}  // namespace
+
+int main(int argc, char** argv) {
+  const struct { const char* name; std::string (*check)(); } checks[] = {
+      {"entries", entries},
+      {"unmarked", unmarked},
+  };
+  for (const auto& c : checks)
+    if (argc > 1 && !strcmp(argv[1], c.name)) {
+      const std::string r = c.check();
+      puts(r.c_str());
+      return r == "ok" ? 0 : 1;
+    }
+  return 2;
+}

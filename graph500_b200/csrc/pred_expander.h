@@ -65,6 +65,7 @@ class PredExpander {
       ++gen_;
     }
     cv_.notify_all();
+    failing_ = false;  // what an earlier run saw says nothing about this one
     work(0, &state);
     std::unique_lock<std::mutex> lk(mu_);
     cv_done_.wait(lk, [&] { return pending_ == 0; });

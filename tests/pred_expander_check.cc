@@ -71,12 +71,30 @@ std::string unmarked() {
   return "ok";
 }
 
+// a state refused once near the end of a run that went well says nothing about a later run
+std::string refused_once() {
+  Fixture f;
+  PredExpander x(2, milliseconds(50));
+  for (uint32_t run = 1; run <= 2; ++run) {
+    int calls = 0;
+    // refused at the first query; the marks come with the second
+    const bool done = x.run(f.src.data(), f.dst.data(), N, CHUNKS, f.ready, run, [&] {
+      if (++calls > 1) f.mark_all(run);
+      return calls == 1 ? WorkState::refused : WorkState::complete;
+    });
+    if (!done) return "run " + std::to_string(run) + " given up after " + std::to_string(calls) + " queries";
+    std::this_thread::sleep_for(milliseconds(80));
+  }
+  return "ok";
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
   const struct { const char* name; std::string (*check)(); } checks[] = {
       {"entries", entries},
       {"unmarked", unmarked},
+      {"refused_once", refused_once},
   };
   for (const auto& c : checks)
     if (argc > 1 && !strcmp(argv[1], c.name)) {

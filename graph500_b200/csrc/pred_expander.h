@@ -48,8 +48,10 @@ class PredExpander {
   }
 
   // Expand src[0, n) into dst, nchunks chunks of equal length, as run `run` marks
-  // them (ready[c] >> 1); state() tells about the work that does.  False if it
-  // ended without marking them all (nothing is waited for any more then).
+  // them (ready[c] >> 1); state() tells about the work that does.  A mark's low
+  // bit says that an entry up to there did not fit: nothing more is expanded, for
+  // the caller copies the whole array another way.  False if the work ended
+  // without marking them all (nothing is waited for any more then).
   bool run(const uint32_t* src, int64_t* dst, int64_t n, int nchunks, const volatile uint32_t* ready, uint32_t run,
            const std::function<WorkState()>& state) {
     {
@@ -126,6 +128,7 @@ class PredExpander {
       const int64_t b = len_ * k;
       const int64_t lo = b + len_ * t / n_, hi = b + len_ * (t + 1) / n_;
       if (!wait_for(k, state)) return;
+      if (ready_[k] & 1u) return;
       const uint32_t* src = src_;
       int64_t* d = dst_;
       for (int64_t i = lo; i < hi; ++i) {

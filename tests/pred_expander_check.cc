@@ -88,6 +88,23 @@ std::string refused_once() {
   return "ok";
 }
 
+// a run whose entries do not fit is over for the expander: the caller copies it another way
+std::string does_not_fit() {
+  for (int threads : {1, 4}) {
+    Fixture f;
+    PredExpander x(threads);
+    for (int c = 0; c < CHUNKS; ++c) f.mark(c, 1, c >= 2);
+    if (!x.run(f.src.data(), f.dst.data(), N, CHUNKS, f.ready, 1, [] { return WorkState::running; })) return "given up";
+    for (int64_t i = 2 * (N / CHUNKS); i < N; ++i)
+      if (f.dst[(size_t)i] != 0x5A5A5A5A5A5A5A5A) return "entry " + std::to_string(i) + " written";
+    f.mark_all(2);
+    if (!x.run(f.src.data(), f.dst.data(), N, CHUNKS, f.ready, 2, [] { return WorkState::running; }) ||
+        !f.expanded(0, N))
+      return "the next run";
+  }
+  return "ok";
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -95,6 +112,7 @@ int main(int argc, char** argv) {
       {"entries", entries},
       {"unmarked", unmarked},
       {"refused_once", refused_once},
+      {"does_not_fit", does_not_fit},
   };
   for (const auto& c : checks)
     if (argc > 1 && !strcmp(argv[1], c.name)) {

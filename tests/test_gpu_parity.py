@@ -450,6 +450,27 @@ def test_packed_host_pred_chunks(g500, oracle_mod, blocks64k, ids_used):
     bfs.close()
 
 
+@pytest.mark.parametrize("depth", [29, 30, 31, 32])
+def test_host_pred_at_the_deepest_packed_level(g500, oracle_mod, depth):
+    """Level 30 is the last that the packed entries hold: paths that end there, before and after it, from both
+    ends and from the middle in turn."""
+    n = 1 << 17
+    edges = np.zeros(depth, g500.EDGE_DTYPE)
+    edges["v0_low"], edges["v1_low"] = n - 1 - np.arange(depth), n - 2 - np.arange(depth)
+    og = oracle_mod.Graph(edges, 0)
+    bfs = g500.BfsOnGPU(reorder_mode=0)
+    bfs.construct(edges)
+    bfs.prepare_bfs()
+    host = np.zeros(bfs.graph_.pred_size(), np.int64)
+    for root in (n - 1, n - 1 - depth // 2, n - 1 - depth):
+        host[:] = 0x5A5A5A5A5A5A5A5A
+        bfs.run_bfs(root, host)
+        assert np.array_equal(g500.levels_from_pred(host), og.bfs_levels(root)), root
+        ok, _, rep = oracle_mod.validate(edges, bfs.graph_.info.max_used_vertex + 1, len(host), root, host)
+        assert ok, rep
+    bfs.close()
+
+
 def test_many_handles_at_once(g500):
     """More BFS handles than share a page of pinned memory (128), run in turn, given back in mixed order and from
     several threads, and made again: each keeps its own counts."""

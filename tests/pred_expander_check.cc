@@ -5,6 +5,7 @@
 
 #include <stdio.h>
 #include <string.h>
+#include <time.h>
 
 #include <algorithm>
 #include <string>
@@ -105,6 +106,32 @@ std::string does_not_fit() {
   return "ok";
 }
 
+double cpu_seconds() {
+  timespec t;
+  clock_gettime(CLOCK_PROCESS_CPUTIME_ID, &t);
+  return (double)t.tv_sec + 1e-9 * (double)t.tv_nsec;
+}
+
+// while nothing is marked, only the calling thread polls without a break
+std::string long_wait() {
+  Fixture f;
+  PredExpander x(16);
+  f.mark_all(1);
+  x.run(f.src.data(), f.dst.data(), N, CHUNKS, f.ready, 1, [] { return WorkState::running; });  // every thread is up
+  std::thread marks([&] {
+    std::this_thread::sleep_for(milliseconds(300));
+    f.mark_all(2);
+  });
+  const double c0 = cpu_seconds();
+  const auto t0 = std::chrono::steady_clock::now();
+  const bool done = x.run(f.src.data(), f.dst.data(), N, CHUNKS, f.ready, 2, [] { return WorkState::running; });
+  const double wall = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+  const double cpus = (cpu_seconds() - c0) / wall;
+  marks.join();
+  if (!done || !f.expanded(0, N)) return "entries";
+  return cpus < 2.5 ? "ok" : std::to_string(cpus) + " processors busy while nothing had arrived";
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -113,6 +140,7 @@ int main(int argc, char** argv) {
       {"unmarked", unmarked},
       {"refused_once", refused_once},
       {"does_not_fit", does_not_fit},
+      {"long_wait", long_wait},
   };
   for (const auto& c : checks)
     if (argc > 1 && !strcmp(argv[1], c.name)) {

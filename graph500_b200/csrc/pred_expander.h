@@ -14,6 +14,7 @@
 #include <condition_variable>
 #include <functional>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -39,8 +40,13 @@ inline void cpu_pause() {
 class PredExpander {
  public:
   explicit PredExpander(int nthreads, std::chrono::steady_clock::duration give_up = std::chrono::seconds(5))
-      : n_(nthreads), give_up_(give_up) {
-    for (int t = 1; t < nthreads; ++t) th_.emplace_back([this, t] { loop(t); });
+      : give_up_(give_up) {
+    th_.reserve((size_t)nthreads);
+    try {
+      for (int t = 1; t < nthreads; ++t) th_.emplace_back([this, t] { loop(t); });
+    } catch (const std::system_error&) {  // no more threads to be had: those there are do the work
+    }
+    n_ = (int)th_.size() + 1;  // read by them in a run only
   }
   ~PredExpander() {
     {

@@ -5,9 +5,11 @@
 
 #include <stdio.h>
 #include <string.h>
+#include <sys/resource.h>
 #include <time.h>
 
 #include <algorithm>
+#include <fstream>
 #include <string>
 
 using namespace g500;
@@ -132,6 +134,26 @@ std::string long_wait() {
   return cpus < 2.5 ? "ok" : std::to_string(cpus) + " processors busy while nothing had arrived";
 }
 
+// where the system gives fewer threads than asked for, those do the work
+std::string few_threads() {
+  std::ifstream statm("/proc/self/statm");
+  long pages = 0;
+  statm >> pages;
+  // room for two or three more stacks
+  const rlimit limit{(rlim_t)pages * 4096 + (24u << 20), RLIM_INFINITY};
+  if (setrlimit(RLIMIT_AS, &limit)) return "setrlimit";
+  Fixture f;
+  PredExpander x(64);
+  for (uint32_t run = 1; run <= 3; ++run) {
+    std::fill(f.dst.begin(), f.dst.end(), 7);
+    f.mark_all(run);
+    if (!x.run(f.src.data(), f.dst.data(), N, CHUNKS, f.ready, run, [] { return WorkState::running; }) ||
+        !f.expanded(0, N))
+      return "run " + std::to_string(run);
+  }
+  return "ok";
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -141,6 +163,7 @@ int main(int argc, char** argv) {
       {"refused_once", refused_once},
       {"does_not_fit", does_not_fit},
       {"long_wait", long_wait},
+      {"few_threads", few_threads},
   };
   for (const auto& c : checks)
     if (argc > 1 && !strcmp(argv[1], c.name)) {

@@ -17,7 +17,7 @@ def program(tmp_path_factory):
     return str(exe)
 
 
-@pytest.mark.parametrize("check", ["entries", "unmarked", "refused_once", "does_not_fit", "long_wait"])
+@pytest.mark.parametrize("check", ["entries", "unmarked", "refused_once", "does_not_fit", "long_wait", "few_threads"])
 def test_expander(program, check):
     r = subprocess.run([program, check], capture_output=True, text=True, timeout=60)
     assert r.stdout.strip() == "ok" and r.returncode == 0, (check, r.stdout, r.returncode)

@@ -49,17 +49,12 @@ constexpr int BFS_THREADS = 512;
 // pred at random during the search costs a DRAM read-modify-write per
 // discovered vertex once pred no longer fits in L2.
 constexpr uint64_t BFS_DEFERRED_PRED_BYTES = 100ull << 20;
-// Packed deferred entries: parent original id in the low PACK_SHIFT bits, the
-// level above it, in 32 bits instead of 64.  At SCALE 26 that halves the
-// array the final pass gathers from (131 MB against 262 MB), so most of the
-// gathers hit L2.  Graphs with more than 2^PACK_SHIFT vertex ids use 64-bit
-// entries; a search that reaches level PACK_LEVELS - 1 stops, and the host
-// runs it again with 64-bit entries (and keeps them for that handle), so that
-// the all-ones word never is an entry: it marks an unreached vertex
-// (PACK_NONE; -1 in 64-bit entries).
-constexpr int PACK_SHIFT = 27;
-constexpr int PACK_LEVELS = 1 << (32 - PACK_SHIFT);
-constexpr uint32_t PACK_NONE = 0xFFFFFFFFu;
+// Packed deferred entries (packed_entry.h): 32 bits instead of 64.  At SCALE 26
+// that halves the array the final pass gathers from (131 MB against 262 MB), so
+// most of the gathers hit L2.  Graphs with more than 2^PACK_BITS vertex ids use
+// 64-bit entries (-1: unreached); a search that goes past PACK_MAX_LEVEL stops,
+// and the host runs it again with 64-bit entries (and keeps them for that
+// handle).
 constexpr int64_t BFS_SMALL_VERTS = 1 << 20;
 constexpr int BFS_MIN_BLOCKS = 2;        // co-resident blocks per SM (64 registers, no spills)
 constexpr int TD_UNROLL = TD_CHUNK / 32;  // virtual edges per lane per pass
@@ -120,7 +115,7 @@ __device__ __forceinline__ void fill_pred(const RunParams& p, int64_t tid, int64
 // vertex r (parent's original id, level << 48)
 template <int DEF>
 __device__ __forceinline__ void put_deferred(const RunParams& p, int64_t r, uint32_t parent, int64_t lvl) {
-  if constexpr (DEF == 2) p.pred_p[r] = parent | ((uint32_t)(lvl >> 48) << PACK_SHIFT);
+  if constexpr (DEF == 2) p.pred_p[r] = parent | ((uint32_t)(lvl >> 48) << PACK_BITS);
   else p.pred_r[r] = (int64_t)parent | lvl;
 }
 
@@ -150,12 +145,12 @@ __device__ __forceinline__ void append_row(uint64_t rb, uint64_t deg, uint32_t o
       nch = 0;
     }
   }
-  unsigned long long base = 0;
   const uint32_t incl = warp_incl_scan(nch);
   const uint32_t total = __shfl_sync(FULL_MASK, incl, 31);
   if (total == 0) return;
   if (lane == 0) *items += total;
   const uint32_t excl = incl - nch;
+  unsigned long long base = 0;
   if (lane == 31) base = atomicAdd(qcount, (unsigned long long)total);
   base = __shfl_sync(FULL_MASK, base, 31);
   if (base + total > (unsigned long long)cap) {
@@ -826,7 +821,7 @@ __global__ void __launch_bounds__(BFS_THREADS, BFS_MIN_BLOCKS) bfs_persistent_ke
   (blockIdx.x == 0 && threadIdx.x < P_NUM ? (void)(ctl->pos[(phase + 1) % 3][threadIdx.x] = 0) : (void)0), \
       ctl->cnt[phase % 3]
   for (;; ++level) {
-    if (DEF == 2 && level >= PACK_LEVELS - 1) {  // the packed level field is full: the host reruns unpacked
+    if (DEF == 2 && level > PACK_MAX_LEVEL) {  // the packed level field is full: the host reruns unpacked
       if (tid == 0) atomicOr(&ctl->bar.err, (unsigned)BFS_ERR_PACK);
       return;
     }
@@ -984,7 +979,7 @@ __device__ __forceinline__ long long final_entry(const RunParams& p, uint32_t r)
   if constexpr (DEF == 2) {
     const uint32_t e = __ldcg(p.pred_p + r);
     return e == PACK_NONE ? -1ll
-                          : (long long)((int64_t)(e & ((1u << PACK_SHIFT) - 1u)) | ((int64_t)(e >> PACK_SHIFT) << 48));
+                          : (long long)((int64_t)(e & PACK_ID) | ((int64_t)(e >> PACK_BITS) << 48));
   }
   return (long long)__ldcg(p.pred_r + r);
 }
@@ -1088,7 +1083,7 @@ static int make_params(g500_bfs* b, int64_t root, int64_t* pred, RunParams* out)
   p.pred = pred;
   int mode = b->pred_mode;
   if (mode == 0) mode = (uint64_t)g->nolv * 8 > BFS_DEFERRED_PRED_BYTES ? 3 : 1;
-  if (mode == 3 && (b->pack_off || g->nolv > (1ll << PACK_SHIFT))) mode = 2;
+  if (mode == 3 && (b->pack_off || g->nolv > (1ll << PACK_BITS))) mode = 2;
   p.deferred = mode == 1 ? 0 : (mode == 2 ? 1 : 2);
   if (p.deferred && !b->d_pred_r) {  // a mode asked for on a graph that defaults to another
     G500_TRY(dev_alloc_n(&b->d_pred_r, std::max<int64_t>(g->nlv, 1), "deferred pred"));

@@ -88,10 +88,10 @@ __device__ __forceinline__ unsigned atom_add_acq_rel_gpu(unsigned* p, unsigned v
 // counters are first added to flush_slot (one global atomic per non-zero
 // counter per block).  Thread 0 then arrives on a counter with acquire-release
 // semantics (the block's writes, ordered before it by __syncthreads, are
-// released with it).  The counter only grows during a launch (it starts at
-// zero): barrier k is complete once it reaches (k + 1) * gridDim.x, a target
-// each block computes from the value its own arrival returned, so the last
-// arrival has nothing more to publish.  The others poll the counter and take
+// released with it).  The counter only grows, from a multiple of gridDim.x: a
+// barrier is complete once it reaches the next multiple, a target each block
+// computes from the value its own arrival returned, so the last arrival has
+// nothing more to publish.  The others poll the counter and take
 // an acquire fence once it reached the target.  Polls are bounded; on
 // timeout (or an error raised elsewhere, checked every 16 polls) the barrier
 // reports failure and the caller returns.  On success thread 0 copies

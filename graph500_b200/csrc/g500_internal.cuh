@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "../../include/g500.h"
+#include "packed_entry.h"
 
 namespace g500 {
 
@@ -170,9 +171,10 @@ struct __align__(16) TdItem {
 enum BfsErr { BFS_ERR_QUEUE = 1, BFS_ERR_TIMEOUT = 2, BFS_ERR_DEPTH = 4, BFS_ERR_PACK = 8 };
 constexpr unsigned GRID_ERR_TIMEOUT = 2;  // same bit as BFS_ERR_TIMEOUT
 
-// State of a grid-wide barrier of a cooperative kernel (device memory, zeroed
-// before each launch): arrivals of every barrier of the launch so far, sticky
-// error bits.
+// State of a grid-wide barrier of a cooperative kernel, in device memory:
+// arrivals so far, a multiple of the grid's blocks before each launch (a launch
+// whose barriers all complete leaves it so), and sticky error bits, clear before
+// each launch.
 struct GridBarrier {
   unsigned count;
   unsigned reserved;

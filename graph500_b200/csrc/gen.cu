@@ -128,7 +128,7 @@ struct GenParams {
 
 // Mersenne folding: x mod (2^31 - 1) without a division.
 __device__ __forceinline__ uint64_t fold31(uint64_t x) { return (x & MRG_P) + (x >> 31); }
-__device__ __forceinline__ uint32_t reduce31(uint64_t x) {  // x < 2^62
+__device__ __forceinline__ uint32_t reduce31(uint64_t x) {  // x < 2^63
   x = fold31(x);
   x = fold31(x);
   return (uint32_t)(x >= MRG_P ? x - MRG_P : x);

@@ -12,9 +12,8 @@
 // values either way (bfs.hpp:1203, :2470 encoding: parent | level << 48, -1
 // unreached).
 //
-// Packed entry: parent original id in the low PACK_BITS bits, the level
-// above it; 0xFFFFFFFF = unreached.  Graphs with more than 2^PACK_BITS ids,
-// and runs with a level of 31 or more, copy the int64 entries instead.
+// Graphs with more than 2^PACK_BITS ids, and runs with a level over
+// PACK_MAX_LEVEL, copy the int64 entries instead (packed_entry.h).
 #include "g500_internal.cuh"
 #include "pred_expander.h"
 
@@ -78,7 +77,7 @@ __global__ void __launch_bounds__(PACK_THREADS) pack_to_host_kernel(const int64_
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         if (x[k] == -1) {
-          e[k] = PACK_UNREACHED;
+          e[k] = PACK_NONE;
         } else {
           const uint64_t parent = (uint64_t)x[k] & ((1ull << 48) - 1);
           const uint64_t level = (uint64_t)x[k] >> 48;

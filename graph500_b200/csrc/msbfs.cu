@@ -1131,10 +1131,11 @@ __global__ void __launch_bounds__(MS_THREADS, MS_MIN_BLOCKS) msbfs_kernel(MsPara
     const bool settled = pull && p.nhubs == 0;
     if (!settled && !grid_sync<M_NUM>(&ctl->bar, nullptr, sh_acc, nullptr, sh_cnt, &sh_flag)) return;
     if (tid == 0 && !settled) ctl->level_mid_ns[level] = globaltimer();
-    if (settled) {
-    } else if (pull) ms_settle_hubs<NW, SP>(p, act, Fn, level, la);
-    else if (sparse) ms_apply_marked<NW>(p, act, Fn, level, la);
-    else ms_apply<NW, SP>(p, act, Fn, level, la);
+    if (!settled) {
+      if (pull) ms_settle_hubs<NW, SP>(p, act, Fn, level, la);
+      else if (sparse) ms_apply_marked<NW>(p, act, Fn, level, la);
+      else ms_apply<NW, SP>(p, act, Fn, level, la);
+    }
     flush_level<NW, COUNT>(la, sh_acc, sh_or, alive);
     if (!grid_sync_sum<M_NUM>(cnt, &ctl->bar, sh_acc, sh_cnt)) return;
     ++phase;
@@ -1469,9 +1470,8 @@ struct g500_msbfs {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_done = nullptr;
   unsigned grid_full[3] = {0, 0, 0};                  // the whole device's co-resident blocks
   int want_stats = 0;                                 // root statistics enqueued with every one-launch call
-  int in_flight = 0, fl_batches = 0, fl_stats = 0, stats_valid = 0;
+  int in_flight = 0, fl_nroots = 0, fl_batches = 0, fl_stats = 0, stats_valid = 0;
   int run_width = 64;                                 // lane width of the last launch: the layout of V and L
-  std::vector<int64_t> fl_roots, last_roots;
   std::chrono::steady_clock::time_point t_launch;
   cudaGraphExec_t graphs[3][4] = {};                  // [log2(W/32)][batch]
   uint32_t* deg = nullptr;                            // [nlv] row lengths
@@ -1855,7 +1855,7 @@ static int ms_launch(g500_msbfs* m, const int64_t* roots, int nroots, uint8_t* l
   m->fl_stats = m->want_stats && batches == 1;
   if (m->fl_stats) G500_TRY(ms_enqueue_stats(m, nroots, s));
   G500_CUDA(cudaEventRecord(m->ev_done, s));
-  m->fl_roots.assign(roots, roots + nroots);
+  m->fl_nroots = nroots;
   m->fl_batches = batches;
   m->in_flight = 1;
   return G500_OK;
@@ -1869,8 +1869,7 @@ static int ms_complete(g500_msbfs* m, g500_msbfs_stats* stats) {
   cudaError_t ce = cudaEventSynchronize(m->ev_done);
   if (ce != cudaSuccess) return cuda_error(ce, "cudaEventSynchronize", __FILE__, __LINE__);
   const int batches = m->fl_batches;
-  m->last_roots = m->fl_roots;
-  m->last_nroots = (int)m->fl_roots.size();
+  m->last_nroots = m->fl_nroots;
   m->last_batches = batches;
   m->stats_valid = m->fl_stats;
   unsigned err = 0;

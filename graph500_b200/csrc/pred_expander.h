@@ -18,13 +18,9 @@
 #include <thread>
 #include <vector>
 
-namespace g500 {
+#include "packed_entry.h"
 
-// Packed entry: parent original id in the low PACK_BITS bits, the level
-// above it; all ones = unreached.
-constexpr int PACK_BITS = 27;
-constexpr uint32_t PACK_UNREACHED = 0xFFFFFFFFu;
-constexpr int PACK_MAX_LEVEL = 30;  // level 31 with an all-ones parent would read as unreached
+namespace g500 {
 
 // What is known of the work that marks the chunks.
 enum class WorkState { running, complete, refused };
@@ -163,7 +159,7 @@ class PredExpander {
       int64_t* d = dst_;
       for (int64_t i = lo; i < hi; ++i) {
         const uint32_t e = src[i];
-        d[i] = e == PACK_UNREACHED ? -1 : (int64_t)(e & ((1u << PACK_BITS) - 1u)) | ((int64_t)(e >> PACK_BITS) << 48);
+        d[i] = e == PACK_NONE ? -1 : (int64_t)(e & PACK_ID) | ((int64_t)(e >> PACK_BITS) << 48);
       }
     }
   }

@@ -23,15 +23,10 @@ namespace g500 {
 // VE_UNPACKED: entries that do not fit the packed form below (a flag, no error)
 enum { VE_RANGE, VE_ROOT, VE_SELF, VE_DEPTH, VE_EDGE, VE_MISSING, VE_COUNT_EDGES, VE_UNPACKED, VE_N };
 
-// Packed entries: parent in the low VAL_SHIFT bits, the depth above it, for
-// graphs of at most 2^VAL_SHIFT vertex ids and depths of at most 30, and
-// VAL_NONE for an unreached vertex.  The edge pass reads two entries per input
-// edge at random, so their size decides how many come from L2 (SCALE 24: 67 MB
-// instead of 134 MB).
-constexpr int VAL_SHIFT = 27;
-constexpr uint32_t VAL_ID = (1u << VAL_SHIFT) - 1u;
-constexpr uint32_t VAL_NONE = 0xFFFFFFFFu;
-constexpr int VAL_MAX_DEPTH = 30;
+// Packed entries (packed_entry.h) for graphs of at most 2^PACK_BITS vertex ids
+// and depths of at most PACK_MAX_LEVEL.  The edge pass reads two entries per
+// input edge at random, so their size decides how many come from L2 (SCALE 24:
+// 67 MB instead of 134 MB).
 constexpr int VAL_VERTS = 4;  // vertices per thread in flight (vertex and parent passes: 86 / 81 us at SCALE 24 with one)
 
 __device__ __forceinline__ int64_t pred_of(int64_t e) { return (int64_t)((uint64_t)e << 16) >> 16; }  // :809
@@ -72,8 +67,8 @@ __global__ void __launch_bounds__(256) val_vertex_kernel(const int64_t* __restri
       if (i >= nlocal) continue;
       if (pack) {
         const bool none = p == -1 && d == 0xFFFF;
-        unpacked |= !none && (p < 0 || p > (int64_t)VAL_ID || d > VAL_MAX_DEPTH);
-        pack[i] = none ? VAL_NONE : (uint32_t)p | ((uint32_t)d << VAL_SHIFT);
+        unpacked |= !none && (p < 0 || p > (int64_t)PACK_ID || d > PACK_MAX_LEVEL);
+        pack[i] = none ? PACK_NONE : (uint32_t)p | ((uint32_t)d << PACK_BITS);
       }
       if (p < -1 || p >= nglobal) {
         ++range;
@@ -128,15 +123,15 @@ struct EdgeCheck {
   }
   // the same from packed entries: two unreached ends are neither bad nor counted
   __device__ __forceinline__ void packed(uint32_t src, uint32_t tgt, uint32_t ps, uint32_t pt, uint8_t* valid) {
-    if (ps == VAL_NONE || pt == VAL_NONE) {
+    if (ps == PACK_NONE || pt == PACK_NONE) {
       bad += ps != pt;
     } else {
-      const int diff = (int)(ps >> VAL_SHIFT) - (int)(pt >> VAL_SHIFT);
+      const int diff = (int)(ps >> PACK_BITS) - (int)(pt >> PACK_BITS);
       if (diff < -1 || diff > 1) ++bad;
       else ++count;
     }
-    if (ps != VAL_NONE && (ps & VAL_ID) == tgt) valid[src] = 1;
-    if (pt != VAL_NONE && (pt & VAL_ID) == src) valid[tgt] = 1;
+    if (ps != PACK_NONE && (ps & PACK_ID) == tgt) valid[src] = 1;
+    if (pt != PACK_NONE && (pt & PACK_ID) == src) valid[tgt] = 1;
   }
 };
 
@@ -179,8 +174,8 @@ __global__ void __launch_bounds__(256) val_edge_kernel(const g500_packed_edge* _
       uint32_t ps[VAL_EDGES], pt[VAL_EDGES];
 #pragma unroll
       for (int u = 0; u < VAL_EDGES; ++u) {
-        ps[u] = in[u] ? __ldg(pack + ed[u].v0_low) : VAL_NONE;
-        pt[u] = in[u] ? __ldg(pack + ed[u].v1_low) : VAL_NONE;
+        ps[u] = in[u] ? __ldg(pack + ed[u].v0_low) : PACK_NONE;
+        pt[u] = in[u] ? __ldg(pack + ed[u].v1_low) : PACK_NONE;
       }
 #pragma unroll
       for (int u = 0; u < VAL_EDGES; ++u)
@@ -213,7 +208,7 @@ __global__ void __launch_bounds__(256) val_parent_kernel(const int64_t* __restri
 #pragma unroll
     for (int u = 0; u < VAL_VERTS; ++u) {
       const int64_t i = i0 + u * nthreads;
-      reached[u] = i < nlocal && i != root && (use_pack ? pack[i] != VAL_NONE : pred_of(pred[i]) != -1);
+      reached[u] = i < nlocal && i != root && (use_pack ? pack[i] != PACK_NONE : pred_of(pred[i]) != -1);
       ok[u] = i < nlocal && valid[i];
     }
 #pragma unroll
@@ -290,7 +285,7 @@ extern "C" int g500_validate(g500_graph* g, const g500_packed_edge* edges, int64
   scratch.add(&d_valid, nlocal);
   Slab small = scratch;
   uint32_t* d_pack = nullptr;  // packed entries, where the ids allow them
-  const bool can_pack = nlocal <= (int64_t(1) << VAL_SHIFT);
+  const bool can_pack = nlocal <= (int64_t(1) << PACK_BITS);
   if (can_pack) scratch.add(&d_pack, nlocal);
   KeptScratch kept{g, g->d_val.exchange(nullptr), scratch.bytes};
   if (kept.p) scratch.place(kept.p);

@@ -26,7 +26,7 @@ struct Fixture {
   volatile uint32_t ready[CHUNKS] = {};
   Fixture() {
     for (int64_t i = 0; i < N; ++i)
-      src[(size_t)i] = i % 7 == 0 ? PACK_UNREACHED : (uint32_t)(i * 2654435761u) % (31u << PACK_BITS);
+      src[(size_t)i] = i % 7 == 0 ? PACK_NONE : (uint32_t)(i * 2654435761u) % (31u << PACK_BITS);
   }
   void mark(int c, uint32_t run, bool bad = false) {
     std::atomic_thread_fence(std::memory_order_release);
@@ -38,7 +38,7 @@ struct Fixture {
   bool expanded(int64_t b, int64_t e) const {
     for (int64_t i = b; i < e; ++i) {
       const uint32_t p = src[(size_t)i];
-      const int64_t want = p == PACK_UNREACHED ? -1 : (int64_t)(p % (1u << PACK_BITS)) + ((int64_t)(p >> PACK_BITS) << 48);
+      const int64_t want = p == PACK_NONE ? -1 : (int64_t)(p % (1u << PACK_BITS)) + ((int64_t)(p >> PACK_BITS) << 48);
       if (dst[(size_t)i] != want) return false;
     }
     return true;

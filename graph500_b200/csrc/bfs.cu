@@ -524,10 +524,11 @@ __device__ void bu_level(const RunParams& p, const uint32_t* __restrict__ vis_cu
 
 // Late bottom-up levels.  Once few vertices are unvisited, a pass over the
 // bitmap costs more than they do (SCALE 26: 18 us a level for 20 thousand
-// vertices).  So, on graphs of at least BU_LIST_WORDS bitmap words per warp
-// (listing costs 3 us, as much as three listed levels save at SCALE 22 with 16
-// words per warp; SCALE 26 has 221: levels 5-7 29 / 18 / 18 -> 19 / 6 / 5 us) and
-// where the direction rule lets a search with so few unvisited vertices stay
+// vertices).  So, on graphs of at least BU_LIST_WORDS bitmap words per warp (the
+// search without and with lists, where it stays bottom-up: 89.9 / 92.2 us at SCALE
+// 22 with 16 words per warp, 147.4 / 148.5 at SCALE 23 with 30, 199.6 / 196.2 at 24
+// with 59, 346.6 / 335.7 at 25, 658 / 647 at 26, there levels 6-8 18.7 / 17.4 / 17.3
+// -> 12.4 / 5.1 / 4.5) and where the direction rule lets a search with so few unvisited vertices stay
 // bottom-up, a bottom-up level that follows another one ends by listing, per
 // warp and in shared memory, the vertices its own words leave unvisited; if no
 // warp has more than BU_LIST of them, the following bottom-up levels only scan

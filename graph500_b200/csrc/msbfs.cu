@@ -1704,10 +1704,15 @@ extern "C" int g500_msbfs_create(g500_graph* g, g500_msbfs** out) {
     // Fewer blocks on small graphs, whose levels are short against a barrier of
     // all of them.  Launch times in us by blocks per SM, for 32 lanes and 24
     // roots / 64 and 64 / 128 and 128:
-    //   SCALE 16 (65 k vertices)   4: 142 / 191 / 295    2: 129 / 167 / 252
-    //   SCALE 18 (197 k)           4: 248 / 323 / 477    3: 220 / 281 / 423    2: 216 / 261 / 396
-    //   SCALE 20 (655 k)           4: 291 / 390 / 590    3: 292 / 384 / 566    2: 323 / 422 / 615
-    //   SCALE 21 (1.2 M)           4: 282 / 403 / 1551   3: 299 / 403 / 1441   2: 351 / 481 / 1492
+    //   SCALE 16 (66 k vertices)   2: 144 / 189 / 299    3: 150 / 199 / 323    4: 160 / 214 / 353
+    //   SCALE 18 (197 k)           2: 175 / 218 / 324    3: 179 / 226 / 338    4: 193 / 252 / 388
+    //   SCALE 19 (393 k)           2: 146 / 257 / 408    3: 144 / 251 / 403    4: 152 / 260 / 441
+    //   SCALE 20 (655 k)           2: 263 / 396 / 578    3: 241 / 370 / 543    4: 243 / 366 / 548
+    //   SCALE 21 (1.2 M)           2: 323 / 458 / 877    3: 286 / 394 / 759    4: 278 / 400 / 742
+    //   SCALE 22 (2.4 M)           2: 622 / 1025 / 1698  3: 509 / 848 / 1396   4: 480 / 800 / 1350
+    // The lane widths agree on where the lines lie to within 3 %; one block per
+    // SM beats two by 7 % at SCALE 14 with 128 lanes, is within 3 % of it at SCALE
+    // 16 and slower from SCALE 18.
     const unsigned per = g->nlv <= MS_SMALL_VERTS ? 2u : (g->nlv <= MS_MEDIUM_VERTS ? 3u : 4u);
     m->grid[i] = std::min(m->grid_full[i], per * (unsigned)num_sms());
   }

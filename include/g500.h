@@ -339,7 +339,7 @@ int g500_msbfs_get_grid(const g500_msbfs* m, int lane_width, int* blocks, int* m
 /* Sparse levels: a push level whose last frontier has a degree sum of at most
  * `limit` (0 = nlv / 8) works on the marked vertices only (the frontier rows
  * and the vertices it touches) instead of every vertex; on = 0 makes every
- * level dense.  Default: on with nlv / 8 from 2^22 vertices with edges, off
+ * level dense.  Default: on with nlv / 8 from 2^22 num_local_verts, off
  * below.  The levels are the same either way. */
 int g500_msbfs_set_sparse(g500_msbfs* m, int on, int64_t limit);
 /* Device memory one handle on this graph allocates (an upper bound). */

@@ -6,11 +6,10 @@
 // cross.  The runtime's own pageable copy goes through its staging buffers at
 // about half the pinned rate, and a pack kernel followed by one copy and one
 // event per chunk left the link idle between copies and the threads asleep until
-// the first: 470 -> 390 us a call at SCALE 21, 290 -> 125 at SCALE 16, the search
-// included.  A pinned
-// pred keeps its single DMA copy.  The caller's array holds the same int64
-// values either way (bfs.hpp:1203, :2470 encoding: parent | level << 48, -1
-// unreached).
+// the first: a call with its search took 265 / 293 / 1090 / 850 us at SCALE 16 / 18 /
+// 21 / 22 and takes 120 / 148 / 370 / 555.  A pinned pred keeps its single DMA
+// copy.  The caller's array holds the same int64 values either way (bfs.hpp:1203,
+// :2470 encoding: parent | level << 48, -1 unreached).
 //
 // Graphs with more than 2^PACK_BITS ids, and runs with a level over
 // PACK_MAX_LEVEL, copy the int64 entries instead (packed_entry.h).

@@ -297,8 +297,8 @@ __device__ void ms_pull_rows(const MsParams& p, const Mask<NW>& act, const Mask<
   // The loads of a row wait for one another (visited mask, row start, neighbours,
   // their masks), and a launch is bound by that (two thirds of its stalls at SCALE
   // 23), so the mask is loaded two rows ahead, the row start one, and a walk's
-  // next neighbours while it gathers: 64 lanes at SCALE 24 search 1826 -> 1716 us,
-  // 32 at SCALE 18 82 -> 78.  128 lanes have no registers for it (spills, 4 %
+  // next neighbours while it gathers: 64 lanes at SCALE 24 search 1957 -> 1829 us,
+  // 32 at SCALE 18 151 -> 144.  128 lanes have no registers for it (spills, 4 %
   // slower; three blocks per SM instead of four with the registers: 2-5 % faster
   // up to SCALE 21, 6-9 % slower from SCALE 23).
   constexpr bool AHEAD = NW <= 2;
@@ -912,7 +912,7 @@ constexpr int MS_SURVEY_DIV = 64;  // a lane is pushed when its frontier degree 
 // With one survey per launch, spent where the second level already pulled, lanes
 // whose roots lie a step further out kept every row of the dense level scanned
 // to its end, the longest by one warp: 128 roots at SCALE 22 took 7.5 ms (level 3
-// 6.4) and take 1.5 (0.4) with a survey at both; launches that surveyed at the
+// 6.4) and take 1.35 (0.37) with a survey at both; launches that surveyed at the
 // dense level before are the same within 1 %.
 constexpr int MS_SURVEY_FOUND = 4;
 constexpr int MS_SURVEYS = 4;  // at most, each with its own sums

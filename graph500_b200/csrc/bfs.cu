@@ -1189,8 +1189,9 @@ extern "C" int g500_bfs_create(g500_graph* g, g500_bfs** out) {
       st = set_error(G500_E_DEVICE, "device cannot co-schedule the persistent BFS kernel");
     b->grid_full = (unsigned)(num_sms() * std::max(per_sm, 1));
     // one block per SM on small graphs: a barrier of half the blocks is shorter,
-    // and the levels have no work for more (SCALE 16 / 18 / 20: 63.8 / 68.0 / 83.2
-    // us with two blocks per SM, 59.9 / 63.4 / 79.8 with one; SCALE 21: 101.4 / 102.5)
+    // and the levels have no work for more (default thresholds, one block / two:
+    // SCALE 16 53.6 / 57.1 us, 18 60.3 / 64.8, 20 80.6 / 83.5, 21 96.6 / 95.3; without
+    // reordering, 20 92.4 / 89.8 and 21 145.5 / 124.8)
     b->grid = g->nlv <= BFS_SMALL_VERTS ? std::min(b->grid_full, (unsigned)num_sms()) : b->grid_full;
   }
   if (st != G500_OK) {

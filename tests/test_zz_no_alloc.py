@@ -163,9 +163,9 @@ def test_validation_scratch_is_reported_and_not_needed_whole(g500):
     room it keeps its scratch and the graph's device_bytes say so."""
     import torch
 
-    warm = g500.Graph2DCSR.generate(10)  # the kernels are loaded before memory runs short
-    g500.validate_bfs_result(warm, 0, np.full(warm.pred_size(), -1, np.int64))
-    warm.close()
+    small = g500.BfsOnGPU()
+    small.construct(g500.EdgeList(None, 10, 16))
+    g500.validate_bfs_result(small.graph_, 0, np.full(small.graph_.pred_size(), -1, np.int64))  # loads the kernels
     bfs = g500.BfsOnGPU(reorder_mode=2)
     bfs.construct(g500.EdgeList(None, 22, 1))
     bfs.prepare_bfs()
@@ -189,12 +189,11 @@ def test_validation_scratch_is_reported_and_not_needed_whole(g500):
             pass
 
     before, full = held(), []
-    spare = torch.empty(14 << 20, dtype=torch.uint8, device="cuda")  # the flags take 4.2 MB, the rest 17
+    small.prepare_bfs()  # a device allocation of 7 MB; the flags take 4.2, with the packed entries 21
     try:
         for size in (1 << 30, 16 << 20, 1 << 20):
             fill(size, full)
-        del spare
-        torch.cuda.empty_cache()
+        small.end_bfs()
         got = g500.validate_bfs_result(g, root, pred)
     finally:
         full.clear()
@@ -203,6 +202,7 @@ def test_validation_scratch_is_reported_and_not_needed_whole(g500):
     assert got == g500.validate_bfs_result(g, root, pred) and got[0]
     assert before + 5 * n <= held() <= before + 5 * n + 4096
     bfs.close()
+    small.close()
 
 
 @pytest.mark.parametrize("validated", [False, True])

@@ -55,7 +55,7 @@ constexpr uint64_t BFS_DEFERRED_PRED_BYTES = 100ull << 20;
 // 64-bit entries (-1: unreached); a search that goes past PACK_MAX_LEVEL stops,
 // and the host runs it again with 64-bit entries (and keeps them for that
 // handle).
-constexpr int64_t BFS_SMALL_VERTS = 1 << 20;
+constexpr int64_t BFS_SMALL_VERTS = 3 << 18;
 constexpr int BFS_MIN_BLOCKS = 2;        // co-resident blocks per SM (64 registers, no spills)
 constexpr int TD_UNROLL = TD_CHUNK / 32;  // virtual edges per lane per pass
 constexpr int BU_WORDS = 4;               // 32-vertex words a warp keeps in flight (bottom-up pass A)
@@ -1189,9 +1189,10 @@ extern "C" int g500_bfs_create(g500_graph* g, g500_bfs** out) {
       st = set_error(G500_E_DEVICE, "device cannot co-schedule the persistent BFS kernel");
     b->grid_full = (unsigned)(num_sms() * std::max(per_sm, 1));
     // one block per SM on small graphs: a barrier of half the blocks is shorter,
-    // and the levels have no work for more (default thresholds, one block / two:
-    // SCALE 16 53.6 / 57.1 us, 18 60.3 / 64.8, 20 80.6 / 83.5, 21 96.6 / 95.3; without
-    // reordering, 20 92.4 / 89.8 and 21 145.5 / 124.8)
+    // and the levels have no work for more (one block / two, default thresholds and
+    // bottom-up to the end: 66 k vertices 53.6 / 57.1 us, 590 k 81.9 / 84.9 and 65.8 /
+    // 66.5, 786 k 77.8 / 80.4 and 65.0 / 66.1; 852 k 85.3 / 84.8 and 66.0 / 64.8, 983 k
+    // 98.9 / 99.0 and 81.4 / 79.2, 1.05 M unsorted 92.9 / 90.6 and 79.1 / 75.9)
     b->grid = g->nlv <= BFS_SMALL_VERTS ? std::min(b->grid_full, (unsigned)num_sms()) : b->grid_full;
   }
   if (st != G500_OK) {

@@ -38,7 +38,6 @@ namespace g500 {
 constexpr int MS_THREADS = 256;
 constexpr int MS_MIN_BLOCKS = 4;
 constexpr int MS_MAX_LANES = 128;
-constexpr int64_t MS_SMALL_VERTS = 3 << 17, MS_MEDIUM_VERTS = 1 << 20;  // grid choice at creation
 constexpr int MS_MAX_LEVEL = 254;  // level bytes: 255 marks unreached
 // M_ROWS / M_SECT (counting launches only): row and chunk offset reads, and
 // the 32-byte adjacency sectors the level's entries span
@@ -1647,6 +1646,34 @@ static int ms_enqueue_batch(g500_msbfs* m, int b, cudaStream_t s) {
   return G500_OK;
 }
 
+// Blocks per SM of a new handle.  Small graphs' levels are short against a
+// barrier of all the blocks that fit; where the line lies depends on how the ids
+// are ordered: sorted by degree, the warps of the first rows have most of the
+// work, unsorted every warp has its share.  Launch times in us by blocks per SM,
+// for 32 lanes and 24 roots / 64 and 64 / 128 and 128:
+//   sorted (VERTEX_REORDERING 2)
+//     66 k vertices   2: 144 / 189 / 299     3: 150 / 199 / 323    4: 160 / 214 / 353
+//     197 k           2: 175 / 218 / 324     3: 179 / 226 / 338    4: 193 / 252 / 388
+//     393 k           2: 146 / 257 / 408     3: 144 / 251 / 403    4: 152 / 260 / 441
+//     655 k           2: 263 / 396 / 578     3: 241 / 370 / 543    4: 243 / 366 / 548
+//     1.2 M           2: 323 / 458 / 877     3: 286 / 394 / 759    4: 278 / 400 / 742
+//   vertices with edges first (1)
+//     66 k            2: 124 / 168 / 228     3: 127 / 177 / 250    4: 138 / 187 / 273
+//     131 k           2: 138 / 181 / 246     3: 130 / 165 / 230    4: 140 / 180 / 251
+//     393 k           2: 179 / 297 / 474     3: 163 / 264 / 419    4: 175 / 285 / 453
+//     655 k           2: 389 / 526 / 845     3: 337 / 451 / 706    4: 326 / 432 / 678
+//   original order (0)
+//     66 k            2: 119 / 149 / 201     3: 124 / 156 / 222    4: 133 / 169 / 248
+//     131 k           2: 132 / 171 / 240     3: 138 / 181 / 254    4: 138 / 171 / 246
+//     262 k           2: 168 / 243 / 382     3: 156 / 226 / 347    4: 156 / 218 / 341
+//     1.0 M           2: 358 / 607 / 1033    3: 309 / 516 / 877    4: 293 / 471 / 764
+// One block per SM beats two by up to 7 % on the smallest graphs with 128 lanes
+// and loses from 131 k vertices.
+static unsigned ms_blocks_per_sm(int reorder_mode, int64_t nlv) {
+  static const int64_t two[3] = {1 << 17, 1 << 16, 3 << 17}, three[3] = {1 << 17, 3 << 17, 1 << 20};
+  return nlv <= two[reorder_mode] ? 2u : nlv <= three[reorder_mode] ? 3u : 4u;
+}
+
 extern "C" int g500_msbfs_create(g500_graph* g, g500_msbfs** out) {
   if (!g || !out) return set_error(G500_E_INVAL, "null argument");
   G500_CUDA(cudaSetDevice(g->device));
@@ -1701,19 +1728,7 @@ extern "C" int g500_msbfs_create(g500_graph* g, g500_msbfs** out) {
     chk(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernels[i], MS_THREADS, 0), "occupancy");
     if (st == G500_OK && per_sm <= 0) st = set_error(G500_E_DEVICE, "multi-source kernel cannot be co-scheduled");
     m->grid_full[i] = (unsigned)(num_sms() * std::max(per_sm, 1));
-    // Fewer blocks on small graphs, whose levels are short against a barrier of
-    // all of them.  Launch times in us by blocks per SM, for 32 lanes and 24
-    // roots / 64 and 64 / 128 and 128:
-    //   SCALE 16 (66 k vertices)   2: 144 / 189 / 299    3: 150 / 199 / 323    4: 160 / 214 / 353
-    //   SCALE 18 (197 k)           2: 175 / 218 / 324    3: 179 / 226 / 338    4: 193 / 252 / 388
-    //   SCALE 19 (393 k)           2: 146 / 257 / 408    3: 144 / 251 / 403    4: 152 / 260 / 441
-    //   SCALE 20 (655 k)           2: 263 / 396 / 578    3: 241 / 370 / 543    4: 243 / 366 / 548
-    //   SCALE 21 (1.2 M)           2: 323 / 458 / 877    3: 286 / 394 / 759    4: 278 / 400 / 742
-    //   SCALE 22 (2.4 M)           2: 622 / 1025 / 1698  3: 509 / 848 / 1396   4: 480 / 800 / 1350
-    // The lane widths agree on where the lines lie to within 3 %; one block per
-    // SM beats two by 7 % at SCALE 14 with 128 lanes, is within 3 % of it at SCALE
-    // 16 and slower from SCALE 18.
-    const unsigned per = g->nlv <= MS_SMALL_VERTS ? 2u : (g->nlv <= MS_MEDIUM_VERTS ? 3u : 4u);
+    const unsigned per = ms_blocks_per_sm(g->reorder_mode, g->nlv);
     m->grid[i] = std::min(m->grid_full[i], per * (unsigned)num_sms());
   }
   if (st != G500_OK) {

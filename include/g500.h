@@ -207,7 +207,7 @@ int g500_bfs_set_pred_mode(g500_bfs* b, int mode);
 int g500_bfs_set_host_pack(g500_bfs* b, int on);
 /* Blocks of the persistent kernel (0 = every co-resident block of the device;
  * a new handle starts with that, or with one block per SM on graphs of at most
- * 2^20 num_local_verts); fewer leave SMs to kernels of other handles
+ * 786432 num_local_verts); fewer leave SMs to kernels of other handles
  * running at the same time. */
 int g500_bfs_set_grid(g500_bfs* b, int blocks);
 
@@ -331,8 +331,7 @@ int g500_msbfs_wait(g500_msbfs* m, g500_msbfs_stats* stats);
  * statistics of g500_msbfs_root_stats on the device, in the same stream. */
 int g500_msbfs_set_root_stats(g500_msbfs* m, int on);
 /* Blocks per launch (0 = every co-resident block of the device; a new handle
- * starts with that, or with fewer on graphs of at most 2^20 num_local_verts).
- * Fewer blocks leave SMs to launches of other handles running at the
+ * starts with that, or with fewer on small graphs).  Fewer blocks leave SMs to launches of other handles running at the
  * same time. */
 int g500_msbfs_set_grid(g500_msbfs* m, int blocks);
 int g500_msbfs_get_grid(const g500_msbfs* m, int lane_width, int* blocks, int* max_blocks);

@@ -251,6 +251,21 @@ def test_msbfs_levels_into_device_memory(g500, s13, offset, lanes, n):
     ms.close()
 
 
+@pytest.mark.parametrize("vr,scale,per_sm", [(0, 17, 2), (0, 18, 4), (1, 16, 2), (1, 18, 3), (1, 20, 4), (2, 18, 2),
+                                             (2, 20, 3), (2, 21, 4)])
+def test_msbfs_default_grid_follows_size_and_order(g500, vr, scale, per_sm):
+    """A new handle's blocks per SM, by graph size and vertex order, at most what the device can hold."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    g = g500.Graph2DCSR.generate(scale, 16, vr)
+    ms = g500.MultiSourceBFS(g, 64)
+    for lanes in (32, 64, 128):
+        blocks, most = ms.grid(lanes)
+        assert blocks == min(per_sm * sms, most)
+    ms.close()
+    g.close()
+
+
 @pytest.mark.parametrize("spare", [0, 1])
 def test_msbfs_refuses_device_memory_shorter_than_its_rows(g500, spare):
     """A device allocation that ends inside the rows is refused by the call (the output pass must not write past

@@ -1325,8 +1325,14 @@ __global__ void ms_degree_kernel(const uint64_t* __restrict__ off, int64_t nlv, 
 // reached count follow).  Nearly every vertex is reached by every lane, so a
 // warp looks at single lanes only for the words where one of its 32 vertices
 // lacks some: SCALE 24, 64 roots: two reductions per lane and 32 vertices took
-// 1.03 ms, now 0.13 ms with its launches.  A vertex without edges can
-// only be a root itself: its lane's missing sums get it taken off.
+// 1.03 ms, now 0.13 ms with its launches.  Lanes that lack a word's vertices
+// altogether (roots in small components lack nearly all) get its totals without a
+// look of their own, and each thread keeps the sums of one lane per mask word, so
+// that no lane costs an atomic per word: 2^21 pairs of vertices, 64 roots: 455 us
+// a call with shared-memory atomics, 59 now, 193 when every lane was reduced;
+// SCALE 24, 64 roots 114 -> 96 us.
+// A vertex without edges can only be a root itself: its lane's missing sums get it
+// taken off.
 // The last block to finish turns the sums into each root's reached count and 2 x
 // nedge (a root outside the CSR range, without edges, reached only itself; its
 // self-loop occurrences are its edge count) and clears them for the next call.
@@ -1348,6 +1354,9 @@ __global__ void __launch_bounds__(256) ms_stats_kernel(const uint32_t* __restric
   __syncthreads();
   const int lane = threadIdx.x & 31;
   unsigned long long nv = 0, ne = 0;
+  unsigned long long miss[NW], miss_e2[NW];  // of lane 32 * k + this thread's place in its warp
+#pragma unroll
+  for (int k = 0; k < NW; ++k) miss[k] = miss_e2[k] = 0;
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < nlv;  // nlv: a multiple of 32
        base += (int64_t)gridDim.x * blockDim.x) {
     const int64_t v = base + lane;
@@ -1365,18 +1374,26 @@ __global__ void __launch_bounds__(256) ms_stats_kernel(const uint32_t* __restric
       any |= x[k] != 0;
     }
     if (!__any_sync(FULL_MASK, any)) continue;
+    const unsigned word_v = __popc(__ballot_sync(FULL_MASK, has));
+    const unsigned word_e = __reduce_add_sync(FULL_MASK, has ? e : 0u);
 #pragma unroll
     for (int k = 0; k < NW; ++k) {
-      unsigned todo = __reduce_or_sync(FULL_MASK, has ? x[k] : 0u);
+      const unsigned lack = __reduce_or_sync(FULL_MASK, has ? x[k] : 0u);
+      const unsigned some = __reduce_or_sync(FULL_MASK, has ? m.w[k] : 0u);  // lanes that reached one of the word
+      if ((lack & ~some) >> lane & 1u) {
+        miss[k] += word_v;
+        miss_e2[k] += word_e;
+      }
+      unsigned todo = lack & some;
       while (todo) {
         const int b = __ffs(todo) - 1;
         todo &= todo - 1;
-        const bool miss = has && ((x[k] >> b) & 1u);
-        const unsigned rs = __popc(__ballot_sync(FULL_MASK, miss));
-        const unsigned es = __reduce_add_sync(FULL_MASK, miss ? e : 0u);
-        if (lane == 0) {
-          atomicAdd(&s_r[k * 32 + b], (unsigned long long)rs);
-          atomicAdd(&s_e[k * 32 + b], (unsigned long long)es);
+        const bool mine = has && ((x[k] >> b) & 1u);
+        const unsigned rs = __popc(__ballot_sync(FULL_MASK, mine));
+        const unsigned es = __reduce_add_sync(FULL_MASK, mine ? e : 0u);
+        if (lane == b) {
+          miss[k] += rs;
+          miss_e2[k] += es;
         }
       }
       if (!has)
@@ -1387,6 +1404,12 @@ __global__ void __launch_bounds__(256) ms_stats_kernel(const uint32_t* __restric
         }
     }
   }
+#pragma unroll
+  for (int k = 0; k < NW; ++k)
+    if (miss[k]) {
+      atomicAdd(&s_r[k * 32 + lane], miss[k]);
+      atomicAdd(&s_e[k * 32 + lane], miss_e2[k]);
+    }
   nv = warp_sum(nv);
   ne = warp_sum(ne);
   if (lane == 0) {

@@ -251,6 +251,38 @@ def test_msbfs_levels_into_device_memory(g500, s13, offset, lanes, n):
     ms.close()
 
 
+@pytest.mark.parametrize("vr", [0, 1, 2])
+def test_msbfs_root_stats_in_small_components(g500, vr):
+    """Components of 1 to 40 vertices (some with self loops and double edges) around bitmap words: a word's
+    vertices reached by no root, by some lanes, whole or in part, and roots without edges."""
+    rng = np.random.default_rng(7)
+    pairs, ids, nxt = [], rng.permutation(70000), 0
+    for size in list(range(1, 41)) * 4:
+        c = ids[nxt:nxt + size]
+        nxt += size
+        pairs += [(c[rng.integers(0, i)], c[i]) for i in range(1, size)] + [(c[0], c[0])] * int(size % 5 == 0)
+        pairs += [(c[0], c[size - 1])] * int(size % 3)
+    edges = np.zeros(len(pairs), g500.EDGE_DTYPE)
+    edges["v0_low"], edges["v1_low"] = np.array(pairs).T
+    bfs = g500.BfsOnGPU(reorder_mode=vr)
+    bfs.construct(edges)
+    bfs.prepare_bfs()
+    roots = np.concatenate([ids[rng.integers(0, nxt, 120)], ids[-8:]])  # the last: no edges
+    pred = np.zeros(bfs.graph_.pred_size(), np.int64)
+    want = []
+    for r in roots:
+        st = bfs.run_bfs(int(r), pred)
+        want.append((st.reached, st.nedge))
+    for lanes in (32, 64, 128):
+        ms = g500.MultiSourceBFS(bfs.graph_, lanes)
+        for part in (roots[:lanes], roots[-lanes:], roots[:1]):
+            ms.run(part)
+            got = list(zip(*(a.tolist() for a in ms.root_stats(len(part)))))
+            assert got == [want[list(roots).index(r)] for r in part], lanes
+        ms.close()
+    bfs.close()
+
+
 @pytest.mark.parametrize("vr,scale,per_sm", [(0, 17, 2), (0, 18, 4), (1, 16, 2), (1, 18, 3), (1, 20, 4), (2, 18, 2),
                                              (2, 20, 3), (2, 21, 4)])
 def test_msbfs_default_grid_follows_size_and_order(g500, vr, scale, per_sm):

@@ -55,7 +55,6 @@ constexpr uint64_t BFS_DEFERRED_PRED_BYTES = 100ull << 20;
 // 64-bit entries (-1: unreached); a search that goes past PACK_MAX_LEVEL stops,
 // and the host runs it again with 64-bit entries (and keeps them for that
 // handle).
-constexpr int64_t BFS_SMALL_VERTS = 3 << 18;
 constexpr int BFS_MIN_BLOCKS = 2;        // co-resident blocks per SM (64 registers, no spills)
 constexpr int TD_UNROLL = TD_CHUNK / 32;  // virtual edges per lane per pass
 constexpr int BU_WORDS = 4;               // 32-vertex words a warp keeps in flight (bottom-up pass A)
@@ -1009,16 +1008,39 @@ __global__ void __launch_bounds__(FINAL_THREADS, 8) deferred_pred_kernel(RunPara
   }
 }
 
-// endw[w] = sum of endp over the vertices with edges of word w (a warp per word)
-__global__ void __launch_bounds__(256) word_ends_kernel(const uint32_t* __restrict__ vis_init,
+// endw[w] = sum of endp over the vertices with edges of word w (a warp per word);
+// *longest = the longest row, at most 2^32 - 1
+__global__ void __launch_bounds__(256) word_ends_kernel(const uint64_t* __restrict__ off,
+                                                        const uint32_t* __restrict__ vis_init,
                                                         const uint32_t* __restrict__ endp, int64_t nwords,
-                                                        unsigned long long* __restrict__ endw) {
+                                                        unsigned long long* __restrict__ endw, unsigned* longest) {
   const int lane = threadIdx.x & 31;
+  unsigned most = 0;
   for (int64_t wi = gwarp_id(); wi < nwords; wi += gwarp_count()) {
+    const int64_t r = wi * 32 + lane;
     const bool has = !((__ldg(vis_init + wi) >> lane) & 1u);
-    const unsigned long long v = warp_sum(has ? (unsigned long long)__ldg(endp + wi * 32 + lane) : 0ull);
+    const unsigned long long v = warp_sum(has ? (unsigned long long)__ldg(endp + r) : 0ull);
     if (lane == 0) endw[wi] = v;
+    most = max(most, (unsigned)min(__ldg(off + r + 1) - __ldg(off + r), (uint64_t)0xFFFFFFFFu));
   }
+  most = __reduce_max_sync(FULL_MASK, most);
+  if (lane == 0 && most) atomicMax(longest, most);
+}
+
+// Blocks of the search on graphs of few vertices: one per SM where a barrier of
+// half the blocks gains more than the levels lose by half the threads.  That is so
+// on every graph of 66 thousand vertices, and on larger ones while they have few
+// entries (random graphs) or hubs that end most bottom-up rows early (Kronecker
+// graphs).  One block / two per SM in us, default thresholds and bottom-up to the
+// end: SCALE 16 54 / 57 and 48 / 50, 18 64 / 70 and 54 / 58, 20 76 / 80 and 62 / 63;
+// random graphs of 2^16 vertices and 8 M entries 78 / 84, 2^18 and 4 M 89 / 91 and 83 /
+// 84, 2^19 and 8 M 127 / 126 and 109 / 108, but 2^17 and 17 M 138 / 93 and 126 / 93, 2^18
+// and 34 M 261 / 172; Kronecker graphs of 852 k vertices 85.3 / 84.8 and 66.0 / 64.8, of
+// 1.05 M unsorted 92.9 / 90.6 and 79.1 / 75.9.
+static bool bfs_small_grid(const g500_graph* g, unsigned longest_row) {
+  constexpr int64_t ANY = 1 << 16, MOST = 3 << 18, ENTRIES = 1 << 23, HUB = 64;
+  if (g->nlv <= ANY) return true;
+  return g->nlv <= MOST && (g->nge <= ENTRIES || (int64_t)longest_row >= HUB * (g->nge / g->nlv));
 }
 
 }  // namespace g500
@@ -1164,12 +1186,18 @@ extern "C" int g500_bfs_create(g500_graph* g, g500_bfs** out) {
   slab.add(&b->d_rec, MAX_LEVELS);
   slab.add(&b->d_big, BIG_ROWS);
   slab.add(&b->d_endw, nwords);
+  unsigned* longest = nullptr;
+  slab.add(&longest, 1);
+  unsigned longest_row = 0;
   if ((uint64_t)g->nolv * 8 > BFS_DEFERRED_PRED_BYTES) slab.add(&b->d_pred_r, std::max<int64_t>(g->nlv, 1));
   if (st == G500_OK) st = slab.alloc(&b->d_slab, "pred, visited bitmaps and top-down queues");
   if (st == G500_OK && g->nlv > 0) {
     const unsigned wg = (unsigned)std::min<int64_t>(ceil_div(nwords * 32, 256), (int64_t)num_sms() * 8);
-    word_ends_kernel<<<wg, 256, 0, b->own_stream>>>(g->d_vis_init, g->d_endp, g->nlv / 32, b->d_endw);
+    chk(cudaMemsetAsync(longest, 0, sizeof(unsigned), b->own_stream), "longest row");
+    word_ends_kernel<<<wg, 256, 0, b->own_stream>>>(g->d_offsets, g->d_vis_init, g->d_endp, g->nlv / 32, b->d_endw,
+                                                    longest);
     chk(cudaGetLastError(), "endpoint counts per bitmap word");
+    chk(cudaMemcpyAsync(&longest_row, longest, sizeof(unsigned), cudaMemcpyDeviceToHost, b->own_stream), "longest row");
     chk(cudaStreamSynchronize(b->own_stream), "endpoint counts per bitmap word");
   }
   void* h_ctl = nullptr;
@@ -1188,12 +1216,7 @@ extern "C" int g500_bfs_create(g500_graph* g, g500_bfs** out) {
     if (st == G500_OK && (!coop || per_sm <= 0))
       st = set_error(G500_E_DEVICE, "device cannot co-schedule the persistent BFS kernel");
     b->grid_full = (unsigned)(num_sms() * std::max(per_sm, 1));
-    // one block per SM on small graphs: a barrier of half the blocks is shorter,
-    // and the levels have no work for more (one block / two, default thresholds and
-    // bottom-up to the end: 66 k vertices 53.6 / 57.1 us, 590 k 81.9 / 84.9 and 65.8 /
-    // 66.5, 786 k 77.8 / 80.4 and 65.0 / 66.1; 852 k 85.3 / 84.8 and 66.0 / 64.8, 983 k
-    // 98.9 / 99.0 and 81.4 / 79.2, 1.05 M unsorted 92.9 / 90.6 and 79.1 / 75.9)
-    b->grid = g->nlv <= BFS_SMALL_VERTS ? std::min(b->grid_full, (unsigned)num_sms()) : b->grid_full;
+    b->grid = bfs_small_grid(g, longest_row) ? std::min(b->grid_full, (unsigned)num_sms()) : b->grid_full;
   }
   if (st != G500_OK) {
     bfs_free(b);

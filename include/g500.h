@@ -206,9 +206,8 @@ int g500_bfs_set_pred_mode(g500_bfs* b, int mode);
  * the values are the same. */
 int g500_bfs_set_host_pack(g500_bfs* b, int on);
 /* Blocks of the persistent kernel (0 = every co-resident block of the device;
- * a new handle starts with that, or with one block per SM on graphs of at most
- * 786432 num_local_verts); fewer leave SMs to kernels of other handles
- * running at the same time. */
+ * a new handle starts with that, or with one block per SM on small graphs);
+ * fewer leave SMs to kernels of other handles running at the same time. */
 int g500_bfs_set_grid(g500_bfs* b, int blocks);
 
 /* Autotuner: time every (policy, alpha, beta) of a built-in grid on the given

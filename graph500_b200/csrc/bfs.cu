@@ -528,12 +528,21 @@ __device__ void bu_level(const RunParams& p, const uint32_t* __restrict__ vis_cu
 // 22 with 16 words per warp, 147.4 / 148.5 at SCALE 23 with 30, 199.6 / 196.2 at 24
 // with 59, 346.6 / 335.7 at 25, 658 / 647 at 26, there levels 6-8 18.7 / 17.4 / 17.3
 // -> 12.4 / 5.1 / 4.5) and where the direction rule lets a search with so few unvisited vertices stay
-// bottom-up, a bottom-up level that follows another one ends by listing, per
+// bottom-up, a bottom-up level that follows another one may end by listing, per
 // warp and in shared memory, the vertices its own words leave unvisited; if no
 // warp has more than BU_LIST of them, the following bottom-up levels only scan
 // the listed rows.  The visited maps still alternate: a listed level writes the
 // other buffer, which it first brings up to date with its own words (the first
 // such level) or with the vertices it found one level before.
+// Whether a bottom-up level that starts with `left` unvisited vertices, after one
+// that found `found`, is worth ending with a list: the last one took half of them
+// or more, or they fit several times over.  Where many vertices are never reached,
+// a try after every level made each of them 8-9 us longer (16 M vertices of mean
+// degree 3: tail levels 32 us instead of 23).
+__device__ __forceinline__ bool list_now(int64_t left, int64_t found) {
+  return found >= left || left <= BU_LIST * gwarp_count() / 4;
+}
+
 // List what the level leaves; a warp with too many raises C_BIG, which
 // bottom-up levels do not use otherwise.
 __device__ void bu_collect(const RunParams& p, const uint32_t* vis_next, WarpLists& wl, unsigned long long* sh_acc) {
@@ -845,7 +854,10 @@ __global__ void __launch_bounds__(BFS_THREADS, BFS_MIN_BLOCKS) bfs_persistent_ke
         if (tid == 0) ++ctl->list_levels;
       } else {
         bu_level<DEF>(p, p.vis[cur_vis], p.vis[cur_vis ^ 1], sh_acc, lvl);
-        if (LISTS && bu_before) bu_collect(p, p.vis[cur_vis ^ 1], lists, sh_acc);
+        if (LISTS && bu_before) {
+          if (list_now(p.ngv - visited, prev_nq)) bu_collect(p, p.vis[cur_vis ^ 1], lists, sh_acc);
+          else if (tid == 0) sh_acc[C_BIG] = 1;  // not listed
+        }
       }
       if (!grid_sync_sum<C_NUM>(cnt, &ctl->bar, sh_acc, sh_cnt)) return;
       if (LISTS && (listed_levels >= 0 || (bu_before && sh_cnt[C_BIG] == 0))) ++listed_levels;

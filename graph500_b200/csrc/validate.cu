@@ -136,11 +136,10 @@ struct EdgeCheck {
 };
 
 // Bound by the random reads of the ends' entries (two per edge).  pack: the
-// packed entries, or null; used when every entry fitted.  Four edges per
-// thread (three 16-byte loads where the list is aligned to that) keep eight
-// reads in flight.  SCALE 24 (268 M edges, 134 MB of pred): one edge at a time on
-// pred itself 2.85 ms; a repeated validation 3.0 -> 2.4 ms.
-constexpr int VAL_EDGES = 4;
+// packed entries, or null; used when every entry fitted.  U edges per thread, their
+// reads in flight together (four as three 16-byte loads where the list is aligned
+// to that).  What pays depends on where the entries lie (see val_packs).
+template <int U>
 __global__ void __launch_bounds__(256) val_edge_kernel(const g500_packed_edge* __restrict__ edges, int64_t m,
                                                        const int64_t* __restrict__ pred,
                                                        const uint32_t* __restrict__ pack, int64_t nlocal,
@@ -149,46 +148,46 @@ __global__ void __launch_bounds__(256) val_edge_kernel(const g500_packed_edge* _
   const bool wide = (reinterpret_cast<uintptr_t>(edges) & 15) == 0;
   EdgeCheck c;
   const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * VAL_EDGES; i0 < m;
-       i0 += nthreads * VAL_EDGES) {
-    g500_packed_edge ed[VAL_EDGES];
-    const int n = (int)min((int64_t)VAL_EDGES, m - i0);
-    if (wide && n == VAL_EDGES) {  // i0 is a multiple of 4 edges: 48 bytes
+  for (int64_t i0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * U; i0 < m;
+       i0 += nthreads * U) {
+    g500_packed_edge ed[U];
+    const int n = (int)min((int64_t)U, m - i0);
+    if (U == 4 && wide && n == U) {  // i0 is a multiple of 4 edges: 48 bytes
       const uint4* q = reinterpret_cast<const uint4*>(edges + i0);
       const uint4 a = __ldcs(q), b = __ldcs(q + 1), d = __ldcs(q + 2);
       ed[0] = {a.x, a.y, a.z};
-      ed[1] = {a.w, b.x, b.y};
-      ed[2] = {b.z, b.w, d.x};
-      ed[3] = {d.y, d.z, d.w};
+      ed[1 % U] = {a.w, b.x, b.y};
+      ed[2 % U] = {b.z, b.w, d.x};
+      ed[3 % U] = {d.y, d.z, d.w};
     } else {
 #pragma unroll
-      for (int u = 0; u < VAL_EDGES; ++u) ed[u] = u < n ? edges[i0 + u] : edges[i0];
+      for (int u = 0; u < U; ++u) ed[u] = u < n ? edges[i0 + u] : edges[i0];
     }
-    bool in[VAL_EDGES];
+    bool in[U];
 #pragma unroll
-    for (int u = 0; u < VAL_EDGES; ++u) {
+    for (int u = 0; u < U; ++u) {
       in[u] = u < n && ev0(ed[u]) < nlocal && ev1(ed[u]) < nlocal;
       c.bad += u < n && !in[u];
     }
     if (use_pack) {
-      uint32_t ps[VAL_EDGES], pt[VAL_EDGES];
+      uint32_t ps[U], pt[U];
 #pragma unroll
-      for (int u = 0; u < VAL_EDGES; ++u) {
+      for (int u = 0; u < U; ++u) {
         ps[u] = in[u] ? __ldg(pack + ed[u].v0_low) : PACK_NONE;
         pt[u] = in[u] ? __ldg(pack + ed[u].v1_low) : PACK_NONE;
       }
 #pragma unroll
-      for (int u = 0; u < VAL_EDGES; ++u)
+      for (int u = 0; u < U; ++u)
         if (in[u]) c.packed(ed[u].v0_low, ed[u].v1_low, ps[u], pt[u], valid);
     } else {
-      int64_t ps[VAL_EDGES], pt[VAL_EDGES];
+      int64_t ps[U], pt[U];
 #pragma unroll
-      for (int u = 0; u < VAL_EDGES; ++u) {
+      for (int u = 0; u < U; ++u) {
         ps[u] = in[u] ? pred[ev0(ed[u])] : 0;
         pt[u] = in[u] ? pred[ev1(ed[u])] : 0;
       }
 #pragma unroll
-      for (int u = 0; u < VAL_EDGES; ++u)
+      for (int u = 0; u < U; ++u)
         if (in[u]) c.full(ev0(ed[u]), ev1(ed[u]), ps[u], pt[u], valid);
     }
   }
@@ -215,6 +214,39 @@ __global__ void __launch_bounds__(256) val_parent_kernel(const int64_t* __restri
     for (int u = 0; u < VAL_VERTS; ++u) missing += reached[u] && !ok[u];
   }
   warp_add(&err[VE_MISSING], missing);
+}
+
+// Whether the entries are packed for the edge pass, and how many edges a thread
+// takes there.  Up to 2^20 ids the 64-bit entries stay in L2; up to 2^19 more threads
+// with one edge each hide their latency best: a validation at SCALE 16 / 17 / 18 takes
+// 67 / 68 / 82 us so, 81 / 94 / 107 from packed entries by four edges and 81 / 83 / 102
+// by two; at SCALE 20 64-bit entries take 182 us by four edges and 190 by one, packed
+// ones 196 and 206.  Above, packed entries halve what is read, two edges a thread up to
+// 2^23 ids (SCALE 21 / 23 327 / 1164 us, four 327 / 1162, one 340 / 1179), four beyond
+// (SCALE 24 2381 us, two 2478, one 2520).  64-bit entries without the memory for
+// packed ones, SCALE 22: 567 us by four edges, 592 by one.
+static bool val_packs(int64_t nlocal) {
+  return nlocal > int64_t(1) << 20 && nlocal <= int64_t(1) << PACK_BITS;
+}
+static int val_edges(bool packed, int64_t nlocal) {
+  if (packed) return nlocal <= int64_t(1) << 23 ? 2 : 4;
+  return nlocal <= int64_t(1) << 19 ? 1 : 4;
+}
+
+// The three passes over a result (the root's check and the counters' clearing apart).
+static void val_passes(const g500_packed_edge* edges, int64_t m, const int64_t* pred, uint32_t* pack, int64_t nlocal,
+                       int64_t nglobal, int64_t root, uint8_t* valid, unsigned long long* err, cudaStream_t s) {
+  const int64_t most = (int64_t)num_sms() * 16;
+  const unsigned vgrid = (unsigned)std::min<int64_t>(ceil_div(nlocal, 256), most);
+  const unsigned egrid = (unsigned)std::min<int64_t>(ceil_div(m, 256), most);
+  val_vertex_kernel<<<vgrid, 256, 0, s>>>(pred, nlocal, nglobal, root, pack, err);
+  const int per = val_edges(pack != nullptr, nlocal);
+  if (m > 0) {
+    if (per == 1) val_edge_kernel<1><<<egrid, 256, 0, s>>>(edges, m, pred, pack, nlocal, valid, err);
+    else if (per == 2) val_edge_kernel<2><<<egrid, 256, 0, s>>>(edges, m, pred, pack, nlocal, valid, err);
+    else val_edge_kernel<4><<<egrid, 256, 0, s>>>(edges, m, pred, pack, nlocal, valid, err);
+  }
+  val_parent_kernel<<<vgrid, 256, 0, s>>>(pred, pack, nlocal, root, valid, err);
 }
 
 // A call's scratch, given back to the graph at its end (or freed, where another
@@ -285,7 +317,7 @@ extern "C" int g500_validate(g500_graph* g, const g500_packed_edge* edges, int64
   scratch.add(&d_valid, nlocal);
   Slab small = scratch;
   uint32_t* d_pack = nullptr;  // packed entries, where the ids allow them
-  const bool can_pack = nlocal <= (int64_t(1) << PACK_BITS);
+  const bool can_pack = val_packs(nlocal);
   if (can_pack) scratch.add(&d_pack, nlocal);
   KeptScratch kept{g, g->d_val.exchange(nullptr), scratch.bytes};
   if (kept.p) scratch.place(kept.p);
@@ -298,12 +330,8 @@ extern "C" int g500_validate(g500_graph* g, const g500_packed_edge* edges, int64
   cudaError_t e = cudaMemsetAsync(d_err, 0, sizeof(unsigned long long) * VE_N, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_valid, 0, (size_t)nlocal, s);
   if (e != cudaSuccess) { cleanup(); return cuda_error(e, "cudaMemsetAsync", __FILE__, __LINE__); }
-  const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(std::max<int64_t>(nlocal, m), 256),
-                                                    (int64_t)num_sms() * 16);
   val_root_kernel<<<1, 1, 0, s>>>(d_pred, root, nlocal, d_err);
-  val_vertex_kernel<<<grid, 256, 0, s>>>(d_pred, nlocal, nglobal, root, d_pack, d_err);
-  if (m > 0) val_edge_kernel<<<grid, 256, 0, s>>>(d_edges, m, d_pred, d_pack, nlocal, d_valid, d_err);
-  val_parent_kernel<<<grid, 256, 0, s>>>(d_pred, d_pack, nlocal, root, d_valid, d_err);
+  val_passes(d_edges, m, d_pred, d_pack, nlocal, nglobal, root, d_valid, d_err, s);
   e = cudaGetLastError();
   unsigned long long h[VE_N];
   if (e == cudaSuccess) e = cudaMemcpyAsync(h, d_err, sizeof(h), cudaMemcpyDeviceToHost, s);
@@ -406,13 +434,8 @@ extern "C" int g500_validate_noalloc(const g500_packed_edge* dev_edges, int64_t 
   // the arrays keep the last call's contents: clear what must start at zero
   G500_CUDA(cudaMemsetAsync(sc.err, 0, sizeof(unsigned long long) * VE_N, s));
   G500_CUDA(cudaMemsetAsync(sc.valid, 0, (size_t)nlocalverts, s));
-  const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(std::max<int64_t>(nlocalverts, num_edges), 256),
-                                                    (int64_t)num_sms() * 16);
   val_root_kernel<<<1, 1, 0, s>>>(dev_pred, root, nlocalverts, sc.err);
-  val_vertex_kernel<<<grid, 256, 0, s>>>(dev_pred, nlocalverts, nglobalverts, root, nullptr, sc.err);
-  if (num_edges > 0)
-    val_edge_kernel<<<grid, 256, 0, s>>>(dev_edges, num_edges, dev_pred, nullptr, nlocalverts, sc.valid, sc.err);
-  val_parent_kernel<<<grid, 256, 0, s>>>(dev_pred, nullptr, nlocalverts, root, sc.valid, sc.err);
+  val_passes(dev_edges, num_edges, dev_pred, nullptr, nlocalverts, nglobalverts, root, sc.valid, sc.err, s);
   G500_CUDA(cudaGetLastError());
   unsigned long long h[VE_N];
   G500_CUDA(cudaMemcpyAsync(h, sc.err, sizeof(h), cudaMemcpyDeviceToHost, s));

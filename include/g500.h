@@ -250,8 +250,8 @@ typedef struct g500_validate_report {
  * max_used_vertex + 1 and nlocalverts = pred_size, as main.cc:129-133 calls
  * it.  edges == NULL uses the graph's resident edge list.  *ok = 1 when the
  * result is valid; *edge_visit_count = the traversed-edge count TEPS uses.
- * The first call allocates 5 bytes of scratch per original id (1 above 2^27
- * ids), which the graph then holds and counts in device_bytes; where only 1
+ * The first call allocates 5 bytes of scratch per original id (1 up to 2^20
+ * and above 2^27 ids), which the graph then holds and counts in device_bytes; where only 1
  * byte per id is free, a call does with that and holds nothing. */
 int g500_validate(g500_graph* g, const g500_packed_edge* edges, int64_t num_edges,
                   int edges_on_device, int64_t root, const int64_t* pred, int pred_on_device,

@@ -222,3 +222,47 @@ def test_device_bytes_is_what_a_graph_holds(g500, validated):
     g.close()
     held = torch.cuda.mem_get_info()[0] - free
     assert info.device_bytes <= held <= info.device_bytes + (4 << 21)
+
+
+@pytest.mark.parametrize("planted", ["none", "level", "deep", "deepest", "self", "range", "negative", "half_reached",
+                                     "unreached"])
+def test_validation_reports_alike_at_every_size(g500, planted):
+    """The edge pass reads 64-bit entries, one edge a thread up to 2^19 ids and four up to 2^20, then packed ones,
+    two edges a thread up to 2^23 and four above.  The same small graph among 2^16 to 2^24 ids, right and planted,
+    for edge lists at every alignment and remainder: every count is the same."""
+    import torch
+
+    rng = np.random.default_rng(11)
+    ids = rng.integers(0, 3000, (20001, 2))
+    reports = {}
+    for lg in (16, 19, 20, 21, 23, 24):
+        edges = np.zeros(len(ids) + 1, g500.EDGE_DTYPE)
+        edges["v0_low"][:-1], edges["v1_low"][:-1] = ids.T
+        edges["v0_low"][-1] = edges["v1_low"][-1] = (1 << lg) - 1  # a self loop that sets the number of ids
+        bfs = g500.BfsOnGPU(reorder_mode=2)
+        bfs.construct(edges)
+        bfs.prepare_bfs()
+        g = bfs.graph_
+        assert g.pred_size() == 1 << lg
+        root = int(ids[0, 0])
+        pred = np.zeros(g.pred_size(), np.int64)
+        bfs.run_bfs(root, pred)
+        reached = np.nonzero((pred != -1) & (np.arange(len(pred)) != root))[0]
+        v, w = (int(x) for x in reached[[len(reached) // 3, len(reached) // 2]])
+        parent, level = min(int(n) for n in np.concatenate([ids[ids[:, 0] == v, 1], ids[ids[:, 1] == v, 0]])
+                            if int(pred[n]) >> 48 == (int(pred[v]) >> 48) - 1), int(pred[v]) >> 48
+        pred[v] = {"none": parent | level << 48, "level": parent | (level + 1) << 48, "deep": parent | 30 << 48,
+                   "deepest": parent | 31 << 48, "self": v | level << 48, "range": 1 << 30 | level << 48,
+                   "negative": -2, "half_reached": 0xFFFFFFFFFFFF | level << 48, "unreached": -1}[planted]
+        dev, elist = torch.from_numpy(pred).cuda(), torch.from_numpy(edges.view(np.int32)).cuda()
+        for skip, drop in ((0, 0), (1, 0), (2, 1), (3, 2)):
+            evc, ok, rep = C.c_int64(), C.c_int(), g500.ValidateReport()
+            g500.check(g500.lib().g500_validate(g.h, elist.data_ptr() + 12 * skip, len(edges) - skip - drop, 1, root,
+                                                dev.data_ptr(), 1, C.byref(evc), C.byref(ok), C.byref(rep)))
+            got = (bool(ok.value), evc.value, {f[0]: getattr(rep, f[0]) for f in g500.ValidateReport._fields_})
+            assert got == reports.setdefault((skip, drop), got), (lg, skip, drop)
+            assert got[0] == (planted == "none") or drop or skip
+            if lg <= 21:
+                assert got == _noalloc(g500, elist.data_ptr() + 12 * skip, len(edges) - skip - drop,
+                                       g.info.max_used_vertex + 1, g.pred_size(), root, dev)
+        bfs.close()

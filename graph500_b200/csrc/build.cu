@@ -324,7 +324,7 @@ static int build_from_device_edges(g500_graph* g, const g500_packed_edge* d_edge
   big.add(&keys, nk);
   big.add(&alt, nk);
   const size_t both_bytes = big.bytes;  // keys and alt as one region
-  big.add(&d_sort_tmp, (int64_t)sort_tmp_bytes(INT64_MAX / 2));
+  big.add(&d_sort_tmp, (int64_t)sort_tmp_bytes(nk));
   big.add(&d_scalars, 4);
   G500_TRY(tmp.alloc(big, "construction scratch"));
   G500_CUDA(cudaMemsetAsync(d_scalars, 0, 4 * sizeof(unsigned long long), s));
@@ -344,6 +344,7 @@ static int build_from_device_edges(g500_graph* g, const g500_packed_edge* d_edge
   // degrees
   uint32_t *deg = nullptr, *sl = nullptr, *has_edge = nullptr;
   uint64_t *k = nullptr, *k2 = nullptr;
+  char* d_vsort_tmp = nullptr;
   Slab verts;
   verts.add(&deg, nolv);
   verts.add(&sl, nolv);
@@ -351,6 +352,7 @@ static int build_from_device_edges(g500_graph* g, const g500_packed_edge* d_edge
   if (g->reorder_mode != 0) {
     verts.add(&k, nolv);
     verts.add(&k2, nolv);
+    verts.add(&d_vsort_tmp, (int64_t)sort_tmp_bytes(nolv));
   }
   G500_TRY(tmp.place(verts, keys, both_bytes, "degrees and reorder keys"));
   G500_CUDA(cudaMemsetAsync(deg, 0, sizeof(uint32_t) * nolv, s));
@@ -381,7 +383,7 @@ static int build_from_device_edges(g500_graph* g, const g500_packed_edge* d_edge
     reorder_keys_kernel<<<grid_for(nolv), 256, 0, s>>>(deg, nolv, g->reorder_mode, maxdeg, k);
     G500_CUDA(cudaGetLastError());
     int hi = 32 + (g->reorder_mode == 2 ? std::max(1, bits_for((uint64_t)maxdeg + 1)) : 1);
-    G500_TRY(radix_sort_u64(k, k2, nolv, 32, hi, d_sort_tmp, s, &sorted_v));
+    G500_TRY(radix_sort_u64(k, k2, nolv, 32, hi, d_vsort_tmp, s, &sorted_v));
     maps_from_keys_kernel<<<grid_for(nolv), 256, 0, s>>>(sorted_v, nolv, g->d_invert, g->d_reorder);
   }
   G500_CUDA(cudaGetLastError());

@@ -1328,12 +1328,11 @@ __global__ void ms_degree_kernel(const uint64_t* __restrict__ off, int64_t nlv, 
 // reached count follow).  Nearly every vertex is reached by every lane, so a
 // warp looks at single lanes only for the words where one of its 32 vertices
 // lacks some: SCALE 24, 64 roots: two reductions per lane and 32 vertices took
-// 1.03 ms, now 0.13 ms with its launches.  Lanes that lack a word's vertices
+// 1.02 ms a call, now 0.10.  Lanes that lack a word's vertices
 // altogether (roots in small components lack nearly all) get its totals without a
 // look of their own, and each thread keeps the sums of one lane per mask word, so
 // that no lane costs an atomic per word: 2^21 pairs of vertices, 64 roots: 455 us
-// a call with shared-memory atomics, 59 now, 193 when every lane was reduced;
-// SCALE 24, 64 roots 114 -> 96 us.
+// a call with shared-memory atomics, 59 now, 193 when every lane was reduced.
 // A vertex without edges can only be a root itself: its lane's missing sums get it
 // taken off.
 // The last block to finish turns the sums into each root's reached count and 2 x
